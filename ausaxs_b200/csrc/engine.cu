@@ -295,8 +295,11 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     nb = std::min(nb, cfg.bin_count);
     if (P.manager == cfg.manager && P.weighted == weighted && P.bin_count == cfg.bin_count &&
         P.bin_width == cfg.bin_width && P.n_a == n_a && P.n_w == n_w && P.n_x == n_x && P.T == T && P.nb >= nb &&
-        P.nb <= nb + 64 && (cfg.manager != AUSAXS_MANAGER_FFGRID || n_x < kLatticeMinPoints || lat.tried))
+        P.nb <= nb + 64 && (cfg.manager != AUSAXS_MANAGER_FFGRID || n_x < kLatticeMinPoints || lat.tried) &&
+        std::equal(type_ff, type_ff + T, P.type_ff)) {
+        P.fin_ff.z_exv = cfg.z_exv;  // per call: other molecules of the same shape have other volumes
         return P;
+    }
 
     Ctx& C = *ctx;
     P.manager = cfg.manager;
@@ -307,6 +310,7 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     P.n_w = n_w;
     P.n_x = n_x;
     P.T = T;
+    std::copy(type_ff, type_ff + T, P.type_ff);
     P.nb = nb;
     P.inv_w = inv_w;
     P.c = (float)(1.0 / (double)inv_w);
@@ -688,7 +692,8 @@ static bool enqueue_debye_x(Ctx& C, DebyeArgs& A, XBufs& X, double w) {
         X.qmax = qmax;
     }
     const int K = debye_x_order(X.qmax, w);
-    const bool same = X.H == A.H && X.q == A.q && X.R == A.R && X.nb == A.nb && X.nq == A.nq && X.w == w && XP.K == K;
+    const bool same = X.H == A.H && X.q == A.q && X.R == A.R && X.nb == A.nb && X.nq == A.nq && X.w == w && XP.K == K &&
+                      X.exv_model == A.exv_model;  // (the rows' distance axes follow the model)
     if (!same) {
         XP.w = w;
         XP.nq = A.nq;
@@ -755,6 +760,7 @@ static bool enqueue_debye_x(Ctx& C, DebyeArgs& A, XBufs& X, double w) {
         X.R = A.R;
         X.nb = A.nb;
         X.nq = A.nq;
+        X.exv_model = A.exv_model;
         X.w = w;
     }
     if (!debye_x_enqueue(XP, A.q, s)) return false;

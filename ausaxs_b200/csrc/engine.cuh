@@ -72,7 +72,7 @@ struct XBufs {
     // shape the buffers were made for
     const double* H = nullptr;
     const double* q = nullptr;
-    int R = 0, nb = 0, nq = 0;
+    int R = 0, nb = 0, nq = 0, exv_model = 0;
     double w = 0, qmax = -1;
 };
 
@@ -84,6 +84,7 @@ struct Plan {
     int manager = 0, weighted = 0, bin_count = 0;
     double bin_width = 0;
     int n_a = -1, n_w = -1, n_x = -1, T = -1;
+    int type_ff[kNff] = {};  // the form-factor types behind the rows
     // shapes
     int nb = 0, tile = 256;
     struct Group {  // one pair-kernel launch

@@ -273,3 +273,30 @@ def test_all_pairs_in_one_bin(gpu_ctx):
     z = 1.0 * 0.334 / n
     assert aa[3, 0, 0] == n * (n - 1) * z
     assert aa[0, 0, 0] == (n * (n - 1) + n) * (z * z)
+
+
+@pytest.mark.parametrize("change", ["volume", "types", "manager"])
+def test_one_shot_calls_of_one_shape(gpu_ctx, change):
+    """One-shot calls share a scratch structure: a molecule of the same shape as the one before, but of
+    another volume or with other form-factor types, gives what a fresh context gives."""
+    rng = np.random.default_rng(3)
+    xyz, ff = synth.globule(9, 900)
+    ff = np.where(ff == 12, 3, ff)  # three types
+    w = rng.normal(0, 12, (90, 3))
+    x = np.floor(rng.uniform(-12, 12, (700, 3))) + 0.5
+    q = np.linspace(0.005, 1.0, 400)
+    first = hist.Molecule(atoms=xyz, ff_types=ff, waters=w, exv=x, volume=16000.0)
+    second = hist.Molecule(atoms=xyz, ff_types=np.where(ff == 7, 12, ff) if change == "types" else ff, waters=w, exv=x,
+                           volume=23000.0 if change == "volume" else 16000.0)
+
+    def run(ctx, m, grid):
+        if grid:
+            return hist.profile(hist.HistogramManagerMTFFGrid(m, 0.1, 8000, ctx), q, precision=3)
+        return hist.profile(hist.HistogramManagerMTFFAvg(m, True, 0.1, 8000, ctx), q, precision=3)
+
+    run(gpu_ctx, first, change == "manager")
+    got = run(gpu_ctx, second, False)
+    fresh = _capi.Context(0)
+    want = run(fresh, second, False)
+    fresh.close()
+    np.testing.assert_array_equal(got, want)
