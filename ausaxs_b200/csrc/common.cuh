@@ -88,6 +88,17 @@ __device__ __forceinline__ float pair_sqrt_nr(float s) {
     return __fmaf_rn(__fmaf_rn(-d0, d0, s), h, d0);
 }
 
+// The same root on coordinates scaled by 2^-23 (s = 2^-46 |a - b|^2, result 2^-23 d): every operation
+// scales exactly, half the reciprocal root is its exponent less one, and the guard only touches
+// distances below 1e-11.
+__device__ __forceinline__ float pair_sqrt_scaled(float s) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaxf(s, 1e-36f)));
+    const float d0 = __fmul_rn(s, y);
+    const float h = __int_as_float(__float_as_int(y) - 0x00800000);
+    return __fmaf_rn(__fmaf_rn(-d0, d0, s), h, d0);
+}
+
 // Fixed-point in-bin offset of a pair: the distance is d = bin*c + r with |r| <= c/2 (1 + 2^-10)
 // (c = 1/inv_w rounded to float), r is stored as rint(r * scale) + kResBias in [0, 2^16) with
 // scale = 2^15 / c * (1 - 2^-8).  Sums of these are exact integers, so the per-bin mean distance

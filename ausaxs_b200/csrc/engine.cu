@@ -115,6 +115,13 @@ void Structure::load_begin(const float* atoms, int n_atoms, const float* waters,
     AUSAXS_CUDA(cudaMemcpyAsync(h_stats, d_stats, sizeof(PrepStats), cudaMemcpyDeviceToHost, s));
 }
 
+// layout of Structure::typed: lists, prefix table, chunk counts, places
+static size_t typed_off_pre(int n) { return align_up((size_t)std::max(1, n) * 16, 256); }
+static size_t typed_off_counts(int n) { return typed_off_pre(n) + align_up((size_t)typed_pre_stride(n) * 4 * kMaxTypes + 4, 256); }
+static size_t typed_off_pos(int n) { return typed_off_counts(n) + align_up((size_t)typed_chunks(n) * 16 * 4 + 4, 256); }
+size_t Structure::typed_bytes(int n) { return typed_off_pos(n) + align_up((size_t)std::max(1, n) * 4, 256); }
+int32_t* Structure::typed_pos() const { return typed.as<int32_t>(typed_off_pos(n_a)); }
+
 void Structure::load_end(const PrepStats& st) {
     Ctx& C = *ctx;
     cudaStream_t s = C.stream;
@@ -158,8 +165,27 @@ void Structure::load_end(const PrepStats& st) {
     AUSAXS_CUDA(cudaMemcpyAsync(meta.p, hmeta, sizeof(hmeta), cudaMemcpyHostToDevice, s));
     if (ff_typed) {
         dense_a.ensure(align_up(std::max(1, n_a) * 16, 256));
-        to_dense_launch(raw_a.as<float4>(), dense_a.as<float4>(), n_a, meta.as<int32_t>(kNff * 4), C.sm_count, s);
-        C.check_launch("to_dense");
+        typed.ensure(typed_bytes(n_a));
+        lists = TypedSet{};
+        lists.pts = typed.as<float4>();
+        lists.pre = typed.as<int32_t>(typed_off_pre(n_a));
+        lists.pre_stride = typed_pre_stride(n_a);
+        lists.types = T;
+        TypedOut o{};
+        o.pts = typed.as<float4>();
+        o.pre = typed.as<int32_t>(typed_off_pre(n_a));
+        o.pos = want_pos ? typed_pos() : nullptr;
+        o.types = T;
+        o.pre_stride = lists.pre_stride;
+        for (int t = 0, at = 0; t < T; ++t) {
+            lists.start[t] = o.start[t] = at;
+            lists.count[t] = type_count[t];
+            at += type_count[t];
+        }
+        typed_lists_launch(raw_a.as<float4>(), dense_a.as<float4>(), n_a, meta.as<int32_t>(kNff * 4), o,
+                           typed.as<int32_t>(typed_off_counts(n_a)), s);
+        C.check_launch("typed lists");
+        if (n_a > 0) C.launches += 1;  // two kernels
     }
 }
 
@@ -231,6 +257,73 @@ void append_pair_jobs(const Plan& P, int tile, bool by_class, std::vector<PairJo
     }
 }
 
+void append_pack_jobs(const Plan& P, int outer, bool joint, PackLaunch& L, PackTable& T, bool skip_lattice) {
+    auto up = [](int n, int d) { return (n + d - 1) / d; };
+    const size_t first = T.jobs.size();
+    std::vector<unsigned long long*> sums;  // the open group's offset sums
+    int rows = 0;                           // and its count rows
+    auto close = [&](size_t from) {
+        if (T.jobs.size() == from) return;
+        for (size_t k = from; k < T.jobs.size(); ++k) {
+            T.jobs[k].group = T.groups;
+            T.jobs[k].group_rows = rows;
+            T.jobs[k].group_sums = (int)sums.size();
+            T.jobs[k].group_out = (int)T.out.size() - rows;
+        }
+        T.out.insert(T.out.end(), sums.begin(), sums.end());
+        L.group_rows = std::max(L.group_rows, rows);
+        L.group_sums = std::max(L.group_sums, (int)sums.size());
+        sums.clear();
+        rows = 0;
+        ++T.groups;
+    };
+    for (const JobSpec& j : P.specs) {
+        if (skip_lattice && j.lattice) continue;
+        const bool pair_rows = j.rmode == kRowPair;
+        // the largest row's share of a job's pairs (outer points have the composition of the whole structure)
+        const double share = j.rows == 1 ? 1.0 : P.row_share;
+        for (int t = 0; t < (pair_rows ? j.typed->types : 1); ++t) {
+            PackJob p{};
+            p.A = j.A;
+            p.na = j.na;
+            p.B = pair_rows ? j.typed->pts + j.typed->start[t] : j.B;
+            p.nb = pair_rows ? j.typed->count[t] : j.nbp;
+            if (p.nb == 0) continue;
+            p.self = j.self;
+            p.indexed = pair_rows ? 1 : 0;
+            p.pre = pair_rows ? j.typed->pre + (size_t)t * j.typed->pre_stride : nullptr;
+            p.rows = pair_rows ? P.T : j.rows;
+            p.nbins = P.nb;
+            p.tiles_i = up(p.na, outer);
+            p.tiles_j = up(p.nb, L.tile_j);
+            p.tile_begin = L.total_tiles;
+            p.inv_w = P.inv_w;
+            p.c = P.c;
+            p.scale = P.scale;
+            p.a_base = j.a_base;
+            p.b_base = j.b_base;
+            p.tail_end = j.tail_end >= 0 ? j.tail_end : j.nbp;
+            p.tail_from_outer = j.tail_from_outer >= 0 ? j.tail_from_outer : j.self;
+            p.seg_pairs = pack_segment_pairs(P.nb, share);
+            p.cnt_row = rows;
+            for (int r = 0; r < p.rows; ++r) T.out.push_back(j.counts + (size_t)(pair_rows ? r * P.T + t : r) * P.nb);
+            rows += p.rows;
+            if (j.dsum) {
+                auto it = std::find(sums.begin(), sums.end(), j.dsum);
+                p.sum_slot = (int)(it - sums.begin());
+                if (it == sums.end()) sums.push_back(j.dsum);
+            }
+            T.jobs.push_back(p);
+            L.rows = std::max(L.rows, (int)p.rows);
+            L.bins = std::max(L.bins, P.nb);
+            L.total_tiles += (long long)p.tiles_i * p.tiles_j;
+            if (!joint) close(T.jobs.size() - 1);
+        }
+    }
+    if (joint) close(first);
+    L.n_jobs = (int)T.jobs.size();
+}
+
 bool Structure::lattice_ready() {
     if (lat.tried) return lat.usable;
     lat.tried = true;
@@ -279,6 +372,113 @@ bool Structure::lattice_ready() {
     return true;
 }
 
+// The plan's pair passes as launches of the two-atomic kernel (weighted plans, and widths or row counts
+// the one-atomic kernel does not take).
+static void plan_groups(Plan& P, char* base, Ctx& C) {
+    // Jobs split into launch groups by the rows they keep on chip: one-row jobs (ww, xx, wx and all
+    // Simple jobs) run with a small footprint and high occupancy, multi-row jobs (aa, aw, ax) get the
+    // shared memory they need.  Large structures: one launch per row class (1, T, T*T rows) so each
+    // gets the occupancy its footprint allows; small ones: everything in one launch (launch latency
+    // dominates).  Tiles are numbered per group.
+    const bool split = P.pairs >= 2000000000LL;
+    std::vector<PairJob> group_jobs[3];
+    long long group_tiles[3] = {0, 0, 0};
+    int group_rows[3] = {1, 1, 1};
+    append_pair_jobs(P, P.tile, split, group_jobs, group_tiles, group_rows, 0, true);
+    if (group_jobs[0].size() + group_jobs[1].size() + group_jobs[2].size() > 64)
+        throw Error{AUSAXS_ERR_CAPACITY, "too many row groups"};
+    const bool w_launch = P.manager == AUSAXS_MANAGER_MT;  // Simple histograms always carry weight sums (values)
+    P.n_launch = 0;
+    size_t job_off = P.off_jobs;
+    for (int g = 0; g < 3; ++g) {
+        if (group_jobs[g].empty()) continue;
+        Plan::Group& G = P.group[P.n_launch++];
+        G.tile = P.tile;
+        G.smem = pairhist_launch_smem(group_rows[g], P.nb, w_launch, P.tile);
+        const bool dreg = pairhist_dreg(group_rows[g], P.nb, w_launch, P.tile);
+        const int groups = pairhist_groups(G.smem, P.tile, dreg, w_launch, group_tiles[g], C.sm_count);
+        const int per_sm = pairhist_ctas_per_sm(G.smem, P.tile, dreg, w_launch, groups);
+        G.grid = (int)std::min<long long>((long long)C.sm_count * per_sm, std::max<long long>(1, group_tiles[g]));
+        PairLaunch& L = G.launch;
+        L.groups = groups;
+        L.jobs = reinterpret_cast<const PairJob*>(base + job_off);
+        L.n_jobs = (int)group_jobs[g].size();
+        L.total_tiles = group_tiles[g];
+        L.chunk = (int)std::max<long long>(1, std::min<long long>(8, group_tiles[g] / ((long long)G.grid * 8)));
+        L.smem_rows = group_rows[g];
+        L.smem_bins = P.nb;
+        L.tile_counter = reinterpret_cast<unsigned long long*>(base + P.off_counter) + g;
+        L.overflow = reinterpret_cast<unsigned long long*>(base + P.off_overflow);
+        L.weighted = w_launch;
+        L.dreg = pairhist_dreg(group_rows[g], P.nb, w_launch, P.tile) ? 1 : 0;
+        L.wscale = reinterpret_cast<const float*>(base + P.off_wscale);
+        L.inv_w = P.inv_w;
+        AUSAXS_CUDA(cudaMemcpyAsync(base + job_off, group_jobs[g].data(), sizeof(PairJob) * group_jobs[g].size(),
+                                    cudaMemcpyHostToDevice, C.stream));  // pageable: staged on return
+        job_off += sizeof(PairJob) * group_jobs[g].size();
+    }
+}
+
+// Tiles that hold pairs, about: self passes half of theirs.
+static double pack_tiles(const std::vector<JobSpec>& specs, int outer, int tile_j) {
+    auto up = [](int n, int d) { return (double)((n + d - 1) / d); };
+    double n = 0;
+    for (const JobSpec& j : specs) {
+        if (j.lattice) continue;
+        double tj = 0;
+        if (j.rmode == kRowPair)
+            for (int t = 0; t < j.typed->types; ++t) tj += up(j.typed->count[t], tile_j);
+        else
+            tj = up(j.nbp, tile_j);
+        n += up(j.na, outer) * tj * (j.self ? 0.5 : 1.0);
+    }
+    return n;
+}
+
+bool choose_pack(const Plan& P, int sm_count, PackLaunch& L, int& shape, int& grid, PackTable& T) {
+    L = PackLaunch{};
+    L.nr = pair_sqrt_mode(P.inv_w, P.nb);
+    L.offsets = P.weighted;
+    if (!L.nr || P.specs.empty()) return false;
+    auto table = [&](int s, int tile_j, bool joint) {
+        PackLaunch K{};
+        K.nr = L.nr;
+        K.offsets = L.offsets;
+        K.tile_j = tile_j;
+        T = PackTable{};
+        append_pack_jobs(P, kPackShapes[s].outer(), joint, K, T, true);
+        return K;
+    };
+    L = table(0, kPackMaxTileJ, false);
+    const int s0 = pack_shape(L);
+    if (s0 < 0) return false;
+    // The longest inner tiles that still give every resident CTA two tiles (a tile costs about 3 us beyond
+    // its pairs).  Where even 256 points do not, two thread groups share every tile (shape 2).  Measured
+    // (pair kernel, 256- and 512-point tiles / two groups on 64 to 128): 500 atoms 35 / 17 us, 1,500 atoms
+    // 41 / 18 us, 5,000 atoms 52 / 46 us, 12,000 atoms 123 / 149 us; 20,000 atoms 267 us with 512 or 256
+    // points, 315 us with 128.
+    int tile_j = kPackMaxTileJ;
+    auto pick = [&](int s, int least) {
+        for (int tj = kPackMaxTileJ; tj >= least; tj /= 2) {
+            PackLaunch K = L;
+            K.tile_j = tj;
+            shape = s;
+            tile_j = tj;
+            if (pack_tiles(P.specs, kPackShapes[s].outer(), tj) >= 2.0 * sm_count * pack_ctas_per_sm(s, K)) return true;
+        }
+        return false;
+    };
+    if (!pick(s0, 256) && s0 == 0) pick(2, 64);
+    // one group where its rows cost no CTA per SM: a CTA then flushes once, not at every change of job
+    L = table(shape, tile_j, false);
+    const int per_sm = pack_ctas_per_sm(shape, L);
+    const PackLaunch joint = table(shape, tile_j, true);
+    if (pack_ctas_per_sm(shape, joint) >= per_sm) L = joint;
+    else L = table(shape, tile_j, false);
+    grid = (int)std::min<long long>((long long)sm_count * per_sm, std::max<long long>(1, L.total_tiles));
+    return true;
+}
+
 Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     Plan& P = plan;
     if (cfg.bin_width <= 0 || cfg.bin_count <= 0) throw Error{AUSAXS_ERR_ARGUMENT, "bin_width and bin_count must be positive"};
@@ -296,7 +496,7 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     if (P.manager == cfg.manager && P.weighted == weighted && P.bin_count == cfg.bin_count &&
         P.bin_width == cfg.bin_width && P.n_a == n_a && P.n_w == n_w && P.n_x == n_x && P.T == T && P.nb >= nb &&
         P.nb <= nb + 64 && (cfg.manager != AUSAXS_MANAGER_FFGRID || n_x < kLatticeMinPoints || lat.tried) &&
-        std::equal(type_ff, type_ff + T, P.type_ff)) {
+        std::equal(type_ff, type_ff + T, P.type_ff) && (!P.packed || std::equal(type_count, type_count + T, P.type_count))) {
         P.fin_ff.z_exv = cfg.z_exv;  // per call: other molecules of the same shape have other volumes
         return P;
     }
@@ -311,6 +511,9 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     P.n_x = n_x;
     P.T = T;
     std::copy(type_ff, type_ff + T, P.type_ff);
+    std::copy(type_count, type_count + T, P.type_count);
+    P.row_share = 1.0;
+    if (T > 0 && n_a > 0) P.row_share = (double)*std::max_element(type_count, type_count + T) / n_a;
     P.nb = nb;
     P.inv_w = inv_w;
     P.c = (float)(1.0 / (double)inv_w);
@@ -374,7 +577,7 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     size_t off = 0;
     P.off_jobs = off;
     std::vector<PairJob> jobs;
-    off += align_up(sizeof(PairJob) * 64, 256);
+    off += align_up(std::max(sizeof(PairJob), sizeof(PackJob)) * 64 + sizeof(void*) * 512, 256);
     P.off_acc = off;
     size_t slot_cnt[slots], slot_ds[slots], slot_ws[slots];
     for (int k = 0; k < slots; ++k) {
@@ -452,6 +655,7 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
         sp.dsum = weighted ? reinterpret_cast<unsigned long long*>(base + slot_ds[j.slot]) : nullptr;
         sp.wsum = mt ? reinterpret_cast<long long*>(base + slot_ws[j.slot]) : nullptr;
         sp.lattice = use_lattice && j.slot == 5;
+        sp.typed = j.slot == 0 && !mt ? &lists : nullptr;
         P.specs.push_back(sp);
     }
     P.max_group_rows = max_group_rows;
@@ -472,50 +676,24 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
         LL.tail_fix = lattice_rules_agree(lat.s2_max, inv_w) ? 0 : 1;
     }
 
-    // Jobs split into launch groups by the rows they keep on chip: one-row jobs (ww, xx, wx and all
-    // Simple jobs) run with a small footprint and high occupancy, multi-row jobs (aa, aw, ax) get the
-    // shared memory they need.  Large structures: one launch per row class (1, T, T*T rows) so each
-    // gets the occupancy its footprint allows; small ones: everything in one launch (launch latency
-    // dominates).  Tiles are numbered per group.
     pair_sqrt_prepare(P.inv_w, nb);  // once per width and process: the Newton-Raphson root where it bins exactly
-    const bool split = P.pairs >= 2000000000LL;
-    std::vector<PairJob> group_jobs[3];
-    long long group_tiles[3] = {0, 0, 0};
-    int group_rows[3] = {1, 1, 1};
-    append_pair_jobs(P, tile, split, group_jobs, group_tiles, group_rows, 0, true);
-    if (group_jobs[0].size() + group_jobs[1].size() + group_jobs[2].size() > 64)
-        throw Error{AUSAXS_ERR_CAPACITY, "too many row groups"};
-    const bool w_launch = mt;  // Simple histograms always carry weight sums (values)
     P.n_launch = 0;
-    P.total_tiles = 0;
-    size_t job_off = P.off_jobs;
-    for (int g = 0; g < 3; ++g) {
-        if (group_jobs[g].empty()) continue;
-        Plan::Group& G = P.group[P.n_launch++];
-        G.tile = tile;
-        G.smem = pairhist_launch_smem(group_rows[g], nb, w_launch, tile);
-        const bool dreg = pairhist_dreg(group_rows[g], nb, w_launch, tile);
-        const int groups = pairhist_groups(G.smem, tile, dreg, w_launch, group_tiles[g], C.sm_count);
-        const int per_sm = pairhist_ctas_per_sm(G.smem, tile, dreg, w_launch, groups);
-        G.grid = (int)std::min<long long>((long long)C.sm_count * per_sm, std::max<long long>(1, group_tiles[g]));
-        PairLaunch& L = G.launch;
-        L.groups = groups;
-        L.jobs = reinterpret_cast<const PairJob*>(base + job_off);
-        L.n_jobs = (int)group_jobs[g].size();
-        L.total_tiles = group_tiles[g];
-        L.chunk = (int)std::max<long long>(1, std::min<long long>(8, group_tiles[g] / ((long long)G.grid * 8)));
-        L.smem_rows = group_rows[g];
-        L.smem_bins = nb;
-        L.tile_counter = reinterpret_cast<unsigned long long*>(base + P.off_counter) + g;
-        L.overflow = reinterpret_cast<unsigned long long*>(base + P.off_overflow);
-        L.weighted = w_launch;
-        L.dreg = pairhist_dreg(group_rows[g], nb, w_launch, tile) ? 1 : 0;
-        L.wscale = reinterpret_cast<const float*>(base + P.off_wscale);
-        L.inv_w = P.inv_w;
-        AUSAXS_CUDA(cudaMemcpyAsync(base + job_off, group_jobs[g].data(), sizeof(PairJob) * group_jobs[g].size(),
-                                    cudaMemcpyHostToDevice, C.stream));  // pageable: staged on return
-        job_off += sizeof(PairJob) * group_jobs[g].size();
-        P.total_tiles += group_tiles[g];
+    PackTable table;
+    P.packed = !mt && choose_pack(P, C.sm_count, P.pack, P.pack_shape, P.pack_grid, table);
+    if (P.packed) {
+        const size_t jobs_bytes = sizeof(PackJob) * table.jobs.size();
+        if (jobs_bytes + sizeof(void*) * table.out.size() > P.off_acc - P.off_jobs)
+            throw Error{AUSAXS_ERR_CAPACITY, "too many pair jobs"};
+        P.pack.jobs = reinterpret_cast<const PackJob*>(base + P.off_jobs);
+        P.pack.out = reinterpret_cast<unsigned long long* const*>(base + P.off_jobs + jobs_bytes);
+        P.pack.tile_counter = reinterpret_cast<unsigned long long*>(base + P.off_counter);
+        P.pack.overflow = reinterpret_cast<unsigned long long*>(base + P.off_overflow);
+        // pageable sources: staged on return
+        AUSAXS_CUDA(cudaMemcpyAsync(base + P.off_jobs, table.jobs.data(), jobs_bytes, cudaMemcpyHostToDevice, C.stream));
+        AUSAXS_CUDA(cudaMemcpyAsync(base + P.off_jobs + jobs_bytes, table.out.data(), sizeof(void*) * table.out.size(),
+                                    cudaMemcpyHostToDevice, C.stream));
+    } else {
+        plan_groups(P, base, C);
     }
 
     // finalisation
@@ -614,6 +792,13 @@ void Structure::enqueue_histogram(const ausaxs_hist_config& cfg) {
         weight_square_sum_launch(raw_a.as<float4>(), n_a, reinterpret_cast<double*>(base + P.off_self), s);
         weight_square_sum_launch(raw_w.as<float4>(), n_w, reinterpret_cast<double*>(base + P.off_self) + 1, s);
         C.check_launch("weights");
+    }
+    if (P.packed && P.pack.n_jobs > 0) {
+        cudaEvent_t ev;
+        C.time_begin(0, &ev);
+        pack_launch(P.pack, P.pack_shape, P.pack_grid, s);
+        C.check_launch("pairpack");
+        C.time_end(0, ev);
     }
     for (int g = 0; g < P.n_launch; ++g) {
         const Plan::Group& G = P.group[g];

@@ -11,6 +11,7 @@
 #include "finalize.cuh"
 #include "lattice.cuh"
 #include "pairhist.cuh"
+#include "pairpack.cuh"
 #include "prep.cuh"
 
 namespace ausaxs_b200 {
@@ -47,6 +48,14 @@ struct DevBuf {
 
 struct Ctx;
 
+// A point set's lists by type on the device (typed_lists_launch) with their sizes.
+struct TypedSet {
+    const float4* pts = nullptr;
+    const int32_t* pre = nullptr;
+    int pre_stride = 0, types = 0;
+    int start[16] = {}, count[16] = {};
+};
+
 // One pass of pair binning of a structure before it is cut into tiles: the two point sets, the
 // rows it increments, and where its global accumulators live.
 struct JobSpec {
@@ -62,6 +71,7 @@ struct JobSpec {
     int a_base = 0, b_base = 0, tail_end = -1, tail_from_outer = -1;
     int mult = 1;  // multiplicity of every pair (PairJob::mult)
     bool lattice = false;  // the plan bins this pass with the lattice kernel (the structure's own launches)
+    const TypedSet* typed = nullptr;  // atom-atom passes: the inner atoms' lists (append_pack_jobs)
 };
 
 // Buffers of the exact-accumulation tensor-core transform of one structure's rows (debye_x.cu), kept
@@ -84,7 +94,8 @@ struct Plan {
     int manager = 0, weighted = 0, bin_count = 0;
     double bin_width = 0;
     int n_a = -1, n_w = -1, n_x = -1, T = -1;
-    int type_ff[kNff] = {};  // the form-factor types behind the rows
+    int type_ff[kNff] = {};     // the form-factor types behind the rows
+    int type_count[kNff] = {};  // and the sizes of the typed lists
     // shapes
     int nb = 0, tile = 256;
     struct Group {  // one pair-kernel launch
@@ -93,8 +104,13 @@ struct Plan {
         size_t smem = 0;
     } group[3];
     int n_launch = 0;
-    long long total_tiles = 0, pairs = 0;
+    // the same passes with one atomic per pair (pairpack.cuh) instead of the groups above
+    bool packed = false;
+    PackLaunch pack{};
+    int pack_shape = 0, pack_grid = 0;
+    long long pairs = 0;
     int R = 0;
+    double row_share = 1;  // share of the most frequent atom type
     float inv_w = 0, c = 0, scale = 0;
     // device layout
     DevBuf dev;
@@ -131,6 +147,11 @@ struct Structure {
     int ff_typed = 0;
     int n_a = 0, n_w = 0, n_x = 0;
     DevBuf raw_a, raw_w, raw_x, dense_a, meta;
+    DevBuf typed;           // the atoms' lists by type (typed_bytes)
+    TypedSet lists;
+    bool want_pos = false;  // also every atom's place in them (typed_pos)
+    static size_t typed_bytes(int n);
+    int32_t* typed_pos() const;
     int T = 0;
     int type_ff[kNff] = {};
     int type_count[kNff] = {};
@@ -210,6 +231,22 @@ struct Ctx {
 // skip_lattice: leave out the passes the plan bins with the lattice kernel.
 void append_pair_jobs(const Plan& P, int tile, bool by_class, std::vector<PairJob> (&jobs)[3], long long (&tiles)[3],
                       int (&rows)[3], int max_rows = 0, bool skip_lattice = false);
+
+// The same passes as jobs of the one-atomic-per-pair kernel, atom-atom passes cut by inner type, for
+// outer tiles of `outer` and L.tile_j inner points.  The jobs and the accumulators they flush to are
+// appended; L's row, sum and bin maxima, job and tile counts grow with them.  joint: one group for all of the
+// plan's jobs, else a group per job.
+struct PackTable {
+    std::vector<PackJob> jobs;
+    std::vector<unsigned long long*> out;
+    int groups = 0;
+};
+void append_pack_jobs(const Plan& P, int outer, bool joint, PackLaunch& L, PackTable& T, bool skip_lattice = false);
+
+// Shape of a launch of the one-atomic-per-pair kernel over the plan's passes, and its jobs; false where
+// the kernel does not apply: an inverse width whose root is not verified, or more rows and bins than
+// fit on chip.
+bool choose_pack(const Plan& P, int sm_count, PackLaunch& L, int& shape, int& grid, PackTable& T);
 
 // Clears n device ranges of u64 words in one launch (table in device memory); a range with a
 // source is set to the source's words instead.

@@ -23,6 +23,8 @@
 //     (or before a 32-bit count could wrap), so the global traffic is one atomic per non-empty
 //     on-chip bin per flush instead of one per pair.
 // All accumulations are integer, so results do not depend on scheduling.
+#include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -590,6 +592,10 @@ __global__ void sqrt_check_kernel(uint32_t hi_bits, float inv_w, unsigned long l
         const float xa = __fmul_rn(__fsqrt_rn(s), inv_w), xb = __fmul_rn(pair_sqrt_nr(s), inv_w);
         // ties to even (the SIMD evaluators) and ties away from zero (the scalar tail)
         if (rintf(xa) != rintf(xb) || roundf(xa) != roundf(xb)) ++bad;
+        // the same root on scaled coordinates: the same distance, except where underflow of the scaled
+        // residual can show (below 1e-8), far under a step of the 16-bit offset in bin 0
+        const float ds = __fmul_rn(pair_sqrt_scaled(__fmul_rn(s, 0x1p-46f)), 8388608.0f), dn = pair_sqrt_nr(s);
+        if (ds != dn && !(fmaxf(ds, dn) * inv_w * 32768.f < 0.25f)) ++bad;
     }
     for (int o = 16; o > 0; o >>= 1) bad += __shfl_xor_sync(0xffffffffu, bad, o);
     if ((threadIdx.x & 31) == 0 && bad) atomicAdd(mismatches, bad);
@@ -597,7 +603,8 @@ __global__ void sqrt_check_kernel(uint32_t hi_bits, float inv_w, unsigned long l
 
 struct SqrtVerified {
     std::mutex m;
-    std::map<uint32_t, int> bins;  // inverse bin width (bits) -> bins verified (0: failed)
+    std::map<uint32_t, int> bins;    // inverse bin width (bits) -> bins verified
+    std::map<uint32_t, int> failed;  // -> bins at which the check failed (never tried again from there on)
 };
 SqrtVerified g_sqrt;
 
@@ -624,7 +631,9 @@ bool pair_sqrt_prepare(float inv_w, int bins) {
     {
         std::lock_guard<std::mutex> lk(g_sqrt.m);
         auto it = g_sqrt.bins.find(key);
-        if (it != g_sqrt.bins.end() && (it->second == 0 || it->second >= want)) return it->second >= bins;
+        if (it != g_sqrt.bins.end() && it->second >= bins) return true;
+        auto bad = g_sqrt.failed.find(key);
+        if (bad != g_sqrt.failed.end() && want >= bad->second) return false;
     }
     // every float below the squared distance of bin want + 2 (the overflow clamp lies below it)
     const double dmax = (want + 2.0) / inv_w;
@@ -643,26 +652,27 @@ bool pair_sqrt_prepare(float inv_w, int bins) {
     }
     cudaGetLastError();
     std::lock_guard<std::mutex> lk(g_sqrt.m);
-    g_sqrt.bins[key] = ok ? want : 0;
-    return ok && want >= bins;
+    if (ok) g_sqrt.bins[key] = std::max(g_sqrt.bins[key], want);
+    else g_sqrt.failed[key] = want;
+    return ok;
+}
+
+int pair_sqrt_mode(float inv_w, int bins) {
+    std::lock_guard<std::mutex> lk(g_sqrt.m);
+    uint32_t key;
+    std::memcpy(&key, &inv_w, 4);
+    auto it = g_sqrt.bins.find(key);
+    if (!(inv_w > 0) || it == g_sqrt.bins.end() || it->second < bins) return 0;
+    // a power-of-two inverse width (0.25 A bins): the product d inv_w is exact, so the rounding to a
+    // bin fuses with it (one FMA per pair instead of a product and a sum)
+    int e = 0;
+    return std::frexp(inv_w, &e) == 0.5f ? 2 : 1;
 }
 
 void pairhist_launch(const PairLaunch& L0, int tile, int grid, size_t smem, cudaStream_t s) {
     PairLaunch L = L0;
     // the Newton-Raphson root where every job's width was verified for its bins (pair_sqrt_prepare)
-    L.nr_sqrt = 0;
-    {
-        // the jobs live in device memory; the launch's bins and the width recorded with them decide
-        std::lock_guard<std::mutex> lk(g_sqrt.m);
-        uint32_t key;
-        std::memcpy(&key, &L.inv_w, 4);
-        auto it = g_sqrt.bins.find(key);
-        L.nr_sqrt = (L.inv_w > 0 && it != g_sqrt.bins.end() && it->second >= L.smem_bins) ? 1 : 0;
-        // a power-of-two inverse width (0.25 A bins): the product d inv_w is exact, so the rounding to
-        // a bin fuses with it (one FFMA per pair instead of FMUL + FADD)
-        int e = 0;
-        if (L.nr_sqrt && std::frexp(L.inv_w, &e) == 0.5f) L.nr_sqrt = 2;
-    }
+    L.nr_sqrt = pair_sqrt_mode(L.inv_w, L.smem_bins);
     // double-buffered staging when the launch was given the room for it
     L.stages = smem >= pairhist_layout_bytes(L.smem_rows, L.smem_bins, L.weighted != 0, tile, L.dreg != 0, 2) ? 2 : 1;
     if (tile == 1024) launch_tile<1024>(L, grid, smem, s);

@@ -148,5 +148,8 @@ void pairhist_launch(const PairLaunch& L, int tile, int grid, size_t smem, cudaS
 // when planning, outside stream capture).  Launches over at most `bins` bins of a verified width then
 // take the Newton-Raphson root.  Returns whether the width is verified.
 bool pair_sqrt_prepare(float inv_w, int bins);
+// The root launches over at most `bins` bins of this width may take: 0 the correctly rounded one, 1 the
+// Newton-Raphson root (verified), 2 that with a power-of-two inv_w.
+int pair_sqrt_mode(float inv_w, int bins);
 
 }  // namespace ausaxs_b200

@@ -79,13 +79,67 @@ __global__ void radius_kernel(const float4* a, int na, const float4* w, int nw, 
     if ((threadIdx.x & 31) == 0 && r2 > 0) atomicMax(&st->r2, static_cast<unsigned long long>(__double_as_longlong(r2)));
 }
 
-__global__ void to_dense_kernel(const float4* in, float4* out, int n, const int32_t* ff_to_type) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+// Dense copy of the points (w = dense type; type map null: w already is), and the points of each
+// type in every chunk of kTypedChunk points.
+__global__ void __launch_bounds__(kTypedChunk) dense_count_kernel(const float4* in, float4* out, int n, const int32_t* ff_to_type,
+                                                                  int32_t* counts) {
+    __shared__ int s_count[16];
+    if (threadIdx.x < 16) s_count[threadIdx.x] = 0;
+    __syncthreads();
+    const int i = blockIdx.x * kTypedChunk + threadIdx.x;
+    if (i < n) {
         float4 v = in[i];
-        int t = __float_as_int(v.w);
-        int d = (t > kExv && t < kNff) ? ff_to_type[t] : 0;
+        const int t = __float_as_int(v.w);
+        const int d = !ff_to_type ? t : ((t > kExv && t < kNff) ? ff_to_type[t] : 0);
         v.w = __int_as_float(d);
-        out[i] = v;
+        if (out) out[i] = v;
+        const unsigned same = __match_any_sync(__activemask(), d);
+        if ((threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&s_count[d], __popc(same));
+    }
+    __syncthreads();
+    if (threadIdx.x < 16) counts[blockIdx.x * 16 + threadIdx.x] = s_count[threadIdx.x];
+}
+
+// The lists of points by type, ascending index (a stable partition): chunk c writes its points after
+// those of the earlier chunks.  w of a listed point is its index.
+__global__ void __launch_bounds__(kTypedChunk) typed_scatter_kernel(const float4* dense, int n, TypedOut o, const int32_t* counts) {
+    constexpr int kW = kTypedChunk / 32;
+    __shared__ int s_warp[kW + 1][16];  // points of a type in the warps before
+    __shared__ int s_base[16];          // ... in the chunks before
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x < 16 * (kW + 1)) (&s_warp[0][0])[threadIdx.x] = 0;
+    __syncthreads();
+    const int i = blockIdx.x * kTypedChunk + threadIdx.x;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    int d = 15, rank = 0;
+    if (i < n) {
+        v = dense[i];
+        d = __float_as_int(v.w);
+    }
+    const unsigned same = __match_any_sync(0xffffffffu, d);
+    rank = __popc(same & ((1u << lane) - 1u));
+    if (rank == 0) s_warp[warp + 1][d] = __popc(same);
+    if (warp < o.types) {  // one warp per type adds up the earlier chunks (kW warps, at most 15 types)
+        int b = 0;
+        for (int c = lane; c < static_cast<int>(blockIdx.x); c += 32) b += counts[c * 16 + warp];
+        b = __reduce_add_sync(0xffffffffu, b);
+        if (lane == 0) s_base[warp] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x < o.types)
+        for (int w = 1; w <= kW; ++w) s_warp[w][threadIdx.x] += s_warp[w - 1][threadIdx.x];
+    __syncthreads();
+    if (i < n) {
+        const int at = o.start[d] + s_base[d] + s_warp[warp][d] + rank;
+        o.pts[at] = make_float4(v.x, v.y, v.z, __int_as_float(i));
+        if (o.pos) o.pos[i] = at;
+    }
+    // points with an index below every multiple of 256 of the chunk (and below n after the last)
+    constexpr int kSub = kTypedChunk / kTypedPre;
+    for (int k = threadIdx.x; k < kSub * o.types; k += kTypedChunk) {
+        const int t = k / kSub, sub = k - t * kSub;
+        const int c = blockIdx.x * kSub + sub;
+        if (c < o.pre_stride) o.pre[t * o.pre_stride + c] = s_base[t] + s_warp[sub * (kTypedPre / 32)][t];
     }
 }
 
@@ -111,11 +165,12 @@ void radius_launch(const float4* a, int na, const float4* w, int nw, const float
     radius_kernel<<<(int)blocks, 256, 0, s>>>(a, na, w, nw, x, nx, st);
 }
 
-void to_dense_launch(const float4* in, float4* out, int n, const int32_t* ff_to_type, int sm_count, cudaStream_t s) {
+void typed_lists_launch(const float4* in, float4* dense, int n, const int32_t* ff_to_type, const TypedOut& o, int32_t* counts,
+                        cudaStream_t s) {
     if (n <= 0) return;
-    int blocks = (n + 255) / 256;
-    if (blocks > sm_count * 4) blocks = sm_count * 4;
-    to_dense_kernel<<<blocks, 256, 0, s>>>(in, out, n, ff_to_type);
+    const int chunks = typed_chunks(n);
+    dense_count_kernel<<<chunks, kTypedChunk, 0, s>>>(in, dense, n, ff_to_type, counts);
+    typed_scatter_kernel<<<chunks, kTypedChunk, 0, s>>>(dense ? dense : in, n, o, counts);
 }
 
 void set_type_launch(float4* p, int n, int32_t value, int sm_count, cudaStream_t s) {

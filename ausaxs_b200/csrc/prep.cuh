@@ -19,7 +19,25 @@ void census_launch(const float4* p, int n, int ff_typed, PrepStats* st, int sm_c
 // (every pair distance is at most twice it).
 void radius_launch(const float4* a, int na, const float4* w, int nw, const float4* x, int nx, PrepStats* st,
                    int sm_count, cudaStream_t s);
-void to_dense_launch(const float4* in, float4* out, int n, const int32_t* ff_to_type, int sm_count, cudaStream_t s);
+
+// Lists of a point set by type: the points of dense type t at pts[start[t] ...] in ascending index, w =
+// the index (int bits); pre[t * pre_stride + c] = points of type t with an index below kTypedPre * c.
+constexpr int kTypedChunk = 1024;
+constexpr int kTypedPre = 256;
+struct TypedOut {
+    float4* pts;
+    int32_t* pre;
+    int32_t* pos;        // position of every point in pts, or null
+    int32_t types;
+    int32_t pre_stride;  // typed_pre_stride(n)
+    int32_t start[16];
+};
+inline int typed_chunks(int n) { return (n + kTypedChunk - 1) / kTypedChunk; }
+inline int typed_pre_stride(int n) { return (n + kTypedPre - 1) / kTypedPre; }
+// dense (w = dense type through ff_to_type; in already dense: both null) and the lists, two kernels;
+// counts: typed_chunks(n) * 16 ints of scratch
+void typed_lists_launch(const float4* in, float4* dense, int n, const int32_t* ff_to_type, const TypedOut& o, int32_t* counts,
+                        cudaStream_t s);
 void set_type_launch(float4* p, int n, int32_t value, int sm_count, cudaStream_t s);
 float ordered_to_float(unsigned int o);
 
