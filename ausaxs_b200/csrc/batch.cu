@@ -44,6 +44,8 @@ struct PointsItem {
     float4* raw_a;
     float4* dense_a;
     float4* raw_w;
+    float4* typed;       // the atoms' lists by type, and every atom's place in them
+    const int32_t* pos;
 };
 
 __device__ __forceinline__ bool finite3(const float4& v) { return isfinite(v.x) && isfinite(v.y) && isfinite(v.z); }
@@ -69,6 +71,8 @@ __global__ void set_points_kernel(const PointsItem* items, int n, const float4* 
             it.raw_a[k] = v;
             const float dense_type = it.dense_a[k].w;
             it.dense_a[k] = make_float4(v.x, v.y, v.z, dense_type);
+            const int at = it.pos[k];
+            it.typed[at] = make_float4(v.x, v.y, v.z, it.typed[at].w);
         }
         for (long long k = first; k < it.nw; k += stride) {
             const float4 v = waters[it.w0 + k];
@@ -96,12 +100,14 @@ struct Batch {
         PairLaunch L{};
         int tile = 256, grid = 0;
         size_t smem = 0;
+        PackLaunch K{};  // the one-atomic-per-pair kernel instead
+        int shape = -1;
     };
     std::vector<Launch> launches;
     int choice = -1;
     // misc: tile counters [0, 16), overflow [16] (set from [24] at the start of every profile), q values
     // recomputed in FP64 [20], points rejected by the last set_points [24] (kept across profiles)
-    DevBuf jobs, misc, zero, fin, args;
+    DevBuf jobs, outs, misc, zero, fin, args;
     DevBuf qfactors;      // the per-q factor table every structure's transform reads
     DebyeArgs qf_args{};  // q and parameters of the table
     std::vector<long long> a_off, w_off;  // creation offsets of the concatenated atoms and waters
@@ -171,7 +177,7 @@ struct Batch {
             const int64_t nx = grid ? xoff[i + 1] - xoff[i] : 0;
             if (na < 0 || nw < 0 || nx < 0 || na > INT32_MAX || nw > INT32_MAX || nx > INT32_MAX)
                 throw Error{AUSAXS_ERR_ARGUMENT, "bad offsets"};
-            arena_bytes += 2 * pts(na) + pts(nw) + pts(nx) + 256;
+            arena_bytes += 2 * pts(na) + pts(nw) + pts(nx) + 256 + align_up(Structure::typed_bytes((int)na), 256);
         }
         arena.ensure(arena_bytes);
         a_off.assign(aoff, aoff + n + 1);
@@ -191,6 +197,8 @@ struct Batch {
             take(S->raw_w, pts(nw));
             take(S->raw_x, pts(nx));
             take(S->meta, 256);
+            take(S->typed, align_up(Structure::typed_bytes((int)na), 256));
+            S->want_pos = true;
             S->load_begin(atoms ? atoms + 4 * aoff[i] : nullptr, (int)na, waters ? waters + 4 * woff[i] : nullptr,
                           (int)nw, grid && exv ? exv + 4 * xoff[i] : nullptr, (int)nx, 1, host, h_stats + i,
                           d_stats.as<PrepStats>() + i);
@@ -241,9 +249,79 @@ struct Batch {
 
     std::tuple<int, long long, int, int> shape() const { return {(int)items.size(), pairs, max_nb, ctx->sm_count}; }
 
+    // the candidate's launches of the one-atomic-per-pair kernel (its tile sizes are the inner tiles, its row
+    // classes one-row and multi-row passes); false where a structure's plan does not take that kernel
+    bool build_packed(const Candidate& c) {
+        for (auto& S : items)
+            if (!S->plan.packed && S->plan.pairs > 0) return false;
+        const int nr = pair_sqrt_mode(items[order[0]]->plan.inv_w, max_nb);
+        if (!nr) return false;
+        const bool grid = cfg.manager == AUSAXS_MANAGER_FFGRID;
+        std::vector<Launch> found;
+        std::vector<PackTable> tables;
+        for (int b = 0; b < 2; ++b)
+            for (int cls = 0; cls < 2; ++cls) {
+                if (c.by_class == 0 && cls == 1) continue;
+                auto table = [&](int shape, bool joint, PackTable& T) {
+                    PackLaunch K{};
+                    K.nr = nr;
+                    K.offsets = cfg.weighted_bins ? 1 : 0;
+                    K.tile_j = b ? c.tile_large : c.tile_small;
+                    T = PackTable{};
+                    for (int i : order) {
+                        const Structure& S = *items[i];
+                        const int biggest = std::max({S.n_a, S.n_w, grid ? S.n_x : 0});
+                        if ((c.tile_small != c.tile_large && biggest >= c.threshold ? 1 : 0) != b) continue;
+                        append_pack_jobs(S.plan, kPackShapes[shape].outer(), joint, K, T, false, c.by_class ? cls : -1);
+                    }
+                    return K;
+                };
+                Launch La;
+                PackTable T;
+                La.K = table(0, false, T);
+                if (T.jobs.empty()) continue;
+                La.shape = pack_shape(La.K);
+                if (La.shape < 0) return false;
+                // one group per structure where its rows cost no CTA per SM
+                const int per_sm = pack_ctas_per_sm(La.shape, La.K);
+                const PackLaunch joint = table(La.shape, true, T);
+                La.K = pack_ctas_per_sm(La.shape, joint) >= per_sm ? joint : table(La.shape, false, T);
+                La.grid = (int)std::min<long long>((long long)ctx->sm_count * per_sm, std::max<long long>(1, La.K.total_tiles));
+                La.K.tile_counter = misc.as<unsigned long long>() + found.size();
+                La.K.overflow = overflow();
+                found.push_back(La);
+                tables.push_back(T);
+            }
+        size_t n_jobs = 0, n_out = 0;
+        for (auto& T : tables) n_jobs += T.jobs.size(), n_out += T.out.size();
+        jobs.ensure(sizeof(PackJob) * std::max<size_t>(1, n_jobs));
+        outs.ensure(sizeof(void*) * std::max<size_t>(1, n_out));
+        size_t at = 0, out = 0;
+        for (size_t k = 0; k < found.size(); ++k) {
+            const PackTable& T = tables[k];
+            found[k].K.jobs = jobs.as<PackJob>() + at;
+            found[k].K.out = outs.as<unsigned long long*>() + out;
+            AUSAXS_CUDA(cudaMemcpy(jobs.as<PackJob>() + at, T.jobs.data(), sizeof(PackJob) * T.jobs.size(), cudaMemcpyHostToDevice));
+            AUSAXS_CUDA(cudaMemcpy(outs.as<unsigned long long*>() + out, T.out.data(), sizeof(void*) * T.out.size(),
+                                   cudaMemcpyHostToDevice));
+            at += T.jobs.size();
+            out += T.out.size();
+        }
+        launches = found;
+        return true;
+    }
+
     // job tables and launch shapes of one candidate
     void build(int c_idx) {
         const Candidate& c = kCandidates[c_idx];
+        if (exec) {
+            cudaGraphExecDestroy(exec);
+            exec = nullptr;
+        }
+        if (build_packed(c)) {
+            choice = c_idx;
+            return;
+        }
         std::vector<PairJob> js[2][3];
         long long tiles[2][3] = {{0, 0, 0}, {0, 0, 0}};
         int rows[2][3] = {{1, 1, 1}, {1, 1, 1}};
@@ -261,10 +339,6 @@ struct Batch {
         size_t n_jobs = 0;
         for (auto& bb : js)
             for (auto& g : bb) n_jobs += g.size();
-        if (exec) {
-            cudaGraphExecDestroy(exec);
-            exec = nullptr;
-        }
         jobs.ensure(sizeof(PairJob) * std::max<size_t>(1, n_jobs));
         launches.clear();
         size_t at = 0;
@@ -312,7 +386,8 @@ struct Batch {
             cudaStream_t sk = k == 0 ? s : side[(k - 1) % 2];
             if (k > 0 && k <= 2) AUSAXS_CUDA(cudaStreamWaitEvent(sk, fork, 0));
             const Launch& La = launches[k];
-            pairhist_launch(La.L, La.tile, La.grid, La.smem, sk);
+            if (La.shape >= 0) pack_launch(La.K, La.shape, La.grid, sk);
+            else pairhist_launch(La.L, La.tile, La.grid, La.smem, sk);
             C.check_launch("pairhist");
         }
         for (int k = 1; k <= std::min(2, n - 1); ++k) {
@@ -533,7 +608,7 @@ struct Batch {
             for (int i = 0; i < n; ++i) {
                 Structure& S = *items[i];
                 v[i] = {a_off[i] - a_off[0], S.n_a, w_off[i] - w_off[0], S.n_w,
-                        S.raw_a.as<float4>(), S.dense_a.as<float4>(), S.raw_w.as<float4>()};
+                        S.raw_a.as<float4>(), S.dense_a.as<float4>(), S.raw_w.as<float4>(), S.typed.as<float4>(), S.typed_pos()};
             }
             points_items.ensure(sizeof(PointsItem) * n);
             AUSAXS_CUDA(cudaMemcpy(points_items.p, v.data(), sizeof(PointsItem) * n, cudaMemcpyHostToDevice));

@@ -122,6 +122,28 @@ static size_t typed_off_pos(int n) { return typed_off_counts(n) + align_up((size
 size_t Structure::typed_bytes(int n) { return typed_off_pos(n) + align_up((size_t)std::max(1, n) * 4, 256); }
 int32_t* Structure::typed_pos() const { return typed.as<int32_t>(typed_off_pos(n_a)); }
 
+TypedSet typed_lists(const float4* in, float4* dense, int n, const int32_t* ff_to_type, int types, const int* count, char* mem,
+                     bool want_pos, cudaStream_t s) {
+    TypedOut o{};
+    o.pts = reinterpret_cast<float4*>(mem);
+    o.pre = reinterpret_cast<int32_t*>(mem + typed_off_pre(n));
+    o.pos = want_pos ? reinterpret_cast<int32_t*>(mem + typed_off_pos(n)) : nullptr;
+    o.types = types;
+    o.pre_stride = typed_pre_stride(n);
+    TypedSet set{};
+    set.pts = o.pts;
+    set.pre = o.pre;
+    set.pre_stride = o.pre_stride;
+    set.types = types;
+    for (int t = 0, at = 0; t < types; ++t) {
+        set.start[t] = o.start[t] = at;
+        set.count[t] = count[t];
+        at += count[t];
+    }
+    typed_lists_launch(in, dense, n, ff_to_type, o, reinterpret_cast<int32_t*>(mem + typed_off_counts(n)), s);
+    return set;
+}
+
 void Structure::load_end(const PrepStats& st) {
     Ctx& C = *ctx;
     cudaStream_t s = C.stream;
@@ -166,24 +188,8 @@ void Structure::load_end(const PrepStats& st) {
     if (ff_typed) {
         dense_a.ensure(align_up(std::max(1, n_a) * 16, 256));
         typed.ensure(typed_bytes(n_a));
-        lists = TypedSet{};
-        lists.pts = typed.as<float4>();
-        lists.pre = typed.as<int32_t>(typed_off_pre(n_a));
-        lists.pre_stride = typed_pre_stride(n_a);
-        lists.types = T;
-        TypedOut o{};
-        o.pts = typed.as<float4>();
-        o.pre = typed.as<int32_t>(typed_off_pre(n_a));
-        o.pos = want_pos ? typed_pos() : nullptr;
-        o.types = T;
-        o.pre_stride = lists.pre_stride;
-        for (int t = 0, at = 0; t < T; ++t) {
-            lists.start[t] = o.start[t] = at;
-            lists.count[t] = type_count[t];
-            at += type_count[t];
-        }
-        typed_lists_launch(raw_a.as<float4>(), dense_a.as<float4>(), n_a, meta.as<int32_t>(kNff * 4), o,
-                           typed.as<int32_t>(typed_off_counts(n_a)), s);
+        lists = typed_lists(raw_a.as<float4>(), dense_a.as<float4>(), n_a, meta.as<int32_t>(kNff * 4), T, type_count,
+                            typed.as<char>(), want_pos, s);
         C.check_launch("typed lists");
         if (n_a > 0) C.launches += 1;  // two kernels
     }
@@ -257,7 +263,8 @@ void append_pair_jobs(const Plan& P, int tile, bool by_class, std::vector<PairJo
     }
 }
 
-void append_pack_jobs(const Plan& P, int outer, bool joint, PackLaunch& L, PackTable& T, bool skip_lattice) {
+void append_pack_jobs(const Plan& P, int outer, bool joint, PackLaunch& L, PackTable& T, bool skip_lattice,
+                      int row_class) {
     auto up = [](int n, int d) { return (n + d - 1) / d; };
     const size_t first = T.jobs.size();
     std::vector<unsigned long long*> sums;  // the open group's offset sums
@@ -280,6 +287,7 @@ void append_pack_jobs(const Plan& P, int outer, bool joint, PackLaunch& L, PackT
     for (const JobSpec& j : P.specs) {
         if (skip_lattice && j.lattice) continue;
         const bool pair_rows = j.rmode == kRowPair;
+        if (row_class >= 0 && (j.rmode != kRowSingle) != (row_class == 1)) continue;
         // the largest row's share of a job's pairs (outer points have the composition of the whole structure)
         const double share = j.rows == 1 ? 1.0 : P.row_share;
         for (int t = 0; t < (pair_rows ? j.typed->types : 1); ++t) {
@@ -304,7 +312,7 @@ void append_pack_jobs(const Plan& P, int outer, bool joint, PackLaunch& L, PackT
             p.b_base = j.b_base;
             p.tail_end = j.tail_end >= 0 ? j.tail_end : j.nbp;
             p.tail_from_outer = j.tail_from_outer >= 0 ? j.tail_from_outer : j.self;
-            p.seg_pairs = pack_segment_pairs(P.nb, share);
+            p.seg_pairs = pack_segment_pairs(j.spread_bins > 0 ? std::min(j.spread_bins, P.nb) : P.nb, share);
             p.cnt_row = rows;
             for (int r = 0; r < p.rows; ++r) T.out.push_back(j.counts + (size_t)(pair_rows ? r * P.T + t : r) * P.nb);
             rows += p.rows;
@@ -435,7 +443,7 @@ static double pack_tiles(const std::vector<JobSpec>& specs, int outer, int tile_
     return n;
 }
 
-bool choose_pack(const Plan& P, int sm_count, PackLaunch& L, int& shape, int& grid, PackTable& T) {
+bool choose_pack(const Plan& P, int sm_count, PackLaunch& L, int& shape, int& grid, PackTable& T, bool may_join) {
     L = PackLaunch{};
     L.nr = pair_sqrt_mode(P.inv_w, P.nb);
     L.offsets = P.weighted;
@@ -472,9 +480,11 @@ bool choose_pack(const Plan& P, int sm_count, PackLaunch& L, int& shape, int& gr
     // one group where its rows cost no CTA per SM: a CTA then flushes once, not at every change of job
     L = table(shape, tile_j, false);
     const int per_sm = pack_ctas_per_sm(shape, L);
-    const PackLaunch joint = table(shape, tile_j, true);
-    if (pack_ctas_per_sm(shape, joint) >= per_sm) L = joint;
-    else L = table(shape, tile_j, false);
+    if (may_join) {
+        const PackLaunch joint = table(shape, tile_j, true);
+        if (pack_ctas_per_sm(shape, joint) >= per_sm) L = joint;
+        else L = table(shape, tile_j, false);
+    }
     grid = (int)std::min<long long>((long long)sm_count * per_sm, std::max<long long>(1, L.total_tiles));
     return true;
 }

@@ -56,6 +56,10 @@ struct TypedSet {
     int start[16] = {}, count[16] = {};
 };
 
+// The lists of `in` (typed_lists_launch) in mem (Structure::typed_bytes(n)); count: points of each type.
+TypedSet typed_lists(const float4* in, float4* dense, int n, const int32_t* ff_to_type, int types, const int* count, char* mem,
+                     bool want_pos, cudaStream_t s);
+
 // One pass of pair binning of a structure before it is cut into tiles: the two point sets, the
 // rows it increments, and where its global accumulators live.
 struct JobSpec {
@@ -71,6 +75,7 @@ struct JobSpec {
     int a_base = 0, b_base = 0, tail_end = -1, tail_from_outer = -1;
     int mult = 1;  // multiplicity of every pair (PairJob::mult)
     bool lattice = false;  // the plan bins this pass with the lattice kernel (the structure's own launches)
+    int spread_bins = 0;   // bins the distances spread over, about (0: all of the plan's)
     const TypedSet* typed = nullptr;  // atom-atom passes: the inner atoms' lists (append_pack_jobs)
 };
 
@@ -235,18 +240,20 @@ void append_pair_jobs(const Plan& P, int tile, bool by_class, std::vector<PairJo
 // The same passes as jobs of the one-atomic-per-pair kernel, atom-atom passes cut by inner type, for
 // outer tiles of `outer` and L.tile_j inner points.  The jobs and the accumulators they flush to are
 // appended; L's row, sum and bin maxima, job and tile counts grow with them.  joint: one group for all of the
-// plan's jobs, else a group per job.
+// plan's jobs, else a group per job.  row_class 0: only one-row passes, 1: only multi-row ones, -1: all.
 struct PackTable {
     std::vector<PackJob> jobs;
     std::vector<unsigned long long*> out;
     int groups = 0;
 };
-void append_pack_jobs(const Plan& P, int outer, bool joint, PackLaunch& L, PackTable& T, bool skip_lattice = false);
+void append_pack_jobs(const Plan& P, int outer, bool joint, PackLaunch& L, PackTable& T, bool skip_lattice = false,
+                      int row_class = -1);
 
 // Shape of a launch of the one-atomic-per-pair kernel over the plan's passes, and its jobs; false where
 // the kernel does not apply: an inverse width whose root is not verified, or more rows and bins than
 // fit on chip.
-bool choose_pack(const Plan& P, int sm_count, PackLaunch& L, int& shape, int& grid, PackTable& T);
+// joint: may put all jobs in one group.
+bool choose_pack(const Plan& P, int sm_count, PackLaunch& L, int& shape, int& grid, PackTable& T, bool joint = true);
 
 // Clears n device ranges of u64 words in one launch (table in device memory); a range with a
 // source is set to the source's words instead.

@@ -23,6 +23,7 @@
 // persistent grid, so the block scheduler hands SMs to a small move as soon as running CTAs finish
 // instead of after a large move's whole launch.
 #include <algorithm>
+#include <cstring>
 #include <array>
 #include <chrono>
 #include <cmath>
@@ -43,7 +44,18 @@ struct Pose {
 
 // x <- R x + t in FP64 from the body's original coordinates (Body::rotate then Body::translate,
 // source/core/data/Body.cpp:135-156, composed on the host), rounded to float
-__global__ void transform_kernel(const float4* __restrict__ src, float4* __restrict__ dst, int n, Pose p) {
+struct MovedSet {
+    const float4* src;
+    float4* dst;
+    int n;
+};
+struct MovedSets {
+    MovedSet set[3];  // a body's atoms, their lists by type, its waters
+};
+__global__ void transform_kernel(MovedSets m, Pose p) {
+    const float4* __restrict__ src = m.set[blockIdx.y].src;
+    float4* __restrict__ dst = m.set[blockIdx.y].dst;
+    const int n = m.set[blockIdx.y].n;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 v = src[i];
         const double x = v.x, y = v.y, z = v.z;
@@ -108,6 +120,7 @@ struct Assembly {
     int B = 0, N = 0, W = 0;
     std::vector<int> a_off, w_off;
     std::vector<std::array<double, 3>> c0;  // body centroids of the original coordinates
+    std::vector<double> radius;             // about them
     std::vector<Pose> pose;
     DevBuf orig, part, tables, io;
     struct Part {
@@ -120,8 +133,15 @@ struct Assembly {
         size_t zero_off = 0;
         int n_zero = 0;
         PairLaunch L{};
+        PackLaunch K{};  // the one-atomic-per-pair kernel instead (packed): a CTA per tile
+        int shape = 0;
         int grid = 0;
     };
+    bool packed = false;
+    DevBuf lists;                    // per body: its atoms' lists by type (Structure::typed's layout), current
+    DevBuf lists_orig;               // and the listed points' original coordinates
+    std::vector<TypedSet> body_lists;
+    std::vector<size_t> list_off;    // byte offset of body k's lists in both
     std::vector<Work> work;  // [B]: moves of body k; [B]: every partial (initial state)
     MasterSum msum{};
     int tile = 256;
@@ -196,6 +216,13 @@ struct Assembly {
                 for (int d = 0; d < 3; ++d) m[d] += atoms[4 * (size_t)i + d];
             for (int d = 0; d < 3; ++d) m[d] = n ? m[d] / n : 0.0;
             c0.push_back(m);
+            double r2 = 0;
+            for (int i = a_off[k]; i < a_off[k + 1]; ++i) {
+                double d2 = 0;
+                for (int d = 0; d < 3; ++d) d2 += (atoms[4 * (size_t)i + d] - m[d]) * (atoms[4 * (size_t)i + d] - m[d]);
+                r2 = std::max(r2, d2);
+            }
+            radius.push_back(std::sqrt(r2));
             Pose id{};
             id.R[0] = id.R[4] = id.R[8] = 1.0;
             pose.push_back(id);
@@ -211,6 +238,7 @@ struct Assembly {
         AUSAXS_CUDA(cudaMemcpyAsync(orig.p, S.atoms_for_pairs(), (size_t)N * 16, cudaMemcpyDeviceToDevice, C.stream));
         if (W) AUSAXS_CUDA(cudaMemcpyAsync(orig.as<char>(align_up(a_bytes, 256)), S.raw_w.p, (size_t)W * 16,
                                            cudaMemcpyDeviceToDevice, C.stream));
+        build_lists(atoms);
         // partial blocks
         size_t off = 0;
         auto add = [&](int kind, int k, int l, int rows) {
@@ -237,6 +265,8 @@ struct Assembly {
             j.wsum = nullptr;
             j.rows = pt.rows;
             const int k = pt.k, l = pt.l;
+            // two compact bodies: their distances spread over little more than the sum of their radii
+            j.spread_bins = std::max(16, (int)(0.7 * (radius[k] + radius[l]) * P.inv_w));
             if (pt.kind == 0) {  // aa: body k atoms outer, body l atoms inner, rows of the full self loop
                 j.A = A + a_off[k];
                 j.na = a_off[k + 1] - a_off[k];
@@ -248,6 +278,7 @@ struct Assembly {
                 j.b_base = a_off[l];
                 j.tail_end = N;
                 j.tail_from_outer = 1;
+                j.typed = &body_lists[l];
             } else if (pt.kind == 1) {  // aw: atoms of k outer, waters of l inner, rows over all waters
                 j.A = A + a_off[k];
                 j.na = a_off[k + 1] - a_off[k];
@@ -274,6 +305,8 @@ struct Assembly {
             return j;
         };
         tile = P.tile;
+        packed = P.packed;
+        PackTable pack_tables;
         std::vector<PairJob> all_jobs;
         std::vector<ZeroRange> all_zero;
         work.resize(B + 1);
@@ -286,6 +319,8 @@ struct Assembly {
             tmp.c = P.c;
             tmp.scale = P.scale;
             tmp.max_group_rows = P.max_group_rows;
+            tmp.row_share = P.row_share;
+            tmp.weighted = P.weighted;
             std::vector<ZeroRange> zr;
             for (const Part& pt : parts) {
                 // every partial with the moved body, its self partials included: the moved coordinates are
@@ -319,6 +354,21 @@ struct Assembly {
             Wk.L.jobs = reinterpret_cast<const PairJob*>(all_jobs.size());  // index, rebased below
             all_jobs.insert(all_jobs.end(), js[0].begin(), js[0].end());
             max_rows = std::max(max_rows, rows[0]);
+            if (packed) {
+                // Short-lived CTAs of one tile each, so that the block scheduler mixes moves (measured: two moves
+                // of a 10,000-atom body of 70,000 2.21 ms against 2.23 with two tiles per CTA and 2.73 with the
+                // two-atomic kernel).
+                PackTable T1;
+                int persistent = 0;
+                packed = choose_pack(tmp, sms, Wk.K, Wk.shape, persistent, T1, false) || tmp.specs.empty();
+                Wk.K.jobs = reinterpret_cast<const PackJob*>(pack_tables.jobs.size());  // indices, rebased below
+                Wk.K.out = reinterpret_cast<unsigned long long* const*>(pack_tables.out.size());
+                pack_tables.jobs.insert(pack_tables.jobs.end(), T1.jobs.begin(), T1.jobs.end());
+                pack_tables.out.insert(pack_tables.out.end(), T1.out.begin(), T1.out.end());
+                Wk.K.tile_counter = Wk.L.tile_counter;
+                Wk.K.overflow = Wk.L.overflow;
+                Wk.K.max_tiles = 1;
+            }
         }
         smem = pairhist_launch_smem(max_rows, nb, false, tile);
         // two thread groups per CTA (pairhist_groups): a tile of a move's short-lived CTAs takes half
@@ -339,7 +389,15 @@ struct Assembly {
             ptr_off[s] = toff;
             toff += align_up(sizeof(void*) * std::max<size_t>(1, ptrs[s].size()), 256);
         }
+        const size_t pack_jobs_off = toff, pack_out_off = toff + align_up(sizeof(PackJob) * pack_tables.jobs.size(), 256);
+        toff = pack_out_off + align_up(sizeof(void*) * pack_tables.out.size(), 256);
         tables.ensure(toff);
+        if (packed) {
+            AUSAXS_CUDA(cudaMemcpy(tables.as<char>(pack_jobs_off), pack_tables.jobs.data(), sizeof(PackJob) * pack_tables.jobs.size(),
+                                   cudaMemcpyHostToDevice));
+            AUSAXS_CUDA(cudaMemcpy(tables.as<char>(pack_out_off), pack_tables.out.data(), sizeof(void*) * pack_tables.out.size(),
+                                   cudaMemcpyHostToDevice));
+        }
         AUSAXS_CUDA(cudaMemcpy(tables.p, all_jobs.data(), sizeof(PairJob) * all_jobs.size(), cudaMemcpyHostToDevice));
         AUSAXS_CUDA(cudaMemcpy(tables.as<char>(jobs_bytes), all_zero.data(), sizeof(ZeroRange) * all_zero.size(),
                                cudaMemcpyHostToDevice));
@@ -355,6 +413,11 @@ struct Assembly {
             const long long need = (Wk.L.total_tiles + kServeTilesPerCta - 1) / kServeTilesPerCta;
             Wk.grid = (int)std::max<long long>(1, std::min<long long>(need, (long long)INT32_MAX));
             (void)per_sm;
+            if (packed) {
+                Wk.K.jobs = tables.as<PackJob>(pack_jobs_off) + reinterpret_cast<size_t>(Wk.K.jobs);
+                Wk.K.out = tables.as<unsigned long long*>(pack_out_off) + reinterpret_cast<size_t>(Wk.K.out);
+                Wk.grid = (int)std::max<long long>(1, std::min<long long>(Wk.K.total_tiles, (long long)INT32_MAX));
+            }
         }
         // pair evaluations of a move of each body (the body against the rest, and its own pairs)
         const long long NW = (long long)N + W;
@@ -404,13 +467,41 @@ struct Assembly {
         enqueue_pairs(work[B]);
         AUSAXS_CUDA(cudaStreamSynchronize(C.stream));
         footprint = S.raw_a.n + S.raw_w.n + S.raw_x.n + S.dense_a.n + S.meta.n + P.dev.n + orig.n + part.n + tables.n +
-                    io.n + C.stats.n;
+                    io.n + C.stats.n + S.typed.n + lists.n + lists_orig.n;
+    }
+
+    // every body's atom lists by type (of the loaded, dense coordinates) and their original coordinates
+    void build_lists(const float* atoms) {
+        size_t at = 0;
+        for (int k = 0; k < B; ++k) {
+            list_off.push_back(at);
+            at += align_up(Structure::typed_bytes(a_off[k + 1] - a_off[k]), 256);
+        }
+        lists.ensure(std::max<size_t>(at, 256));
+        lists_orig.ensure(std::max<size_t>(at, 256));
+        body_lists.resize(B);
+        for (int k = 0; k < B; ++k) {
+            const int n = a_off[k + 1] - a_off[k];
+            int count[16] = {};
+            for (int i = a_off[k]; i < a_off[k + 1]; ++i) {
+                int32_t f;
+                std::memcpy(&f, atoms + 4 * (size_t)i + 3, 4);
+                ++count[S.ff_to_type[f]];  // validated by the load
+            }
+            body_lists[k] = typed_lists(S.atoms_for_pairs() + a_off[k], nullptr, n, nullptr, S.T, count, lists.as<char>(list_off[k]),
+                                        false, C.stream);
+            C.check_launch("typed lists");
+        }
+        AUSAXS_CUDA(cudaMemcpyAsync(lists_orig.p, lists.p, at, cudaMemcpyDeviceToDevice, C.stream));
     }
 
     void enqueue_pairs(const Work& Wk) {
         zero_ranges_launch(tables.as<ZeroRange>(Wk.zero_off), Wk.n_zero, C.stream);
         C.check_launch("zero");
-        if (Wk.L.n_jobs > 0) {
+        if (packed && Wk.K.n_jobs > 0) {
+            pack_launch(Wk.K, Wk.shape, Wk.grid, C.stream);
+            C.check_launch("pairpack");
+        } else if (Wk.L.n_jobs > 0) {
             pairhist_launch(Wk.L, tile, Wk.grid, smem, C.stream);
             C.check_launch("pairhist");
         }
@@ -423,12 +514,12 @@ struct Assembly {
             compose(pose[body], R, t);
             const int na = a_off[body + 1] - a_off[body], nw = w_off[body + 1] - w_off[body];
             const size_t a_bytes = align_up((size_t)std::max(1, N) * 16, 256);
-            if (na)
-                transform_kernel<<<std::min(1024, (na + 255) / 256), 256, 0, s>>>(
-                    orig.as<float4>() + a_off[body], const_cast<float4*>(S.atoms_for_pairs()) + a_off[body], na, pose[body]);
-            if (nw)
-                transform_kernel<<<std::min(1024, (nw + 255) / 256), 256, 0, s>>>(
-                    orig.as<float4>(a_bytes) + w_off[body], S.raw_w.as<float4>() + w_off[body], nw, pose[body]);
+            MovedSets m{};
+            m.set[0] = {orig.as<float4>() + a_off[body], const_cast<float4*>(S.atoms_for_pairs()) + a_off[body], na};
+            m.set[1] = {lists_orig.as<float4>(list_off[body]), lists.as<float4>(list_off[body]), na};
+            m.set[2] = {orig.as<float4>(a_bytes) + w_off[body], S.raw_w.as<float4>() + w_off[body], nw};
+            const int most = std::max({1, na, nw});
+            transform_kernel<<<dim3(std::min(1024, (most + 255) / 256), 3), 256, 0, s>>>(m, pose[body]);
             C.check_launch("transform");
             enqueue_pairs(work[body]);
         }
