@@ -515,7 +515,6 @@ struct Batch {
         AUSAXS_CUDA(cudaEventRecordWithFlags(pair_t1, s, cudaEventRecordExternal));
         ff_finalize_batch_launch(fin.as<FinalizeFF>(), (int)items.size(), max_nb, s);
         ctx->check_launch("finalize");
-        ctx->launches += 1;  // two kernels
         if (x.on) {
             if (!debye_x_enqueue(x.plan, q, s)) throw Error{AUSAXS_ERR_CUDA, "cannot launch the tensor-core Debye transform"};
             ctx->check_launch("debye_x");

@@ -706,7 +706,8 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
         plan_groups(P, base, C);
     }
 
-    // finalisation
+    // finalisation (its counter is cleared with the accumulators, or here where they are not)
+    AUSAXS_CUDA(cudaMemsetAsync(base + P.off_maxbin, 0, 256, C.stream));
     auto cnt = [&](int k) { return reinterpret_cast<const unsigned long long*>(base + slot_cnt[k]); };
     auto ds = [&](int k) { return reinterpret_cast<const unsigned long long*>(base + slot_ds[k]); };
     if (mt) {
@@ -729,6 +730,7 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
         F.scale = P.scale;
         F.weighted = weighted;
         F.max_bin = reinterpret_cast<int32_t*>(base + P.off_maxbin);
+        F.done = reinterpret_cast<unsigned*>(base + P.off_maxbin) + 16;
         F.H = reinterpret_cast<double*>(base + P.off_H);
         F.tot = reinterpret_cast<double*>(base + P.off_tot);
         F.d_axis = reinterpret_cast<double*>(base + P.off_d);
@@ -760,6 +762,7 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
         F.scale = P.scale;
         F.weighted = weighted;
         F.max_bin = reinterpret_cast<int32_t*>(base + P.off_maxbin);
+        F.done = reinterpret_cast<unsigned*>(base + P.off_maxbin) + 16;
         F.H = reinterpret_cast<double*>(base + P.off_H);
         F.tot = reinterpret_cast<double*>(base + P.off_tot);
         F.d_axis = reinterpret_cast<double*>(base + P.off_d);
@@ -830,7 +833,6 @@ void Structure::enqueue_histogram(const ausaxs_hist_config& cfg) {
     if (mt) mt_finalize_launch(P.fin_mt, s);
     else ff_finalize_launch(P.fin_ff, s);
     C.check_launch("finalize");
-    C.launches += 1;  // finalize is two kernels
     C.time_end(1, evf);
 }
 

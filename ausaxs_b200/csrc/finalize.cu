@@ -30,112 +30,137 @@ __device__ __forceinline__ double weighted_bin(double dsum, double count, int b,
     return (static_cast<double>(dsum == 0) * dv + dsum) / static_cast<double>((cnt == 0) + cnt);
 }
 
-__device__ void ff_maxbin_body(const FinalizeFF& F) {
-    const int T = F.T;
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicMax(F.max_bin, 10);  // minimum size (HistogramManagerMT.cpp:48)
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < F.nb; b += gridDim.x * blockDim.x) {
-        unsigned long long tot = 0;
-        for (int r = 0; r < T * T; ++r) tot += 2ull * F.cnt_aa[static_cast<size_t>(r) * F.nb + b];
-        for (int t = 0; t < T; ++t) tot += F.cnt_aw[static_cast<size_t>(t) * F.nb + b];
-        tot += 2ull * F.cnt_ww[b];
-        if (b == 0) tot += static_cast<unsigned long long>(F.n_a) + F.n_w;
-        bool nz = tot != 0;
-        if (F.kind == kKindGrid) {
-            unsigned long long xx = 2ull * F.cnt_xx[b] + (b == 0 ? F.n_x : 0);
-            nz = nz || xx != 0 || F.cnt_wx[b] != 0;
-        }
-        if (nz && b >= 10) atomicMax(F.max_bin, b + 1);
+// Post-processing takes one launch: the blocks write the rows of their bins and raise max_bin, and the
+// block that finishes last forms the distance axes, which depend on it (their bin width is
+// (max_bin * width) / max_bin, bins beyond it are zero).  Bound: the latency of one round of loads; a
+// thread per (bin, row slice) has all of its loads in flight at once (two launches with a thread per bin
+// and serial row loads took 7 + 17 us at any size, this one 5).
+constexpr int kFinBins = 32, kFinSlices = 8;
+
+// Whether this block is the last of `blocks` of its structure to get here; what the others wrote is then
+// visible (read it past L1).  The counter returns to 0 for the next launch.
+__device__ bool last_block(unsigned* done, unsigned blocks) {
+    __shared__ bool s_last;
+    __threadfence();
+    __syncthreads();
+    const bool first = threadIdx.x == 0 && threadIdx.y == 0;
+    if (first) {
+        const unsigned n = atomicAdd(done, 1u);
+        s_last = n + 1 == blocks;
+        if (s_last) *done = 0;
     }
+    __syncthreads();
+    __threadfence();
+    return s_last;
 }
 
-__device__ void ff_rows_body(const FinalizeFF& F) {
+__device__ void ff_finalize_body(const FinalizeFF& F, unsigned blocks) {
+    __shared__ unsigned long long s_n[3][kFinSlices][kFinBins];  // aa pairs, aw pairs, ax pairs of the slice's types
     const int T = F.T;
-    const int mb = *F.max_bin;
-    const double width = (static_cast<double>(mb) * F.bin_width) / mb;  // Axis(0, mb*width, mb).width()
-    const int R = ff_rows(T);
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < F.nb; b += gridDim.x * blockDim.x) {
-        const size_t nb = F.nb;
-        if (b >= mb) {
-            for (int r = 0; r < R; ++r) F.H[r * nb + b] = 0;
-            F.tot[b] = 0;
-            F.d_axis[b] = 0;
-            if (F.d_axis_ax) F.d_axis_ax[b] = 0;
-            if (F.d_axis_xx) F.d_axis_xx[b] = 0;
-            continue;
-        }
-        // atom-atom rows: factor 2, self terms (ff, ff, 0) += atoms of that type
-        unsigned long long n_aa = 0, tot = 0;
-        double xx_sum = 0;
-        for (int ta = 0; ta < T; ++ta) {
-            double ax_sum = 0;
+    const size_t nb = F.nb;
+    const int lane = threadIdx.x, slice = threadIdx.y;
+    const int b = blockIdx.x * kFinBins + lane;
+    const bool grid = F.kind == kKindGrid;
+    unsigned long long n_aa = 0, n_aw = 0, n_ax = 0;
+    if (b < F.nb) {
+        for (int ta = slice; ta < T; ta += kFinSlices) {
+            // atom-atom rows: factor 2, self terms (ff, ff, 0) += atoms of that type
+            unsigned long long of_type = 0;
+#pragma unroll 4
             for (int tb = 0; tb < T; ++tb) {
-                unsigned long long c = F.cnt_aa[static_cast<size_t>(ta * T + tb) * nb + b];
-                n_aa += c;
+                const unsigned long long c = F.cnt_aa[static_cast<size_t>(ta * T + tb) * nb + b];
+                of_type += c;
                 double v = 2.0 * static_cast<double>(c);
                 if (b == 0 && ta == tb) v += F.type_count[ta];
                 F.H[static_cast<size_t>(ta * T + tb) * nb + b] = v;
-                ax_sum += 2.0 * static_cast<double>(c);
-                tot += 2ull * c;
             }
+            n_aa += of_type;
             // [ff][exv] rows: every atom-atom pair also increments (ff_i, exv) with the lower-index
             // atom's type (HistogramManagerMTFFAvg.cpp:27-35), i.e. the marginal over ff_j
             double ax = 0;
-            if (F.kind == kKindAvg) ax = ax_sum * F.z_exv;
-            else if (F.kind == kKindGrid) ax = static_cast<double>(F.cnt_ax[static_cast<size_t>(ta) * nb + b]);
+            if (F.kind == kKindAvg) {
+                ax = 2.0 * static_cast<double>(of_type) * F.z_exv;
+            } else if (grid) {
+                const unsigned long long c = F.cnt_ax[static_cast<size_t>(ta) * nb + b];
+                n_ax += c;
+                ax = static_cast<double>(c);
+            }
             F.H[static_cast<size_t>(T * T + ta) * nb + b] = ax;
-            xx_sum += ax_sum;
-        }
-        if (b == 0) tot += static_cast<unsigned long long>(F.n_a);
-        double xx = 0;
-        // val * (Z * Z): the reference's release build hoists Z*Z (HistogramManagerMTFFAvg.cpp:361-362)
-        if (F.kind == kKindAvg) xx = (xx_sum + (b == 0 ? F.n_a : 0)) * (F.z_exv * F.z_exv);
-        else if (F.kind == kKindGrid) xx = 2.0 * static_cast<double>(F.cnt_xx[b]) + (b == 0 ? F.n_x : 0);
-        F.H[static_cast<size_t>(T * T + T) * nb + b] = xx;
-        // atom-water rows (factor 1) and their exv marginal
-        unsigned long long n_aw = 0;
-        for (int t = 0; t < T; ++t) {
-            unsigned long long c = F.cnt_aw[static_cast<size_t>(t) * nb + b];
+            // atom-water rows (factor 1)
+            const unsigned long long c = F.cnt_aw[static_cast<size_t>(ta) * nb + b];
             n_aw += c;
-            F.H[static_cast<size_t>(T * T + T + 1 + t) * nb + b] = static_cast<double>(c);
+            F.H[static_cast<size_t>(T * T + T + 1 + ta) * nb + b] = static_cast<double>(c);
         }
-        tot += n_aw;
-        double wx = 0;
-        if (F.kind == kKindAvg) wx = static_cast<double>(n_aw) * F.z_exv;
-        else if (F.kind == kKindGrid) wx = static_cast<double>(F.cnt_wx[b]);
+    }
+    s_n[0][slice][lane] = n_aa;
+    s_n[1][slice][lane] = n_aw;
+    s_n[2][slice][lane] = n_ax;
+    __syncthreads();
+    if (slice == 0 && b < F.nb) {
+        for (int k = 1; k < kFinSlices; ++k) {
+            n_aa += s_n[0][k][lane];
+            n_aw += s_n[1][k][lane];
+            n_ax += s_n[2][k][lane];
+        }
+        const unsigned long long n_ww = F.cnt_ww[b];
+        const unsigned long long n_xx = grid ? F.cnt_xx[b] : 0, n_wx = grid ? F.cnt_wx[b] : 0;
+        double xx = 0, wx = 0;
+        // val * (Z * Z): the reference's release build hoists Z*Z (HistogramManagerMTFFAvg.cpp:361-362)
+        if (F.kind == kKindAvg) {
+            xx = (2.0 * static_cast<double>(n_aa) + (b == 0 ? F.n_a : 0)) * (F.z_exv * F.z_exv);
+            wx = static_cast<double>(n_aw) * F.z_exv;
+        } else if (grid) {
+            xx = 2.0 * static_cast<double>(n_xx) + (b == 0 ? F.n_x : 0);
+            wx = static_cast<double>(n_wx);
+        }
+        F.H[static_cast<size_t>(T * T + T) * nb + b] = xx;
         F.H[static_cast<size_t>(T * T + 2 * T + 1) * nb + b] = wx;
-        unsigned long long n_ww = F.cnt_ww[b];
-        double ww = 2.0 * static_cast<double>(n_ww) + (b == 0 ? F.n_w : 0);
-        F.H[static_cast<size_t>(T * T + 2 * T + 2) * nb + b] = ww;
-        tot += 2ull * n_ww + (b == 0 ? static_cast<unsigned long long>(F.n_w) : 0ull);
+        F.H[static_cast<size_t>(T * T + 2 * T + 2) * nb + b] = 2.0 * static_cast<double>(n_ww) + (b == 0 ? F.n_w : 0);
+        unsigned long long tot = 2ull * n_aa + n_aw + 2ull * n_ww;
+        if (b == 0) tot += static_cast<unsigned long long>(F.n_a) + F.n_w;
         F.tot[b] = static_cast<double>(tot);
-
-        // weighted axis of p_tot = aa(ff >= 1) + aw(ff >= 1) + ww, bin 0 pinned to 0
-        if (F.weighted) {
-            double ds = 2.0 * dist_sum(F.ds_aa, n_aa, b, F.c, F.scale) + dist_sum(F.ds_aw, n_aw, b, F.c, F.scale) +
-                        2.0 * dist_sum(F.ds_ww, n_ww, b, F.c, F.scale);
-            F.d_axis[b] = b == 0 ? 0.0 : weighted_bin(ds, static_cast<double>(tot), b, width);
-        } else {
-            F.d_axis[b] = b * width;
+        // the distance sums of the axes, turned into means by the last block
+        if (F.weighted)
+            F.d_axis[b] = 2.0 * dist_sum(F.ds_aa, n_aa, b, F.c, F.scale) + dist_sum(F.ds_aw, n_aw, b, F.c, F.scale) +
+                          2.0 * dist_sum(F.ds_ww, n_ww, b, F.c, F.scale);
+        bool used = tot != 0;
+        if (grid) {
+            F.d_axis_ax[b] = dist_sum(F.ds_ax, n_ax, b, F.c, F.scale) + dist_sum(F.ds_wx, n_wx, b, F.c, F.scale);
+            F.d_axis_xx[b] = 2.0 * dist_sum(F.ds_xx, n_xx, b, F.c, F.scale);
+            used = used || xx != 0 || n_wx != 0;
         }
-        if (F.kind == kKindGrid) {
+        const unsigned at = __ballot_sync(__activemask(), used && b >= 10);
+        if (lane == 0) atomicMax(F.max_bin, max(10, at ? b + 32 - __clz(at) : 0));  // minimum size (HistogramManagerMT.cpp:48)
+    }
+    if (!last_block(F.done, blocks)) return;
+    const int mb = __ldcg(F.max_bin);
+    const double width = (static_cast<double>(mb) * F.bin_width) / mb;  // Axis(0, mb*width, mb).width()
+    for (int k = slice * kFinBins + lane; k < F.nb; k += kFinBins * kFinSlices) {
+        if (k >= mb) {
+            F.d_axis[k] = 0;
+            if (F.d_axis_ax) F.d_axis_ax[k] = 0;
+            if (F.d_axis_xx) F.d_axis_xx[k] = 0;
+            // (atom-dummy pairs do not raise max_bin: the only rows that can hold something here)
+            if (grid)
+                for (int t = 0; t < T; ++t) F.H[static_cast<size_t>(T * T + t) * nb + k] = 0;
+            continue;
+        }
+        // weighted axis of p_tot = aa(ff >= 1) + aw(ff >= 1) + ww, bin 0 pinned to 0
+        if (F.weighted) F.d_axis[k] = k == 0 ? 0.0 : weighted_bin(__ldcg(F.d_axis + k), __ldcg(F.tot + k), k, width);
+        else F.d_axis[k] = k * width;
+        if (grid) {
             // ax + wx share one axis, xx has its own; neither pins bin 0 (CompositeDistanceHistogramFFGrid.cpp:129-134)
-            unsigned long long n_ax = 0;
-            for (int t = 0; t < T; ++t) n_ax += F.cnt_ax[static_cast<size_t>(t) * nb + b];
-            unsigned long long n_wx = F.cnt_wx[b];
-            double ds_ax = dist_sum(F.ds_ax, n_ax, b, F.c, F.scale) + dist_sum(F.ds_wx, n_wx, b, F.c, F.scale);
-            F.d_axis_ax[b] = weighted_bin(ds_ax, static_cast<double>(n_ax + n_wx), b, width);
-            unsigned long long n_xx = F.cnt_xx[b];
-            double ds_xx = 2.0 * dist_sum(F.ds_xx, n_xx, b, F.c, F.scale);
-            F.d_axis_xx[b] = weighted_bin(ds_xx, 2.0 * n_xx + (b == 0 ? F.n_x : 0), b, width);
+            double n = __ldcg(F.H + static_cast<size_t>(T * T + 2 * T + 1) * nb + k);
+            for (int t = 0; t < T; ++t) n += __ldcg(F.H + static_cast<size_t>(T * T + t) * nb + k);
+            F.d_axis_ax[k] = weighted_bin(__ldcg(F.d_axis_ax + k), n, k, width);
+            F.d_axis_xx[k] = weighted_bin(__ldcg(F.d_axis_xx + k), __ldcg(F.H + static_cast<size_t>(T * T + T) * nb + k), k, width);
         }
     }
 }
 
-__global__ void ff_maxbin_kernel(FinalizeFF F) { ff_maxbin_body(F); }
-__global__ void ff_rows_kernel(FinalizeFF F) { ff_rows_body(F); }
+__global__ void ff_finalize_kernel(FinalizeFF F) { ff_finalize_body(F, gridDim.x); }
 // batched: blockIdx.y selects the structure
-__global__ void ff_maxbin_batch_kernel(const FinalizeFF* Fs) { ff_maxbin_body(Fs[blockIdx.y]); }
-__global__ void ff_rows_batch_kernel(const FinalizeFF* Fs) { ff_rows_body(Fs[blockIdx.y]); }
+__global__ void ff_finalize_batch_kernel(const FinalizeFF* Fs) { ff_finalize_body(Fs[blockIdx.y], gridDim.x); }
 
 // Expansion of the compact rows to the reference's [15][15] / [15] layouts, stride max_bin.
 __global__ void ff_expand_kernel(FinalizeFF F, double* aa_out, double* aw_out) {
@@ -210,70 +235,56 @@ __device__ __forceinline__ double weight_sum(const long long* w, const unsigned 
     return static_cast<double>(static_cast<long long>(raw)) * inv;
 }
 
-__global__ void mt_maxbin_kernel(FinalizeMT F) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicMax(F.max_bin, 10);  // minimum size (HistogramManagerMT.cpp:48)
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < F.nb; b += gridDim.x * blockDim.x) {
-        double inv = 1.0 / static_cast<double>(*F.wscale);
-        double v = 2.0 * weight_sum(F.w_aa, F.c_aa, b, inv) + 2.0 * weight_sum(F.w_ww, F.c_ww, b, inv) +
-                   2.0 * weight_sum(F.w_aw, F.c_aw, b, inv);
-        if (b == 0) v += *F.self_aa + *F.self_ww;
-        if (v != 0 && b >= 10) atomicMax(F.max_bin, b + 1);
-    }
-}
-
-__global__ void mt_rows_kernel(FinalizeMT F) {
-    const int mb = *F.max_bin;
-    const double width = (static_cast<double>(mb) * F.bin_width) / mb;
-    const double inv = 1.0 / static_cast<double>(*F.wscale);
+__global__ void mt_finalize_kernel(FinalizeMT F) {
     const size_t nb = F.nb;
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < F.nb; b += gridDim.x * blockDim.x) {
-        if (b >= mb) {
-            F.H[b] = F.H[nb + b] = F.H[2 * nb + b] = 0;
-            F.tot[b] = 0;
-            F.d_axis[b] = 0;
-            continue;
-        }
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b < F.nb) {
+        const double inv = 1.0 / static_cast<double>(*F.wscale);
         double aa = 2.0 * weight_sum(F.w_aa, F.c_aa, b, inv);
         double aw = 2.0 * weight_sum(F.w_aw, F.c_aw, b, inv);
         double ww = 2.0 * weight_sum(F.w_ww, F.c_ww, b, inv);
-        unsigned int c_aa = 2u * static_cast<unsigned int>(F.c_aa[b]);
-        unsigned int c_aw = 2u * static_cast<unsigned int>(F.c_aw[b]);
-        unsigned int c_ww = 2u * static_cast<unsigned int>(F.c_ww[b]);
+        if (F.weighted)
+            F.d_axis[b] = 2.0 * dist_sum(F.ds_aa, F.c_aa[b], b, F.c, F.scale) + 2.0 * dist_sum(F.ds_ww, F.c_ww[b], b, F.c, F.scale) +
+                          2.0 * dist_sum(F.ds_aw, F.c_aw[b], b, F.c, F.scale);
+        double v = aa + ww + aw;  // (the order in which bins count as used)
         if (b == 0) {
             aa += *F.self_aa;
             ww += *F.self_ww;
-            c_aa += static_cast<unsigned int>(*F.self_aa);
-            c_ww += static_cast<unsigned int>(*F.self_ww);
+            v += *F.self_aa + *F.self_ww;
         }
         F.H[b] = aa;
         F.H[nb + b] = aw;
         F.H[2 * nb + b] = ww;
         F.tot[b] = aa + ww + aw;
-        if (F.weighted && b > 0) {
-            double ds = 2.0 * dist_sum(F.ds_aa, F.c_aa[b], b, F.c, F.scale) + 2.0 * dist_sum(F.ds_ww, F.c_ww[b], b, F.c, F.scale) +
-                        2.0 * dist_sum(F.ds_aw, F.c_aw[b], b, F.c, F.scale);
-            F.d_axis[b] = weighted_bin(ds, static_cast<double>(c_aa + c_ww + c_aw), b, width);
+        const unsigned at = __ballot_sync(__activemask(), v != 0 && b >= 10);
+        if ((threadIdx.x & 31) == 0) atomicMax(F.max_bin, max(10, at ? b + 32 - __clz(at) : 0));  // minimum size (HistogramManagerMT.cpp:48)
+    }
+    if (!last_block(F.done, gridDim.x)) return;
+    const int mb = __ldcg(F.max_bin);
+    const double width = (static_cast<double>(mb) * F.bin_width) / mb;
+    for (int k = threadIdx.x; k < F.nb; k += blockDim.x) {
+        if (k >= mb) {
+            F.H[k] = F.H[nb + k] = F.H[2 * nb + k] = 0;
+            F.tot[k] = 0;
+            F.d_axis[k] = 0;
+        } else if (F.weighted && k > 0) {
+            const unsigned int n = 2u * static_cast<unsigned int>(F.c_aa[k]) + 2u * static_cast<unsigned int>(F.c_ww[k]) +
+                                   2u * static_cast<unsigned int>(F.c_aw[k]);
+            F.d_axis[k] = weighted_bin(__ldcg(F.d_axis + k), static_cast<double>(n), k, width);
         } else {
-            F.d_axis[b] = b * width;
+            F.d_axis[k] = k == 0 ? 0.0 : k * width;
         }
-        if (b == 0) F.d_axis[b] = 0;
     }
 }
 
 }  // namespace
 
 void ff_finalize_launch(const FinalizeFF& F, cudaStream_t s) {
-    int threads = 256;
-    int blocks = (F.nb + threads - 1) / threads;
-    ff_maxbin_kernel<<<blocks, threads, 0, s>>>(F);
-    ff_rows_kernel<<<blocks, threads, 0, s>>>(F);
+    ff_finalize_kernel<<<(F.nb + kFinBins - 1) / kFinBins, dim3(kFinBins, kFinSlices), 0, s>>>(F);
 }
 
 void ff_finalize_batch_launch(const FinalizeFF* Fs_dev, int n, int max_nb, cudaStream_t s) {
-    int threads = 256;
-    dim3 grid((max_nb + threads - 1) / threads, n);
-    ff_maxbin_batch_kernel<<<grid, threads, 0, s>>>(Fs_dev);
-    ff_rows_batch_kernel<<<grid, threads, 0, s>>>(Fs_dev);
+    ff_finalize_batch_kernel<<<dim3((max_nb + kFinBins - 1) / kFinBins, n), dim3(kFinBins, kFinSlices), 0, s>>>(Fs_dev);
 }
 
 void ff_expand_launch(const FinalizeFF& F, double* aa_out, double* aw_out, int nb_hint, cudaStream_t s) {
@@ -295,10 +306,7 @@ void weight_square_sum_launch(const float4* p, int n, double* out, cudaStream_t 
 }
 
 void mt_finalize_launch(const FinalizeMT& F, cudaStream_t s) {
-    int threads = 256;
-    int blocks = (F.nb + threads - 1) / threads;
-    mt_maxbin_kernel<<<blocks, threads, 0, s>>>(F);
-    mt_rows_kernel<<<blocks, threads, 0, s>>>(F);
+    mt_finalize_kernel<<<(F.nb + 127) / 128, 128, 0, s>>>(F);
 }
 
 }  // namespace ausaxs_b200

@@ -38,7 +38,8 @@ struct FinalizeFF {
     double bin_width;
     float c, scale;
     int32_t weighted;
-    int32_t* max_bin;  // device, preset to 10
+    int32_t* max_bin;  // device, preset to 0
+    unsigned* done;    // blocks that have finished: 0 between launches
     double* H;         // [ff_rows(T)][nb]
     double* tot;       // [nb]
     double* d_axis;    // [nb]
@@ -59,6 +60,7 @@ struct FinalizeMT {
     float c, scale;
     int32_t weighted;
     int32_t* max_bin;
+    unsigned* done;  // blocks that have finished: 0 between launches
     double* H;  // [3][nb]
     double* tot;
     double* d_axis;
