@@ -105,12 +105,17 @@ void Structure::load_begin(const float* atoms, int n_atoms, const float* waters,
 
     PrepStats init{};
     for (int k = 0; k < 3; ++k) init.lo[k] = 0xffffffffu, init.hi[k] = 0;
+    for (auto& w : init.weights) std::fill(w.bits, w.bits + 16, kNoClass);
     *h_stats = init;  // pinned: the copy below reads it asynchronously, the census result overwrites it
     AUSAXS_CUDA(cudaMemcpyAsync(d_stats, h_stats, sizeof(PrepStats), cudaMemcpyHostToDevice, s));
     census_launch(raw_a.as<float4>(), n_a, ff_typed, d_stats, C.sm_count, s);
     census_launch(raw_w.as<float4>(), n_w, 0, d_stats, C.sm_count, s);
     census_launch(raw_x.as<float4>(), n_x, 0, d_stats, C.sm_count, s);
     radius_launch(raw_a.as<float4>(), n_a, raw_w.as<float4>(), n_w, raw_x.as<float4>(), n_x, d_stats, C.sm_count, s);
+    if (!ff_typed) {
+        weight_classes_launch(raw_a.as<float4>(), n_a, &d_stats->weights[0], C.sm_count, s);
+        weight_classes_launch(raw_w.as<float4>(), n_w, &d_stats->weights[1], C.sm_count, s);
+    }
     C.check_launch("census");
     AUSAXS_CUDA(cudaMemcpyAsync(h_stats, d_stats, sizeof(PrepStats), cudaMemcpyDeviceToHost, s));
 }
@@ -122,7 +127,7 @@ static size_t typed_off_pos(int n) { return typed_off_counts(n) + align_up((size
 size_t Structure::typed_bytes(int n) { return typed_off_pos(n) + align_up((size_t)std::max(1, n) * 4, 256); }
 int32_t* Structure::typed_pos() const { return typed.as<int32_t>(typed_off_pos(n_a)); }
 
-TypedSet typed_lists(const float4* in, float4* dense, int n, const int32_t* ff_to_type, int types, const int* count, char* mem,
+TypedSet typed_lists(const float4* in, float4* dense, int n, const TypeMap& map, int types, const int* count, char* mem,
                      bool want_pos, cudaStream_t s) {
     TypedOut o{};
     o.pts = reinterpret_cast<float4*>(mem);
@@ -140,7 +145,7 @@ TypedSet typed_lists(const float4* in, float4* dense, int n, const int32_t* ff_t
         set.count[t] = count[t];
         at += count[t];
     }
-    typed_lists_launch(in, dense, n, ff_to_type, o, reinterpret_cast<int32_t*>(mem + typed_off_counts(n)), s);
+    typed_lists_launch(in, dense, n, map, o, reinterpret_cast<int32_t*>(mem + typed_off_counts(n)), s);
     return set;
 }
 
@@ -188,10 +193,37 @@ void Structure::load_end(const PrepStats& st) {
     if (ff_typed) {
         dense_a.ensure(align_up(std::max(1, n_a) * 16, 256));
         typed.ensure(typed_bytes(n_a));
-        lists = typed_lists(raw_a.as<float4>(), dense_a.as<float4>(), n_a, meta.as<int32_t>(kNff * 4), T, type_count,
-                            typed.as<char>(), want_pos, s);
+        TypeMap map;
+        map.ff_to_type = meta.as<int32_t>(kNff * 4);
+        lists = typed_lists(raw_a.as<float4>(), dense_a.as<float4>(), n_a, map, T, type_count, typed.as<char>(), want_pos, s);
         C.check_launch("typed lists");
         if (n_a > 0) C.launches += 1;  // two kernels
+        return;
+    }
+    // weighted: the points by class of weight
+    n_cls[0] = n_cls[1] = 0;
+    for (int k = 0; k < 2; ++k) {
+        const int n = k ? n_w : n_a;
+        if (st.weights[k].over || n == 0) continue;
+        std::vector<std::pair<unsigned, int>> found;
+        for (int i = 0; i < kMaxClasses; ++i)
+            if (st.weights[k].bits[i] != kNoClass) found.push_back({st.weights[k].bits[i], st.weights[k].count[i]});
+        std::sort(found.begin(), found.end());
+        TypeMap map;
+        map.classes = n_cls[k] = (int)found.size();
+        for (size_t i = 0; i < found.size(); ++i) {
+            map.bits[i] = found[i].first;
+            std::memcpy(&cls[k][i], &found[i].first, 4);
+            cls_count[k][i] = found[i].second;
+        }
+        DevBuf& dense = k ? dense_w : dense_a;
+        DevBuf& mem = k ? typed_w : typed;
+        dense.ensure(align_up((size_t)n * 16, 256));
+        mem.ensure(typed_bytes(n));
+        (k ? lists_w : lists) = typed_lists((k ? raw_w : raw_a).as<float4>(), dense.as<float4>(), n, map, n_cls[k], cls_count[k],
+                                            mem.as<char>(), false, s);
+        C.check_launch("typed lists");
+        C.launches += 1;  // two kernels
     }
 }
 
@@ -289,7 +321,8 @@ void append_pack_jobs(const Plan& P, int outer, bool joint, PackLaunch& L, PackT
         const bool pair_rows = j.rmode == kRowPair;
         if (row_class >= 0 && (j.rmode != kRowSingle) != (row_class == 1)) continue;
         // the largest row's share of a job's pairs (outer points have the composition of the whole structure)
-        const double share = j.rows == 1 ? 1.0 : P.row_share;
+        const int rows_out = pair_rows ? (j.t_out ? j.t_out : P.T) : j.rows;
+        const double share = rows_out == 1 ? 1.0 : P.row_share;
         for (int t = 0; t < (pair_rows ? j.typed->types : 1); ++t) {
             PackJob p{};
             p.A = j.A;
@@ -300,7 +333,7 @@ void append_pack_jobs(const Plan& P, int outer, bool joint, PackLaunch& L, PackT
             p.self = j.self;
             p.indexed = pair_rows ? 1 : 0;
             p.pre = pair_rows ? j.typed->pre + (size_t)t * j.typed->pre_stride : nullptr;
-            p.rows = pair_rows ? P.T : j.rows;
+            p.rows = rows_out;
             p.nbins = P.nb;
             p.tiles_i = up(p.na, outer);
             p.tiles_j = up(p.nb, L.tile_j);
@@ -314,7 +347,7 @@ void append_pack_jobs(const Plan& P, int outer, bool joint, PackLaunch& L, PackT
             p.tail_from_outer = j.tail_from_outer >= 0 ? j.tail_from_outer : j.self;
             p.seg_pairs = pack_segment_pairs(j.spread_bins > 0 ? std::min(j.spread_bins, P.nb) : P.nb, share);
             p.cnt_row = rows;
-            for (int r = 0; r < p.rows; ++r) T.out.push_back(j.counts + (size_t)(pair_rows ? r * P.T + t : r) * P.nb);
+            for (int r = 0; r < p.rows; ++r) T.out.push_back(j.counts + (size_t)(pair_rows ? r * j.typed->types + t : r) * P.nb);
             rows += p.rows;
             if (j.dsum) {
                 auto it = std::find(sums.begin(), sums.end(), j.dsum);
@@ -506,7 +539,8 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     if (P.manager == cfg.manager && P.weighted == weighted && P.bin_count == cfg.bin_count &&
         P.bin_width == cfg.bin_width && P.n_a == n_a && P.n_w == n_w && P.n_x == n_x && P.T == T && P.nb >= nb &&
         P.nb <= nb + 64 && (cfg.manager != AUSAXS_MANAGER_FFGRID || n_x < kLatticeMinPoints || lat.tried) &&
-        std::equal(type_ff, type_ff + T, P.type_ff) && (!P.packed || std::equal(type_count, type_count + T, P.type_count))) {
+        std::equal(n_cls, n_cls + 2, P.n_cls) && std::memcmp(cls, P.cls, sizeof cls) == 0 &&
+        std::memcmp(cls_count, P.cls_count, sizeof cls_count) == 0 && std::equal(type_ff, type_ff + T, P.type_ff) && (!P.packed || std::equal(type_count, type_count + T, P.type_count))) {
         P.fin_ff.z_exv = cfg.z_exv;  // per call: other molecules of the same shape have other volumes
         return P;
     }
@@ -522,6 +556,9 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     P.T = T;
     std::copy(type_ff, type_ff + T, P.type_ff);
     std::copy(type_count, type_count + T, P.type_count);
+    std::copy(n_cls, n_cls + 2, P.n_cls);
+    std::memcpy(P.cls, cls, sizeof cls);
+    std::memcpy(P.cls_count, cls_count, sizeof cls_count);
     P.row_share = 1.0;
     if (T > 0 && n_a > 0) P.row_share = (double)*std::max_element(type_count, type_count + T) / n_a;
     P.nb = nb;
@@ -555,17 +592,40 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
         int nbp;
         int self, rmode, rows;
         int slot;  // accumulator slot (aa, aw, ww, ax, wx, xx)
+        int t_out = 0;
+        const TypedSet* typed = nullptr;
     };
     std::vector<J> js;
     const float4* A = atoms_for_pairs();
     const float4* W = raw_w.as<float4>();
     const float4* X = raw_x.as<float4>();
-    if (mt) {
+    // Weighted points of few classes of weight: the counts by class pair give the weight sums, so the pairs
+    // go through the one-atomic kernel (20,000 atoms of four weights + 4,000 waters: see the finalisation).
+    bool by_class = false;
+    if (mt && (n_a == 0 || n_cls[0] > 0) && (n_w == 0 || n_cls[1] > 0) && n_a + n_w > 0) {
+        pair_sqrt_prepare(P.inv_w, nb);
+        PackLaunch K{};
+        K.nr = pair_sqrt_mode(P.inv_w, nb);
+        K.rows = K.group_rows = std::max(1, std::max(n_cls[0], n_cls[1]));
+        K.group_sums = 1;
+        K.bins = nb;
+        K.tile_j = kPackMaxTileJ;
+        K.offsets = weighted;
+        by_class = K.nr > 0 && pack_shape(K) >= 0;
+    }
+    if (by_class) {
+        if (n_a > 0) P.row_share = (double)*std::max_element(cls_count[0], cls_count[0] + n_cls[0]) / n_a;
+        const float4* Wd = dense_w.as<float4>();
+        A = dense_a.as<float4>();
+        js.push_back({A, n_a, A, n_a, 1, kRowPair, n_cls[0] * n_cls[0], 0, n_cls[0], &lists});
+        js.push_back({Wd, n_w, A, n_a, 0, kRowPair, n_cls[1] * n_cls[0], 1, n_cls[1], &lists});
+        js.push_back({Wd, n_w, Wd, n_w, 1, kRowPair, n_cls[1] * n_cls[1], 2, n_cls[1], &lists_w});
+    } else if (mt) {
         js.push_back({A, n_a, A, n_a, 1, kRowSingle, 1, 0});
         js.push_back({W, n_w, A, n_a, 0, kRowSingle, 1, 1});  // waters outer, atoms inner (SimpleCalculator.h:187-205)
         js.push_back({W, n_w, W, n_w, 1, kRowSingle, 1, 2});
     } else {
-        js.push_back({A, n_a, A, n_a, 1, kRowPair, T * T, 0});
+        js.push_back({A, n_a, A, n_a, 1, kRowPair, T * T, 0, T, &lists});
         js.push_back({A, n_a, W, n_w, 0, kRowOuter, T, 1});  // atoms outer, waters inner (HistogramManagerMTFFAvg.cpp:236-254)
         js.push_back({W, n_w, W, n_w, 1, kRowSingle, 1, 2});
         if (grid) {
@@ -663,9 +723,10 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
         sp.counts = reinterpret_cast<unsigned long long*>(base + slot_cnt[j.slot]);
         // offset sums only feed the weighted d-axis; weight sums are the Simple histogram's values
         sp.dsum = weighted ? reinterpret_cast<unsigned long long*>(base + slot_ds[j.slot]) : nullptr;
-        sp.wsum = mt ? reinterpret_cast<long long*>(base + slot_ws[j.slot]) : nullptr;
+        sp.wsum = mt && !by_class ? reinterpret_cast<long long*>(base + slot_ws[j.slot]) : nullptr;
         sp.lattice = use_lattice && j.slot == 5;
-        sp.typed = j.slot == 0 && !mt ? &lists : nullptr;
+        sp.t_out = j.t_out;
+        sp.typed = j.typed;
         P.specs.push_back(sp);
     }
     P.max_group_rows = max_group_rows;
@@ -689,7 +750,7 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     pair_sqrt_prepare(P.inv_w, nb);  // once per width and process: the Newton-Raphson root where it bins exactly
     P.n_launch = 0;
     PackTable table;
-    P.packed = !mt && choose_pack(P, C.sm_count, P.pack, P.pack_shape, P.pack_grid, table);
+    P.packed = (!mt || by_class) && choose_pack(P, C.sm_count, P.pack, P.pack_shape, P.pack_grid, table);
     if (P.packed) {
         const size_t jobs_bytes = sizeof(PackJob) * table.jobs.size();
         if (jobs_bytes + sizeof(void*) * table.out.size() > P.off_acc - P.off_jobs)
@@ -731,6 +792,27 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
         F.weighted = weighted;
         F.max_bin = reinterpret_cast<int32_t*>(base + P.off_maxbin);
         F.done = reinterpret_cast<unsigned*>(base + P.off_maxbin) + 16;
+        F.n32 = reinterpret_cast<unsigned long long*>(base + slot_ws[2]);
+        F.ta = F.tw = 0;
+        if (by_class) {
+            F.ta = std::max(1, n_cls[0]);  // (no atoms: their empty row)
+            F.tw = std::max(1, n_cls[1]);
+            std::copy(cls[0], cls[0] + 16, F.class_a);
+            std::copy(cls[1], cls[1] + 16, F.class_w);
+            // 2^k with max|w_i w_j| * 2^k <= 2^30, and the diagonal sums of float(w * w)
+            float m = 0;
+            for (int k = 0; k < 2; ++k) {
+                F.self_v[k] = 0;
+                for (int i = 0; i < n_cls[k]; ++i) {
+                    m = std::max(m, std::fabs(cls[k][i]));
+                    F.self_v[k] += (double)cls_count[k][i] * (double)(cls[k][i] * cls[k][i]);
+                }
+            }
+            const double p = (double)m * m;
+            int e = 0;
+            if (p > 0) std::frexp(p, &e);
+            F.wscale_v = std::ldexp(1.0f, std::min(60, 30 - e));
+        }
         F.H = reinterpret_cast<double*>(base + P.off_H);
         F.tot = reinterpret_cast<double*>(base + P.off_tot);
         F.d_axis = reinterpret_cast<double*>(base + P.off_d);
@@ -800,7 +882,7 @@ void Structure::enqueue_histogram(const ausaxs_hist_config& cfg) {
     char* base = P.dev.as<char>();
     AUSAXS_CUDA(cudaMemsetAsync(base + P.off_acc, 0, P.acc_bytes, s));
     const bool mt = cfg.manager == AUSAXS_MANAGER_MT;
-    if (mt) {
+    if (mt && P.fin_mt.ta == 0) {
         weight_scale_launch(raw_a.as<float4>(), n_a, raw_w.as<float4>(), n_w, reinterpret_cast<float*>(base + P.off_wscale), s);
         weight_square_sum_launch(raw_a.as<float4>(), n_a, reinterpret_cast<double*>(base + P.off_self), s);
         weight_square_sum_launch(raw_w.as<float4>(), n_w, reinterpret_cast<double*>(base + P.off_self) + 1, s);

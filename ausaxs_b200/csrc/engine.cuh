@@ -57,7 +57,7 @@ struct TypedSet {
 };
 
 // The lists of `in` (typed_lists_launch) in mem (Structure::typed_bytes(n)); count: points of each type.
-TypedSet typed_lists(const float4* in, float4* dense, int n, const int32_t* ff_to_type, int types, const int* count, char* mem,
+TypedSet typed_lists(const float4* in, float4* dense, int n, const TypeMap& map, int types, const int* count, char* mem,
                      bool want_pos, cudaStream_t s);
 
 // One pass of pair binning of a structure before it is cut into tiles: the two point sets, the
@@ -76,6 +76,7 @@ struct JobSpec {
     int mult = 1;  // multiplicity of every pair (PairJob::mult)
     bool lattice = false;  // the plan bins this pass with the lattice kernel (the structure's own launches)
     int spread_bins = 0;   // bins the distances spread over, about (0: all of the plan's)
+    int t_out = 0;         // pair rows: types of the outer points (rows [t_out][typed->types])
     const TypedSet* typed = nullptr;  // atom-atom passes: the inner atoms' lists (append_pack_jobs)
 };
 
@@ -101,6 +102,9 @@ struct Plan {
     int n_a = -1, n_w = -1, n_x = -1, T = -1;
     int type_ff[kNff] = {};     // the form-factor types behind the rows
     int type_count[kNff] = {};  // and the sizes of the typed lists
+    int n_cls[2] = {0, 0};      // weighted: the classes of atoms and waters behind the rows (0: by value)
+    float cls[2][16] = {};
+    int cls_count[2][16] = {};
     // shapes
     int nb = 0, tile = 256;
     struct Group {  // one pair-kernel launch
@@ -155,6 +159,13 @@ struct Structure {
     DevBuf typed;           // the atoms' lists by type (typed_bytes)
     TypedSet lists;
     bool want_pos = false;  // also every atom's place in them (typed_pos)
+    // Weighted structures whose atoms and waters have at most kMaxClasses distinct weights each: the classes
+    // (ascending bit patterns), the points with their class as type, and their lists.  n_cls 0: more.
+    int n_cls[2] = {0, 0};
+    float cls[2][16] = {};
+    int cls_count[2][16] = {};
+    DevBuf dense_w, typed_w;
+    TypedSet lists_w;
     static size_t typed_bytes(int n);
     int32_t* typed_pos() const;
     int T = 0;

@@ -228,29 +228,52 @@ __global__ void weight_scale_kernel(const float4* a, int na, const float4* b, in
     }
 }
 
-// Weighted sum of one job in bin b: the pair kernel adds rint(w_i w_j * wscale) + 2^30 per pair
-// (unsigned, wrapping); the bias is removed with n pairs counted in the bin.
-__device__ __forceinline__ double weight_sum(const long long* w, const unsigned long long* n, int b, double inv) {
-    unsigned long long raw = static_cast<unsigned long long>(w[b]) - n[b] * (1ull << 30);
-    return static_cast<double>(static_cast<long long>(raw)) * inv;
+// Pairs and fixed-point weight sum of one job in bin b.  The two-atomic kernel adds rint(w_i w_j * wscale) +
+// 2^30 per pair (unsigned, wrapping) and the bias of n pairs is removed; rows by class give the same sum.
+struct MTSum {
+    unsigned long long n;
+    long long w;
+};
+__device__ MTSum mt_sum(const unsigned long long* cnt, const long long* w, int rows, int cols, const float* cr, const float* cc,
+                        float wscale, size_t nb, int b) {
+    MTSum s{0, 0};
+    if (rows == 0) {
+        s.n = cnt[b];
+        s.w = static_cast<long long>(static_cast<unsigned long long>(w[b]) - s.n * (1ull << 30));
+        return s;
+    }
+    for (int r = 0; r < rows; ++r)
+#pragma unroll 4
+        for (int k = 0; k < cols; ++k) {
+            const unsigned long long n = cnt[static_cast<size_t>(r * cols + k) * nb + b];
+            s.n += n;
+            s.w += static_cast<long long>(n) * __float2int_rn(__fmul_rn(__fmul_rn(cr[r], cc[k]), wscale));
+        }
+    return s;
 }
 
 __global__ void mt_finalize_kernel(FinalizeMT F) {
     const size_t nb = F.nb;
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b < F.nb) {
-        const double inv = 1.0 / static_cast<double>(*F.wscale);
-        double aa = 2.0 * weight_sum(F.w_aa, F.c_aa, b, inv);
-        double aw = 2.0 * weight_sum(F.w_aw, F.c_aw, b, inv);
-        double ww = 2.0 * weight_sum(F.w_ww, F.c_ww, b, inv);
+        const float wscale = F.ta ? F.wscale_v : *F.wscale;
+        const double inv = 1.0 / static_cast<double>(wscale);
+        const MTSum s_aa = mt_sum(F.c_aa, F.w_aa, F.ta, F.ta, F.class_a, F.class_a, wscale, nb, b);
+        const MTSum s_aw = mt_sum(F.c_aw, F.w_aw, F.ta ? F.tw : 0, F.ta, F.class_w, F.class_a, wscale, nb, b);
+        const MTSum s_ww = mt_sum(F.c_ww, F.w_ww, F.ta ? F.tw : 0, F.tw, F.class_w, F.class_w, wscale, nb, b);
+        double aa = 2.0 * (static_cast<double>(s_aa.w) * inv);
+        double aw = 2.0 * (static_cast<double>(s_aw.w) * inv);
+        double ww = 2.0 * (static_cast<double>(s_ww.w) * inv);
+        F.n32[b] = 2u * static_cast<unsigned>(s_aa.n) + 2u * static_cast<unsigned>(s_ww.n) + 2u * static_cast<unsigned>(s_aw.n);
         if (F.weighted)
-            F.d_axis[b] = 2.0 * dist_sum(F.ds_aa, F.c_aa[b], b, F.c, F.scale) + 2.0 * dist_sum(F.ds_ww, F.c_ww[b], b, F.c, F.scale) +
-                          2.0 * dist_sum(F.ds_aw, F.c_aw[b], b, F.c, F.scale);
+            F.d_axis[b] = 2.0 * dist_sum(F.ds_aa, s_aa.n, b, F.c, F.scale) + 2.0 * dist_sum(F.ds_ww, s_ww.n, b, F.c, F.scale) +
+                          2.0 * dist_sum(F.ds_aw, s_aw.n, b, F.c, F.scale);
         double v = aa + ww + aw;  // (the order in which bins count as used)
         if (b == 0) {
-            aa += *F.self_aa;
-            ww += *F.self_ww;
-            v += *F.self_aa + *F.self_ww;
+            const double d_aa = F.ta ? F.self_v[0] : *F.self_aa, d_ww = F.ta ? F.self_v[1] : *F.self_ww;
+            aa += d_aa;
+            ww += d_ww;
+            v += d_aa + d_ww;
         }
         F.H[b] = aa;
         F.H[nb + b] = aw;
@@ -268,9 +291,7 @@ __global__ void mt_finalize_kernel(FinalizeMT F) {
             F.tot[k] = 0;
             F.d_axis[k] = 0;
         } else if (F.weighted && k > 0) {
-            const unsigned int n = 2u * static_cast<unsigned int>(F.c_aa[k]) + 2u * static_cast<unsigned int>(F.c_ww[k]) +
-                                   2u * static_cast<unsigned int>(F.c_aw[k]);
-            F.d_axis[k] = weighted_bin(__ldcg(F.d_axis + k), static_cast<double>(n), k, width);
+            F.d_axis[k] = weighted_bin(__ldcg(F.d_axis + k), static_cast<double>(static_cast<unsigned>(__ldcg(F.n32 + k))), k, width);
         } else {
             F.d_axis[k] = k == 0 ? 0.0 : k * width;
         }

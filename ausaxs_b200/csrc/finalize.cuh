@@ -53,6 +53,13 @@ struct FinalizeMT {
     const unsigned long long *c_aa, *c_aw, *c_ww;
     const unsigned long long *ds_aa, *ds_aw, *ds_ww;
     const long long *w_aa, *w_aw, *w_ww;
+    // Weights of few distinct values (ta > 0): the counts are rows by the two points' classes, [ta][ta], [tw][ta]
+    // and [tw][tw], and the weight sums follow from them; scale and diagonal sums are given by value.
+    int32_t ta, tw;
+    float class_a[16], class_w[16];
+    float wscale_v;
+    double self_v[2];
+    unsigned long long* n32;  // [nb] scratch: may be w_ww, which is read first
     const float* wscale;
     const double* self_aa;  // sum float(w*w) over atoms
     const double* self_ww;

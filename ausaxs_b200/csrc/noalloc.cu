@@ -260,6 +260,7 @@ extern "C" int ausaxs_gpu_histogram_mt_noalloc(const float* atoms, int32_t n_ato
     F.scale = scale;
     F.weighted = weighted_bins ? 1 : 0;
     F.max_bin = dmaxbin;
+    F.n32 = reinterpret_cast<unsigned long long*>(wsm(2));
     F.done = reinterpret_cast<unsigned*>(counters + 6);  // cleared with the accumulators
     F.H = hist_out;                      // rows 0..2: aa, aw, ww
     F.tot = hist_out + 3 * (size_t)nb;   // row 3

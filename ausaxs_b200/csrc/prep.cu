@@ -4,6 +4,8 @@
 // every atom's form-factor type is validated (UNKNOWN and out-of-range types are an error) and
 // remapped, here to a dense index over the types the structure actually contains, so that the
 // on-chip histograms hold T*T rows instead of 15*15.
+#include <algorithm>
+
 #include "prep.cuh"
 
 namespace ausaxs_b200 {
@@ -81,7 +83,7 @@ __global__ void radius_kernel(const float4* a, int na, const float4* w, int nw, 
 
 // Dense copy of the points (w = dense type; type map null: w already is), and the points of each
 // type in every chunk of kTypedChunk points.
-__global__ void __launch_bounds__(kTypedChunk) dense_count_kernel(const float4* in, float4* out, int n, const int32_t* ff_to_type,
+__global__ void __launch_bounds__(kTypedChunk) dense_count_kernel(const float4* in, float4* out, int n, TypeMap map,
                                                                   int32_t* counts) {
     __shared__ int s_count[16];
     if (threadIdx.x < 16) s_count[threadIdx.x] = 0;
@@ -90,7 +92,14 @@ __global__ void __launch_bounds__(kTypedChunk) dense_count_kernel(const float4* 
     if (i < n) {
         float4 v = in[i];
         const int t = __float_as_int(v.w);
-        const int d = !ff_to_type ? t : ((t > kExv && t < kNff) ? ff_to_type[t] : 0);
+        int d = t;
+        if (map.classes > 0) {
+            d = 0;
+            for (int k = 1; k < map.classes; ++k)
+                if (map.bits[k] == static_cast<unsigned>(t)) d = k;
+        } else if (map.ff_to_type) {
+            d = (t > kExv && t < kNff) ? map.ff_to_type[t] : 0;
+        }
         v.w = __int_as_float(d);
         if (out) out[i] = v;
         const unsigned same = __match_any_sync(__activemask(), d);
@@ -143,6 +152,45 @@ __global__ void __launch_bounds__(kTypedChunk) typed_scatter_kernel(const float4
     }
 }
 
+// slot of w in a table of distinct values, inserted where it is new; -1: the table is full
+__device__ int class_slot(unsigned* bits, unsigned w) {
+    for (int k = 0; k < kMaxClasses; ++k) {
+        unsigned have = *reinterpret_cast<volatile unsigned*>(bits + k);
+        if (have == kNoClass) have = atomicCAS(bits + k, kNoClass, w);
+        if (have == kNoClass || have == w) return k;
+    }
+    return -1;
+}
+
+// every block's distinct weights in shared memory, then into the global table
+__global__ void weight_classes_kernel(const float4* p, int n, WeightClasses* out) {
+    __shared__ unsigned s_bits[16];
+    __shared__ int s_count[16], s_over;
+    if (threadIdx.x < 16) {
+        s_bits[threadIdx.x] = kNoClass;
+        s_count[threadIdx.x] = 0;
+    }
+    if (threadIdx.x == 0) s_over = 0;
+    __syncthreads();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const unsigned w = __float_as_uint(p[i].w);
+        const int k = w == kNoClass ? -1 : class_slot(s_bits, w);
+        if (k < 0) {
+            s_over = 1;
+            continue;
+        }
+        const unsigned same = __match_any_sync(__activemask(), k);
+        if ((threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&s_count[k], __popc(same));
+    }
+    __syncthreads();
+    if (threadIdx.x < kMaxClasses && s_bits[threadIdx.x] != kNoClass) {
+        const int k = class_slot(out->bits, s_bits[threadIdx.x]);
+        if (k < 0) out->over = 1;
+        else atomicAdd(&out->count[k], s_count[threadIdx.x]);
+    }
+    if (threadIdx.x == 0 && s_over) out->over = 1;
+}
+
 __global__ void set_type_kernel(float4* p, int n, int32_t value) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i].w = __int_as_float(value);
 }
@@ -165,12 +213,17 @@ void radius_launch(const float4* a, int na, const float4* w, int nw, const float
     radius_kernel<<<(int)blocks, 256, 0, s>>>(a, na, w, nw, x, nx, st);
 }
 
-void typed_lists_launch(const float4* in, float4* dense, int n, const int32_t* ff_to_type, const TypedOut& o, int32_t* counts,
+void typed_lists_launch(const float4* in, float4* dense, int n, const TypeMap& map, const TypedOut& o, int32_t* counts,
                         cudaStream_t s) {
     if (n <= 0) return;
     const int chunks = typed_chunks(n);
-    dense_count_kernel<<<chunks, kTypedChunk, 0, s>>>(in, dense, n, ff_to_type, counts);
+    dense_count_kernel<<<chunks, kTypedChunk, 0, s>>>(in, dense, n, map, counts);
     typed_scatter_kernel<<<chunks, kTypedChunk, 0, s>>>(dense ? dense : in, n, o, counts);
+}
+
+void weight_classes_launch(const float4* p, int n, WeightClasses* out, int sm_count, cudaStream_t s) {
+    if (n <= 0) return;
+    weight_classes_kernel<<<std::min((n + 255) / 256, sm_count * 2), 256, 0, s>>>(p, n, out);
 }
 
 void set_type_launch(float4* p, int n, int32_t value, int sm_count, cudaStream_t s) {

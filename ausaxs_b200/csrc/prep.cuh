@@ -5,6 +5,15 @@
 
 namespace ausaxs_b200 {
 
+// The distinct weights of a point set (bit patterns, in the order they were met) and their points.
+constexpr int kMaxClasses = 15;
+constexpr unsigned kNoClass = 0xffffffffu;  // an empty slot (a NaN pattern)
+struct WeightClasses {
+    unsigned bits[16];
+    int count[16];
+    int over;  // more than kMaxClasses of them (or kNoClass itself)
+};
+
 struct PrepStats {
     unsigned int lo[3];  // order-preserving encodings of the bounding box
     unsigned int hi[3];
@@ -12,6 +21,7 @@ struct PrepStats {
     unsigned int bad;    // bit 0: invalid form-factor type, bit 1: non-finite coordinate
     int count[kNff];     // atoms per form-factor type
     unsigned long long r2;  // bits of max |p - c|^2 (double) over every point, c = centre of the box
+    WeightClasses weights[2];  // weighted structures: atoms, waters
 };
 
 void census_launch(const float4* p, int n, int ff_typed, PrepStats* st, int sm_count, cudaStream_t s);
@@ -34,10 +44,17 @@ struct TypedOut {
 };
 inline int typed_chunks(int n) { return (n + kTypedChunk - 1) / kTypedChunk; }
 inline int typed_pre_stride(int n) { return (n + kTypedPre - 1) / kTypedPre; }
-// dense (w = dense type through ff_to_type; in already dense: both null) and the lists, two kernels;
+// dense (w = dense type through the map; in already dense: no map and null) and the lists, two kernels;
 // counts: typed_chunks(n) * 16 ints of scratch
-void typed_lists_launch(const float4* in, float4* dense, int n, const int32_t* ff_to_type, const TypedOut& o, int32_t* counts,
+struct TypeMap {
+    const int32_t* ff_to_type = nullptr;  // form-factor type -> dense type
+    int classes = 0;                      // or the index of w's bit pattern among these
+    unsigned bits[16] = {};
+};
+void typed_lists_launch(const float4* in, float4* dense, int n, const TypeMap& map, const TypedOut& o, int32_t* counts,
                         cudaStream_t s);
+// the distinct weights of n points, added to *out (slots preset to kNoClass, counts to 0)
+void weight_classes_launch(const float4* p, int n, WeightClasses* out, int sm_count, cudaStream_t s);
 void set_type_launch(float4* p, int n, int32_t value, int sm_count, cudaStream_t s);
 float ordered_to_float(unsigned int o);
 

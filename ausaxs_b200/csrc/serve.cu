@@ -278,6 +278,7 @@ struct Assembly {
                 j.b_base = a_off[l];
                 j.tail_end = N;
                 j.tail_from_outer = 1;
+                j.t_out = T;
                 j.typed = &body_lists[l];
             } else if (pt.kind == 1) {  // aw: atoms of k outer, waters of l inner, rows over all waters
                 j.A = A + a_off[k];
@@ -488,7 +489,7 @@ struct Assembly {
                 std::memcpy(&f, atoms + 4 * (size_t)i + 3, 4);
                 ++count[S.ff_to_type[f]];  // validated by the load
             }
-            body_lists[k] = typed_lists(S.atoms_for_pairs() + a_off[k], nullptr, n, nullptr, S.T, count, lists.as<char>(list_off[k]),
+            body_lists[k] = typed_lists(S.atoms_for_pairs() + a_off[k], nullptr, n, TypeMap{}, S.T, count, lists.as<char>(list_off[k]),
                                         false, C.stream);
             C.check_launch("typed lists");
         }

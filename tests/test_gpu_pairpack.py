@@ -68,3 +68,31 @@ def test_grid_passes(gpu_ctx):
     waters = np.random.default_rng(1).normal(0, 14, (77, 3))
     x = np.random.default_rng(2).normal(0, 9, (1301, 3))  # off the lattice: dummy pairs through this kernel
     check(xyz, ff, waters, 0.1, gpu_ctx, x, True)
+
+
+@pytest.mark.parametrize("classes", [1, 2, 4, 15, 16, 700])
+@pytest.mark.parametrize("n,nw", [(5, 0), (257, 3), (1301, 300)])
+def test_weights_by_class(classes, n, nw, gpu_ctx):
+    """Weighted (Simple) histograms: up to 15 distinct weights go by class of weight, more by value.  A pair's
+    weight product is kept to max|w|^2 2^-30."""
+    rng = np.random.default_rng(classes)
+    xyz, _ = synth.globule(n + 1, n)
+    values = rng.uniform(-2, 16, classes)
+    w = values[rng.integers(0, classes, n)]
+    waters = rng.normal(0, 14, (nw, 3))
+    ww = np.full(nw, 9.25)
+    m = hist.Molecule(atoms=xyz, weights=w, waters=waters, water_weights=ww)
+    h = hist.HistogramManagerMT(m, True, 0.25, 8000, gpu_ctx).calculate_all()
+    sets = [hist.pack(xyz, w, False), hist.pack(waters, ww, False)]
+    jobs = [(0, None, 1, 0)] + ([(0, 1, 1, 0), (1, None, 1, 1)] if nw else [])
+    o = O.calculator(sets, jobs, 0.25, 8000)
+    top = max(np.abs(w).max(), ww.max() if nw else 0.0) ** 2
+    for got, key in ((h.get_aa_counts(), (0, 0)), (h.get_aw_counts(), (1, 0)), (h.get_ww_counts(), (0, 1))):
+        if key not in o:
+            assert not got.any()
+            continue
+        value, count, _ = o[key]
+        k = len(got)
+        # (the self diagonal in bin 0 is not quantised; its sum runs in another order)
+        assert np.all(np.abs(got - value[:k]) <= count[:k] * top * 2.0 ** -30 + 1e-12 * np.abs(value[:k]))
+        assert not value[k:].any() or not np.abs(value[k:]).max() > count[k:].max() * top * 2.0 ** -30
