@@ -522,6 +522,27 @@ bool choose_pack(const Plan& P, int sm_count, PackLaunch& L, int& shape, int& gr
     return true;
 }
 
+// The plan's launch of the one-atomic-per-pair kernel and its tables; false where it does not apply.
+bool Structure::upload_pack(Plan& P) {
+    PackTable table;
+    if (!choose_pack(P, ctx->sm_count, P.pack, P.pack_shape, P.pack_grid, table)) return false;
+    std::copy(type_count, type_count + T, P.type_count);
+    char* base = P.dev.as<char>();
+    const size_t jobs_bytes = sizeof(PackJob) * table.jobs.size(), out_bytes = sizeof(void*) * table.out.size();
+    if (jobs_bytes + out_bytes > P.off_acc - P.off_jobs) throw Error{AUSAXS_ERR_CAPACITY, "too many pair jobs"};
+    P.pack.covered = P.covered;  // this plan's coordinates; batches and servers launch their own tables
+    P.pack.jobs = reinterpret_cast<const PackJob*>(base + P.off_jobs);
+    P.pack.out = reinterpret_cast<unsigned long long* const*>(base + P.off_jobs + jobs_bytes);
+    P.pack.tile_counter = reinterpret_cast<unsigned long long*>(base + P.off_counter);
+    P.pack.overflow = reinterpret_cast<unsigned long long*>(base + P.off_overflow);
+    std::vector<char> bytes(jobs_bytes + out_bytes);
+    std::memcpy(bytes.data(), table.jobs.data(), jobs_bytes);
+    std::memcpy(bytes.data() + jobs_bytes, table.out.data(), out_bytes);
+    // pageable source: staged on return
+    AUSAXS_CUDA(cudaMemcpyAsync(base + P.off_jobs, bytes.data(), bytes.size(), cudaMemcpyHostToDevice, ctx->stream));
+    return true;
+}
+
 Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     Plan& P = plan;
     if (cfg.bin_width <= 0 || cfg.bin_count <= 0) throw Error{AUSAXS_ERR_ARGUMENT, "bin_width and bin_count must be positive"};
@@ -535,12 +556,17 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     const float inv_w = (float)(1.0 / cfg.bin_width);
     int nb = (int)std::ceil((double)(dmax + dmax_extra) * inv_w) + 2;
     nb = std::max(nb, 11);
+    const bool covered = nb <= cfg.bin_count;
     nb = std::min(nb, cfg.bin_count);
     if (P.manager == cfg.manager && P.weighted == weighted && P.bin_count == cfg.bin_count &&
         P.bin_width == cfg.bin_width && P.n_a == n_a && P.n_w == n_w && P.n_x == n_x && P.T == T && P.nb >= nb &&
         P.nb <= nb + 64 && (cfg.manager != AUSAXS_MANAGER_FFGRID || n_x < kLatticeMinPoints || lat.tried) &&
         std::equal(n_cls, n_cls + 2, P.n_cls) && std::memcmp(cls, P.cls, sizeof cls) == 0 &&
-        std::memcmp(cls_count, P.cls_count, sizeof cls_count) == 0 && std::equal(type_ff, type_ff + T, P.type_ff) && (!P.packed || std::equal(type_count, type_count + T, P.type_count))) {
+        std::memcmp(cls_count, P.cls_count, sizeof cls_count) == 0 && std::equal(type_ff, type_ff + T, P.type_ff)) {
+        // one-shot calls of one shape: only the lists by type have other lengths
+        if (P.packed && !std::equal(type_count, type_count + T, P.type_count)) upload_pack(P);
+        P.covered = covered;
+        P.pack.covered = covered;
         P.fin_ff.z_exv = cfg.z_exv;  // per call: other molecules of the same shape have other volumes
         return P;
     }
@@ -559,6 +585,7 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     std::copy(n_cls, n_cls + 2, P.n_cls);
     std::memcpy(P.cls, cls, sizeof cls);
     std::memcpy(P.cls_count, cls_count, sizeof cls_count);
+    P.covered = covered;
     P.row_share = 1.0;
     if (T > 0 && n_a > 0) P.row_share = (double)*std::max_element(type_count, type_count + T) / n_a;
     P.nb = nb;
@@ -749,23 +776,8 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
 
     pair_sqrt_prepare(P.inv_w, nb);  // once per width and process: the Newton-Raphson root where it bins exactly
     P.n_launch = 0;
-    PackTable table;
-    P.packed = (!mt || by_class) && choose_pack(P, C.sm_count, P.pack, P.pack_shape, P.pack_grid, table);
-    if (P.packed) {
-        const size_t jobs_bytes = sizeof(PackJob) * table.jobs.size();
-        if (jobs_bytes + sizeof(void*) * table.out.size() > P.off_acc - P.off_jobs)
-            throw Error{AUSAXS_ERR_CAPACITY, "too many pair jobs"};
-        P.pack.jobs = reinterpret_cast<const PackJob*>(base + P.off_jobs);
-        P.pack.out = reinterpret_cast<unsigned long long* const*>(base + P.off_jobs + jobs_bytes);
-        P.pack.tile_counter = reinterpret_cast<unsigned long long*>(base + P.off_counter);
-        P.pack.overflow = reinterpret_cast<unsigned long long*>(base + P.off_overflow);
-        // pageable sources: staged on return
-        AUSAXS_CUDA(cudaMemcpyAsync(base + P.off_jobs, table.jobs.data(), jobs_bytes, cudaMemcpyHostToDevice, C.stream));
-        AUSAXS_CUDA(cudaMemcpyAsync(base + P.off_jobs + jobs_bytes, table.out.data(), sizeof(void*) * table.out.size(),
-                                    cudaMemcpyHostToDevice, C.stream));
-    } else {
-        plan_groups(P, base, C);
-    }
+    P.packed = (!mt || by_class) && upload_pack(P);
+    if (!P.packed) plan_groups(P, base, C);
 
     // finalisation (its counter is cleared with the accumulators, or here where they are not)
     AUSAXS_CUDA(cudaMemsetAsync(base + P.off_maxbin, 0, 256, C.stream));

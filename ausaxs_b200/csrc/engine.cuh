@@ -119,6 +119,7 @@ struct Plan {
     int pack_shape = 0, pack_grid = 0;
     long long pairs = 0;
     int R = 0;
+    bool covered = false;  // the bins cover every distance of the planned coordinates
     double row_share = 1;  // share of the most frequent atom type
     float inv_w = 0, c = 0, scale = 0;
     // device layout
@@ -193,6 +194,7 @@ struct Structure {
     int32_t hmeta[2 * kNff] = {};  // host copy of meta (type counts, ff -> dense type)
     const float4* atoms_for_pairs() const { return ff_typed ? dense_a.as<float4>() : raw_a.as<float4>(); }
     Plan& plan_for(const ausaxs_hist_config& cfg);
+    bool upload_pack(Plan& P);
     void enqueue_histogram(const ausaxs_hist_config& cfg);
     void enqueue_debye(const ausaxs_hist_config& cfg, const double* q_dev, int nq, const ausaxs_debye_params& p,
                        double* Iq_dev, double* prof_dev);

@@ -128,7 +128,7 @@ struct Consts {
 
 // Four inner points (one quad) against the thread's R outer points.  MASK: only inner positions in
 // [p[k], kt) of outer point k are valid; n counts the valid pairs.
-template <bool MASK, int R, int NR, bool DSUM>
+template <bool MASK, int R, int NR, bool DSUM, bool CLAMP>
 __device__ __forceinline__ void quad_pairs(const Quad* __restrict__ q, int k0, const u64 (&ox)[R], const u64 (&oy)[R],
                                            const u64 (&oz)[R], const uint32_t (&caddr)[R], const int (&p)[R], int kt,
                                            const Consts& K, int& n) {
@@ -151,10 +151,13 @@ __device__ __forceinline__ void quad_pairs(const Quad* __restrict__ q, int k0, c
             unpack2(d0, d00, d01);
             u64 d = fma2(pack2(__fmaf_rn(-d00, d00, s0), __fmaf_rn(-d01, d01, s1)), h, d0);
             // distances past the last bin (also NaN and inf) become that of the overflow column's centre,
-            // so that every added value is 2^23 + an offset below 2^16
-            float d1v, d0v;
-            unpack2(d, d0v, d1v);
-            d = pack2(fminf(d0v, K.dmax), fminf(d1v, K.dmax));
+            // so that every added value is 2^23 + an offset below 2^16.  Launches whose bins cover every
+            // distance (PackLaunch::covered) leave that out: one instruction of 17 per pair.
+            if (CLAMP) {
+                float d1v, d0v;
+                unpack2(d, d0v, d1v);
+                d = pack2(fminf(d0v, K.dmax), fminf(d1v, K.dmax));
+            }
             // bin by the magic number; a power-of-two width (NR == 2) fuses the product
             const u64 xm = NR == 2 ? fma2(d, K.iw, K.mg) : add2(product2(d, K.iw), K.mg);
             float x0, x1;
@@ -238,7 +241,7 @@ __host__ __device__ inline int pack_pad(int bins) { return (bins + 4) & ~3; }
 // at 16 warps, 1,702 at 32), so up to 102 registers per thread buy a loop without spills.
 constexpr int pack_min_blocks(int threads) { return threads >= 512 ? 1 : 640 / threads; }
 
-template <int NT, int G, int NR, bool DSUM>
+template <int NT, int G, int NR, bool DSUM, bool CLAMP>
 __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const PackLaunch L) {
     constexpr int R = 2;
     constexpr int NTG = NT / G;
@@ -501,12 +504,12 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
                 }
                 const int m0 = min(qb, max(qa, mq0)), m1 = max(m0, min(qb, mq1));
                 for (int q = max(qa, q_warp); q < m0; ++q)
-                    quad_pairs<true, R, NR, DSUM>(s_q + q, 4 * q, ox, oy, oz, caddr, p, kt, K, n);
+                    quad_pairs<true, R, NR, DSUM, CLAMP>(s_q + q, 4 * q, ox, oy, oz, caddr, p, kt, K, n);
 #pragma unroll 4
-                for (int q = m0; q < m1; ++q) quad_pairs<false, R, NR, DSUM>(s_q + q, 0, ox, oy, oz, caddr, p, kt, K, n);
+                for (int q = m0; q < m1; ++q) quad_pairs<false, R, NR, DSUM, CLAMP>(s_q + q, 0, ox, oy, oz, caddr, p, kt, K, n);
                 n += (m1 - m0) * (4 * R);
                 for (int q = max(m1, q_warp); q < qb; ++q)
-                    quad_pairs<true, R, NR, DSUM>(s_q + q, 4 * q, ox, oy, oz, caddr, p, kt, K, n);
+                    quad_pairs<true, R, NR, DSUM, CLAMP>(s_q + q, 4 * q, ox, oy, oz, caddr, p, kt, K, n);
             }
             if (!fetched) {
                 // every thread left the other buffer at the previous tile's last barrier
@@ -621,19 +624,19 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
 
 using Kernel = void (*)(const PackLaunch);
 
-template <int NT, int G>
+template <int NT, int G, bool CLAMP>
 Kernel pick(int nr, bool dsum) {
-    if (nr == 2) return dsum ? pack_kernel<NT, G, 2, true> : pack_kernel<NT, G, 2, false>;
-    return dsum ? pack_kernel<NT, G, 1, true> : pack_kernel<NT, G, 1, false>;
+    if (nr == 2) return dsum ? pack_kernel<NT, G, 2, true, CLAMP> : pack_kernel<NT, G, 2, false, CLAMP>;
+    return dsum ? pack_kernel<NT, G, 1, true, CLAMP> : pack_kernel<NT, G, 1, false, CLAMP>;
 }
 
-Kernel kernel_of(int shape, int nr, bool dsum) {
+template <bool CLAMP>
+Kernel pick_shape(int shape, int nr, bool dsum) {
     switch (shape) {
-        case 0: return pick<128, 1>(nr, dsum);
-        case 1: return pick<256, 1>(nr, dsum);
-        case 2: return pick<256, 2>(nr, dsum);
-        case 3: return pick<512, 2>(nr, dsum);
-        default: return pick<512, 4>(nr, dsum);
+        case 0: return pick<128, 1, CLAMP>(nr, dsum);
+        case 1: return pick<256, 1, CLAMP>(nr, dsum);
+        case 2: return pick<256, 2, CLAMP>(nr, dsum);
+        default: return pick<512, 2, CLAMP>(nr, dsum);
     }
 }
 
@@ -666,7 +669,7 @@ int pack_segment_pairs(int bins, double largest_row_share) {
 
 void pack_launch(const PackLaunch& L, int shape, int grid, cudaStream_t s) {
     const size_t smem = pack_smem_bytes(L);
-    Kernel k = kernel_of(shape, L.nr, L.offsets != 0);
+    Kernel k = L.covered ? pick_shape<false>(shape, L.nr, L.offsets != 0) : pick_shape<true>(shape, L.nr, L.offsets != 0);
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     k<<<grid, kPackShapes[shape].threads, smem, s>>>(L);
 }

@@ -44,6 +44,7 @@ struct PackLaunch {
     unsigned long long* overflow;
     int32_t nr;           // 1: every job's width is verified for the Newton-Raphson root; 2: and is a power of two
     int32_t offsets;      // 0: no job has offset sums (counts only)
+    int32_t covered;      // 1: no pair's distance lies beyond its job's bins
     int32_t max_tiles;    // > 0: a CTA exits after this many tiles (grid * max_tiles >= total_tiles)
 };
 
@@ -57,7 +58,7 @@ struct PackShape {
     int threads, groups;
     int outer() const { return threads / groups * 2; }
 };
-constexpr PackShape kPackShapes[] = {{128, 1}, {256, 1}, {256, 2}, {512, 2}, {512, 4}};
+constexpr PackShape kPackShapes[] = {{128, 1}, {256, 1}, {256, 2}, {512, 2}};
 
 // footprint of a launch with L's rows, bins and tile_j
 size_t pack_smem_bytes(const PackLaunch& L);
