@@ -42,8 +42,6 @@ constexpr double kRhoWater = 0.334;        // e / A^3 (include/core/constants/Co
 constexpr double kAvgRadius = 1.62;        // A (Constants.h:90)
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kCB = 128;                       // bins per staged chunk
-constexpr int kRG = 32;                        // rows per group of register accumulators
 constexpr int kMaxRows = 264;
 
 // Excluded volume (A^3) per form_factor_t for explicit excluded volume: the reference's default set
@@ -166,32 +164,53 @@ __global__ void debye_qfactors_kernel(DebyeArgs A, double* out) {
     q_factor(A, A.q[i >> 5], i & 31, F);
 }
 
-// q values per CTA by the transform's q count: 4 up to 256 q, 8 up to 1,024, 16 beyond.  The
-// decomposition depends on nq alone, so a structure's I(q) has the same bits alone or in a batch.
-constexpr int debye_qt(int nq) { return nq <= 256 ? 4 : (nq <= 1024 ? 8 : 16); }
+// q values per CTA by the transform's q count: few enough that small transforms reach most SMs (200 q: 100
+// CTAs), more for larger ones, whose CTAs then share every row they read.  The decomposition depends on
+// nq alone, so a structure's I(q) has the same bits alone or in a batch.
+constexpr int debye_qt(int nq) { return nq <= 296 ? 2 : (nq <= 592 ? 4 : (nq <= 2368 ? 8 : 16)); }
 
-// Layout of a CTA of QT q values: thread (warp w, lane l) owns q value l % QT and bin phase
-// w * (32 / QT) + l / QT of the CTA's 256 / QT phases; a phase holds 128 QT / 256 bins of each chunk.
-// Shared memory: per-q factors, the staged H chunk (reused as the cross-warp reduction buffer), the
-// staged axis chunk, the row sums [QT][R] and the rows' distance-axis groups.
+// Shared memory of a CTA of QT q values: per-q factors, the chunk's sinc values [kCB][QT], the row sums
+// [QT][R] and the rows' distance-axis groups.
 template <int QT>
 struct QTile {
-    static constexpr int kSubs = 32 / QT;
-    static constexpr int kPhases = kThreads / QT;
-    static constexpr int kBinsPerThread = kCB / kPhases;
-    static constexpr size_t kOffRed = ((sizeof(QFactors) * QT + 15) / 16) * 16;
-    static constexpr size_t kOffH = kOffRed;
-    static constexpr size_t kOffAx = kOffH + sizeof(double) * kRG * kCB;
-    static constexpr size_t kOffAcc = kOffAx + sizeof(double) * kCB;
+    static constexpr int kCB = 4096 / QT;  // bins per chunk: 32 KB of sinc values
+    static constexpr size_t kOffS = ((sizeof(QFactors) * QT + 15) / 16) * 16;
+    static constexpr size_t kOffAcc = kOffS + sizeof(double) * kCB * QT;
     static constexpr size_t smem(int R) { return kOffAcc + sizeof(double) * QT * R + sizeof(int) * R; }
-    static_assert(kWarps * kRG * QT <= kRG * kCB, "the reduction buffer must fit in the H chunk");
-    static_assert(kBinsPerThread * kPhases == kCB, "a chunk must split evenly into phases");
 };
 
-// One CTA evaluates QT consecutive q values of one transform.  Each thread evaluates sinc(q d_b) for
-// its q value and the bins of its phase in each 128-bin chunk once and adds H[r][b] sinc into one
-// register accumulator per row (rows in groups of 32).  A (row, q) sum is therefore one serial sum per
-// phase, in bin order, the phases of a warp added by shuffles and then the warps in order.
+// Sums of QT values over the warp: lane l ends with the sum of value qi(l) (halving exchanges: QT - 1 + 5 -
+// log2 QT shuffles instead of 5 QT).
+template <int QT>
+__device__ __forceinline__ double warp_sums(double (&v)[QT], int lane) {
+    int o = 16;
+#pragma unroll
+    for (int n = QT; n > 1; n >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < n / 2; ++i) {
+            const double keep = up ? v[i + n / 2] : v[i], give = up ? v[i] : v[i + n / 2];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+#pragma unroll
+    for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+template <int QT>
+__device__ __forceinline__ int warp_sum_index(int lane) {
+    int q = 0, o = 16;
+#pragma unroll
+    for (int n = QT; n > 1; n >>= 1, o >>= 1) q += (lane & o) ? n / 2 : 0;
+    return q;
+}
+
+// One CTA evaluates QT consecutive q values of one transform: per chunk of bins the sinc values of all its
+// q once, one per thread in turn, then a warp per row: the lanes take the row's bins (coalesced from
+// global memory, a row is read by one warp of the CTA only) against the QT staged values of the bin.  A
+// (row, q) sum is therefore one serial sum per lane and chunk, the lanes added by a fixed tree and the
+// chunks in order.  Bound: latency (FP64 sin, then one pass over the rows); staging H and a register
+// accumulator per row in every thread, as before, took three times the instructions per warp.
 template <int QT>
 __device__ void debye_qtile(const DebyeArgs& A, const int q0, unsigned char* smem) {
     using T = QTile<QT>;
@@ -200,9 +219,7 @@ __device__ void debye_qtile(const DebyeArgs& A, const int q0, unsigned char* sme
     const int R = A.R;
     const int mb = *A.max_bin;
     QFactors* s_F = reinterpret_cast<QFactors*>(smem);
-    double* s_red = reinterpret_cast<double*>(smem + T::kOffRed);  // [kWarps][kRG][QT]
-    double* s_h = reinterpret_cast<double*>(smem + T::kOffH);      // [kRG][kCB]
-    double* s_ax = reinterpret_cast<double*>(smem + T::kOffAx);    // [kCB]
+    double* s_S = reinterpret_cast<double*>(smem + T::kOffS);      // [kCB][QT]
     double* s_acc = reinterpret_cast<double*>(smem + T::kOffAcc);  // [QT][R]
     int* s_grp = reinterpret_cast<int*>(smem + T::kOffAcc + sizeof(double) * QT * R);
     __shared__ int s_fp64[QT];
@@ -316,65 +333,44 @@ __device__ void debye_qtile(const DebyeArgs& A, const int q0, unsigned char* sme
     int any = 0;
     for (int qq = 0; qq < nqt; ++qq) any |= s_fp64[qq];
     if (any) {
-        const int qi = lane % QT, phase = warp * T::kSubs + lane / QT;
-        const bool qon = qi < nqt && s_fp64[qi] != 0;
-        const double q = qi < nqt ? A.q[q0 + qi] : 0.0;
         const int groups = s_groups;
-        for (int rg0 = 0; rg0 < R; rg0 += kRG) {
-            const int rn = min(kRG, R - rg0);
-            double acc[kRG];
+        for (int g = 0; g < groups; ++g) {
+            const double* axis = g == 0 ? A.axis0 : (g == 1 ? A.axis1 : A.axis2);
+            for (int c0 = 0; c0 < mb; c0 += T::kCB) {
+                const int cn = min(T::kCB, mb - c0);
+                __syncthreads();  // the previous chunk's values are read
+                for (int i = tid; i < cn * QT; i += kThreads) {
+                    const int qq = i % QT;
+                    s_S[i] = qq < nqt && s_fp64[qq] ? sinc64(A.q[q0 + qq] * axis[c0 + i / QT]) : 0.0;
+                }
+                __syncthreads();
+                for (int r = warp; r < R; r += kWarps) {
+                    if (s_grp[r] != g) continue;
+                    const double* h = A.H + static_cast<size_t>(r) * A.nb + c0;
+                    double v[QT];
 #pragma unroll
-            for (int i = 0; i < kRG; ++i) acc[i] = 0;
-            for (int g = 0; g < groups; ++g) {
-                const double* axis = g == 0 ? A.axis0 : (g == 1 ? A.axis1 : A.axis2);
-                for (int c0 = 0; c0 < mb; c0 += kCB) {
-                    const int cn = min(kCB, mb - c0);
-                    // the chunk's rows of H and axis values, coalesced, zero past the last bin
-                    __syncthreads();
-                    for (int i = tid; i < rn * kCB; i += kThreads) {
-                        const int r = i / kCB, t = i - r * kCB;
-                        s_h[i] = t < cn ? A.H[static_cast<size_t>(rg0 + r) * A.nb + c0 + t] : 0.0;
-                    }
-                    for (int t = tid; t < kCB; t += kThreads) s_ax[t] = t < cn ? axis[c0 + t] : 0.0;
-                    __syncthreads();
-                    double sv[T::kBinsPerThread];
+                    for (int k = 0; k < QT; ++k) v[k] = 0;
+#pragma unroll 4
+                    for (int t = lane; t < cn; t += 32) {
+                        const double hv = h[t];
+                        const double2* sv = reinterpret_cast<const double2*>(s_S + t * QT);
 #pragma unroll
-                    for (int k = 0; k < T::kBinsPerThread; ++k) {
-                        const int t = phase + k * T::kPhases;
-                        sv[k] = (qon && t < cn) ? sinc64(q * s_ax[t]) : 0.0;
-                    }
-#pragma unroll
-                    for (int i = 0; i < kRG; ++i) {
-                        if (i < rn && s_grp[rg0 + i] == g) {
-                            const double* h = s_h + i * kCB + phase;
-                            double a = acc[i];
-#pragma unroll
-                            for (int k = 0; k < T::kBinsPerThread; ++k) a += h[k * T::kPhases] * sv[k];
-                            acc[i] = a;
+                        for (int k = 0; k < QT / 2; ++k) {
+                            const double2 p = sv[k];
+                            v[2 * k] += hv * p.x;
+                            v[2 * k + 1] += hv * p.y;
                         }
                     }
+                    const double sum = warp_sums<QT>(v, lane);
+                    const int qq = warp_sum_index<QT>(lane);
+                    if ((lane & (32 / QT - 1)) == 0 && qq < nqt && s_fp64[qq]) {
+                        double* a = s_acc + qq * R + r;
+                        *a = c0 == 0 ? sum : *a + sum;
+                    }
                 }
             }
-            // the two phases of a warp by a shuffle, then the warps in order
-            __syncthreads();  // every thread is done with the staged chunk the buffer overlays
-#pragma unroll
-            for (int i = 0; i < kRG; ++i) {
-                double v = acc[i];
-#pragma unroll
-                for (int o = QT; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                if (lane < QT && i < rn) s_red[(warp * kRG + i) * QT + qi] = v;
-            }
-            __syncthreads();
-            for (int i = tid; i < rn * QT; i += kThreads) {
-                const int r = i / QT, qq = i - r * QT;
-                if (qq < nqt && s_fp64[qq]) {
-                    double v = 0;
-                    for (int w = 0; w < kWarps; ++w) v += s_red[(w * kRG + r) * QT + qq];
-                    s_acc[qq * R + rg0 + r] = v;
-                }
-            }
-            __syncthreads();
         }
+        __syncthreads();
     }
 
     for (int qq = warp; qq < nqt; qq += kWarps) {
@@ -427,7 +423,7 @@ bool debye_configure_qt() {
 }
 bool debye_configure() {
     static bool done = false;
-    if (!done) done = debye_configure_qt<4>() && debye_configure_qt<8>() && debye_configure_qt<16>();
+    if (!done) done = debye_configure_qt<2>() && debye_configure_qt<4>() && debye_configure_qt<8>() && debye_configure_qt<16>();
     return done;
 }
 
@@ -444,6 +440,7 @@ void debye_qfactors_launch(const DebyeArgs& A, double* out, cudaStream_t s) {
 void debye_fp64_launch(const DebyeArgs& A, cudaStream_t s) {
     debye_configure();
     switch (debye_qt(A.nq)) {
+        case 2: debye_kernel<2><<<(A.nq + 1) / 2, kThreads, QTile<2>::smem(A.R), s>>>(A); break;
         case 4: debye_kernel<4><<<(A.nq + 3) / 4, kThreads, QTile<4>::smem(A.R), s>>>(A); break;
         case 8: debye_kernel<8><<<(A.nq + 7) / 8, kThreads, QTile<8>::smem(A.R), s>>>(A); break;
         default: debye_kernel<16><<<(A.nq + 15) / 16, kThreads, QTile<16>::smem(A.R), s>>>(A); break;
@@ -452,6 +449,7 @@ void debye_fp64_launch(const DebyeArgs& A, cudaStream_t s) {
 void debye_fp64_batch_launch(const DebyeArgs* As_dev, int n, int nq, int max_R, cudaStream_t s) {
     debye_configure();
     switch (debye_qt(nq)) {
+        case 2: debye_batch_kernel<2><<<dim3((nq + 1) / 2, n), kThreads, QTile<2>::smem(max_R), s>>>(As_dev); break;
         case 4: debye_batch_kernel<4><<<dim3((nq + 3) / 4, n), kThreads, QTile<4>::smem(max_R), s>>>(As_dev); break;
         case 8: debye_batch_kernel<8><<<dim3((nq + 7) / 8, n), kThreads, QTile<8>::smem(max_R), s>>>(As_dev); break;
         default:
