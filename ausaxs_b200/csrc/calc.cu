@@ -33,18 +33,41 @@ struct CalcSlot {
     double* out;        // [3][nb]: value, count, distance sum
 };
 
+// Weights of few distinct values: a slot's counts are rows by the two points' classes, [n][n][nb]
+struct CalcClasses {
+    int n;  // 0: one row, and weight sums
+    float w[16];
+    float wscale;
+};
+
 __device__ __forceinline__ double unbiased_weights(const long long* w, const unsigned long long* n, int b, double inv) {
     const unsigned long long raw = static_cast<unsigned long long>(w[b]) - n[b] * (1ull << 30);
     return static_cast<double>(static_cast<long long>(raw)) * inv;
 }
 
 // grid.y = slot; the nb accumulated bins (every later bin is zero)
-__global__ void calc_finalize_kernel(const CalcSlot* slots, int nb, const float* wscale, float c, float scale) {
+__global__ void calc_finalize_kernel(const CalcSlot* slots, int nb, const float* wscale, float c, float scale, CalcClasses K) {
     const CalcSlot S = slots[blockIdx.y];
-    const double inv = 1.0 / static_cast<double>(*wscale);
+    const double inv = 1.0 / static_cast<double>(K.n ? K.wscale : *wscale);
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-        const unsigned long long cnt = S.cnt[b];
-        double v = 2.0 * unbiased_weights(S.ws, S.cnt, b, inv);
+        unsigned long long cnt = 0;
+        double v;
+        if (K.n) {
+            // the fixed-point weight product of every class pair times its pairs: the sum the weighted
+            // kernel accumulates pair by pair
+            long long w = 0;
+            for (int i = 0; i < K.n; ++i)
+#pragma unroll 4
+                for (int j = 0; j < K.n; ++j) {
+                    const unsigned long long n = S.cnt[static_cast<size_t>(i * K.n + j) * nb + b];
+                    cnt += n;
+                    w += static_cast<long long>(n) * __float2int_rn(__fmul_rn(__fmul_rn(K.w[i], K.w[j]), K.wscale));
+                }
+            v = 2.0 * (static_cast<double>(w) * inv);
+        } else {
+            cnt = S.cnt[b];
+            v = 2.0 * unbiased_weights(S.ws, S.cnt, b, inv);
+        }
         double n = 2.0 * static_cast<double>(cnt);
         double d = 0;
         if (cnt) {
@@ -87,7 +110,6 @@ struct Calculator {
         int index;  // position among the results of its kind (the reference's res_idx)
     };
     std::vector<SlotInfo> slot_info;
-    DevBuf points, acc, table, out;
     std::vector<double> results;  // [slots][3][bin_count] of the last run
     std::vector<SlotInfo> result_info;
 
@@ -131,14 +153,77 @@ struct Calculator {
         results.assign((size_t)n_slots * 3 * bin_count, 0.0);
         result_info = slot_info;
         if (n_slots == 0) return clear();
+        // the points, and every set's distinct weights, counted while the host finds the largest distance
+        // (buffers of the context: a calculator lives for one run, and allocating took longer than the pairs)
+        struct Keep {
+            Ctx& C;
+            ~Keep() {
+                for (DevBuf& b : C.calc)
+                    if (b.n > Ctx::kCalcKeep) b.release();
+            }
+        } keep{C};
+        DevBuf &in = C.calc[0], &acc = C.calc[1], &out = C.calc[2], &table = C.calc[3];
+        const size_t pts_bytes = align_up(std::max<size_t>(1, staged.size()) * 16, 256);
+        size_t list_bytes = 256;
+        for (const Set& q : sets) list_bytes += align_up(Structure::typed_bytes(q.n), 256);
+        const size_t jobs_bytes_in = align_up(sizeof(TypedSetJob) * std::max<size_t>(1, sets.size()), 256);
+        const size_t class_bytes = align_up(sizeof(WeightClasses) * std::max<size_t>(1, sets.size()), 256);
+        in.ensure(2 * pts_bytes + list_bytes + jobs_bytes_in + class_bytes);
+        DevBuf points, dense, lists, set_jobs, classes;
+        points.view(in.p, pts_bytes);
+        dense.view(in.as<char>(pts_bytes), pts_bytes);
+        lists.view(in.as<char>(2 * pts_bytes), list_bytes);
+        set_jobs.view(in.as<char>(2 * pts_bytes + list_bytes), jobs_bytes_in);
+        classes.view(in.as<char>(2 * pts_bytes + list_bytes + jobs_bytes_in), class_bytes);
+        AUSAXS_CUDA(cudaMemcpyAsync(points.p, staged.data(), staged.size() * 16, cudaMemcpyHostToDevice, s));
+        const float4* P = points.as<float4>();
+        const int n_sets = (int)sets.size();
+        int max_n = 0;
+        std::vector<TypedSetJob> sj(n_sets);
+        std::vector<WeightClasses> wc(n_sets);
+        size_t list_at = 0;
+        for (int k = 0; k < n_sets; ++k) {
+            const int n = sets[k].n;
+            char* mem = lists.as<char>(list_at);
+            list_at += align_up(Structure::typed_bytes(n), 256);
+            sj[k] = TypedSetJob{};
+            sj[k].in = P + sets[k].off;
+            sj[k].dense = dense.as<float4>() + sets[k].off;
+            sj[k].counts = reinterpret_cast<int32_t*>(mem + typed_off_counts(n));
+            sj[k].n = n;
+            sj[k].out.pts = reinterpret_cast<float4*>(mem);
+            sj[k].out.pre = reinterpret_cast<int32_t*>(mem + typed_off_pre(n));
+            sj[k].out.pre_stride = typed_pre_stride(n);
+            max_n = std::max(max_n, n);
+            std::fill(wc[k].bits, wc[k].bits + 16, kNoClass);
+            std::fill(wc[k].count, wc[k].count + 16, 0);
+            wc[k].over = 0;
+        }
+        if (max_n > 0) {
+            // pageable sources: staged on return
+            AUSAXS_CUDA(cudaMemcpyAsync(set_jobs.p, sj.data(), sizeof(TypedSetJob) * n_sets, cudaMemcpyHostToDevice, s));
+            AUSAXS_CUDA(cudaMemcpyAsync(classes.p, wc.data(), sizeof(WeightClasses) * n_sets, cudaMemcpyHostToDevice, s));
+            weight_classes_sets_launch(set_jobs.as<TypedSetJob>(), n_sets, max_n, classes.as<WeightClasses>(), s);
+            C.check_launch("calculator weight classes");
+        }
         // the largest pair distance: min(box diagonal, 2 x radius about the box centre) over all points
         double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-        for (const float4& p : staged) {
-            const double v[3] = {p.x, p.y, p.z};
+        std::vector<double> radius(n_sets, 0.0);  // half the largest extent of every set
+        for (int k = 0; k < n_sets; ++k) {
+            double slo[3] = {INFINITY, INFINITY, INFINITY}, shi[3] = {-INFINITY, -INFINITY, -INFINITY};
+            const float4* q = staged.data() + sets[k].off;
+            for (int i = 0; i < sets[k].n; ++i) {
+                const double v[3] = {q[i].x, q[i].y, q[i].z};
+                for (int d = 0; d < 3; ++d) {
+                    if (!std::isfinite(v[d])) throw Error{AUSAXS_ERR_ARGUMENT, "non-finite coordinate"};
+                    slo[d] = std::min(slo[d], v[d]);
+                    shi[d] = std::max(shi[d], v[d]);
+                }
+            }
             for (int d = 0; d < 3; ++d) {
-                if (!std::isfinite(v[d])) throw Error{AUSAXS_ERR_ARGUMENT, "non-finite coordinate"};
-                lo[d] = std::min(lo[d], v[d]);
-                hi[d] = std::max(hi[d], v[d]);
+                lo[d] = std::min(lo[d], slo[d]);
+                hi[d] = std::max(hi[d], shi[d]);
+                if (sets[k].n) radius[k] = std::max(radius[k], 0.5 * (shi[d] - slo[d]));
             }
         }
         double dmax = 0;
@@ -157,26 +242,80 @@ struct Calculator {
         const float inv_w = (float)(1.0 / bin_width);
         int nb = (int)std::ceil(dmax * inv_w) + 2;
         nb = std::max(nb, 11);
+        const bool covered = nb <= bin_count;
         nb = std::min(nb, bin_count);
+        // the classes of all sets together (ascending bit patterns): K.n 0 when there are more than kMaxClasses
+        CalcClasses K{};
+        TypeMap map;
+        std::vector<TypedSet> typed(n_sets);
+        if (max_n > 0) {
+            AUSAXS_CUDA(cudaMemcpyAsync(wc.data(), classes.p, sizeof(WeightClasses) * n_sets, cudaMemcpyDeviceToHost, s));
+            AUSAXS_CUDA(cudaStreamSynchronize(s));
+            std::map<unsigned, int> found;
+            bool few = true;
+            long long total = 0;
+            for (const WeightClasses& w : wc) {
+                few = few && !w.over;
+                for (int i = 0; i < kMaxClasses; ++i)
+                    if (w.bits[i] != kNoClass) found[w.bits[i]] += w.count[i], total += w.count[i];
+            }
+            pair_sqrt_prepare(inv_w, nb);
+            PackLaunch fit{};
+            fit.nr = pair_sqrt_mode(inv_w, nb);
+            fit.rows = fit.group_rows = (int)found.size();
+            fit.group_sums = fit.offsets = 1;
+            fit.bins = nb;
+            fit.tile_j = kPackMaxTileJ;
+            if (few && found.size() <= (size_t)kMaxClasses && fit.nr > 0 && pack_shape(fit) >= 0) {
+                float m = 0;
+                int most = 0;
+                for (auto& f : found) {
+                    map.bits[K.n] = f.first;
+                    std::memcpy(&K.w[K.n], &f.first, 4);
+                    m = std::max(m, std::fabs(K.w[K.n]));
+                    most = std::max(most, f.second);
+                    ++K.n;
+                }
+                map.classes = K.n;
+                class_share = (double)most / total;
+                const double p = (double)m * m;  // as weight_scale_launch
+                int e = 0;
+                if (p > 0) std::frexp(p, &e);
+                K.wscale = std::ldexp(1.0f, std::min(60, 30 - e));
+                for (int k = 0; k < n_sets; ++k) {
+                    TypedSet& t = typed[k];
+                    t.pts = sj[k].out.pts;
+                    t.pre = sj[k].out.pre;
+                    t.pre_stride = sj[k].out.pre_stride;
+                    t.types = sj[k].out.types = K.n;
+                    for (int i = 0; i < kMaxClasses; ++i)
+                        if (wc[k].bits[i] != kNoClass) t.count[std::distance(found.begin(), found.find(wc[k].bits[i]))] = wc[k].count[i];
+                    for (int i = 0, at = 0; i < K.n; ++i) {
+                        t.start[i] = sj[k].out.start[i] = at;
+                        at += t.count[i];
+                    }
+                }
+            }
+        }
+        const int n_rows = K.n ? K.n * K.n : 1;  // count rows of a slot
         if (pairhist_launch_smem(1, nb, true, 512) > kPairSmemCap)
             throw Error{AUSAXS_ERR_CAPACITY, "too many distance bins for the on-chip histogram"};
 
-        // device layout: points, per slot [cnt | ds | ws] (nb each), outputs, slot table, counters
-        const size_t pts_bytes = align_up(std::max<size_t>(1, staged.size()) * 16, 256);
-        points.ensure(pts_bytes);
-        AUSAXS_CUDA(cudaMemcpyAsync(points.p, staged.data(), staged.size() * 16, cudaMemcpyHostToDevice, s));
+        // device layout: per slot [cnt rows | ds | ws] (nb each), outputs, slot table, counters
         const size_t row = align_up((size_t)nb * 8, 256);
-        const size_t acc_bytes = (size_t)n_slots * 3 * row + 1024;
+        const size_t slot_bytes = align_up((size_t)n_rows * nb * 8, 256) + 2 * row;
+        const size_t acc_bytes = (size_t)n_slots * slot_bytes + 1024;
         acc.ensure(acc_bytes);
         AUSAXS_CUDA(cudaMemsetAsync(acc.p, 0, acc_bytes, s));
         char* ab = acc.as<char>();
-        unsigned long long* counter = reinterpret_cast<unsigned long long*>(ab + (size_t)n_slots * 3 * row);
+        unsigned long long* counter = reinterpret_cast<unsigned long long*>(ab + (size_t)n_slots * slot_bytes);
         unsigned long long* overflow = counter + 4;
         float* wscale = reinterpret_cast<float*>(counter + 8);
         out.ensure((size_t)n_slots * 3 * nb * 8);
-        const float4* P = points.as<float4>();
-        weight_scale_launch(P, (int)staged.size(), P, 0, wscale, s);
-        C.check_launch("calculator weight scale");
+        if (!K.n) {
+            weight_scale_launch(P, (int)staged.size(), P, 0, wscale, s);
+            C.check_launch("calculator weight scale");
+        }
 
         Plan plan;  // job-building view
         plan.T = 1;
@@ -185,11 +324,23 @@ struct Calculator {
         plan.c = (float)(1.0 / (double)inv_w);
         plan.scale = (float)(32768.0 / (double)plan.c * (1.0 - 1.0 / 256));
         plan.max_group_rows = 1;
+        plan.weighted = 1;
+        plan.row_share = class_share;
+        const float4* D = K.n ? dense.as<float4>() : P;  // outer points carry their class
+        auto by_class = [&](JobSpec& sp, int outer, int inner) {
+            if (!K.n) return;
+            sp.spread_bins = std::max(16, (int)(0.7 * (radius[outer] + radius[inner]) * inv_w));
+            sp.rmode = kRowPair;
+            sp.rows = n_rows;
+            sp.t_out = K.n;
+            sp.typed = &typed[inner];
+            sp.wsum = nullptr;
+        };
         std::vector<CalcSlot> table_h(n_slots);
         for (int k = 0; k < n_slots; ++k) {
-            table_h[k].cnt = reinterpret_cast<unsigned long long*>(ab + (size_t)(3 * k) * row);
-            table_h[k].ds = reinterpret_cast<unsigned long long*>(ab + (size_t)(3 * k + 1) * row);
-            table_h[k].ws = reinterpret_cast<long long*>(ab + (size_t)(3 * k + 2) * row);
+            table_h[k].cnt = reinterpret_cast<unsigned long long*>(ab + (size_t)k * slot_bytes);
+            table_h[k].ds = reinterpret_cast<unsigned long long*>(ab + (size_t)(k + 1) * slot_bytes - 2 * row);
+            table_h[k].ws = reinterpret_cast<long long*>(ab + (size_t)(k + 1) * slot_bytes - row);
             table_h[k].diag_value = table_h[k].diag_count = 0;
             table_h[k].out = out.as<double>() + (size_t)k * 3 * nb;
         }
@@ -209,7 +360,8 @@ struct Calculator {
                 table_h[j.slot].diag_count += (double)(uint32_t)tw;
                 if (A.n < 2) continue;
                 JobSpec sp{};
-                sp.A = sp.B = P + A.off;
+                sp.A = D + A.off;
+                sp.B = P + A.off;
                 sp.na = sp.nbp = A.n;
                 sp.self = 1;
                 sp.rmode = kRowSingle;
@@ -218,6 +370,7 @@ struct Calculator {
                 sp.dsum = table_h[j.slot].ds;
                 sp.wsum = table_h[j.slot].ws;
                 sp.mult = j.scaling;
+                by_class(sp, j.a, j.a);
                 plan.specs.push_back(sp);
                 pairs += (long long)A.n * (A.n - 1) / 2;
                 biggest = std::max(biggest, A.n);
@@ -226,7 +379,7 @@ struct Calculator {
                 const Set& B = sets[j.b];
                 if (A.n == 0 || B.n == 0) continue;
                 JobSpec sp{};
-                sp.A = P + B.off;
+                sp.A = D + B.off;
                 sp.na = B.n;
                 sp.B = P + A.off;
                 sp.nbp = A.n;
@@ -237,48 +390,78 @@ struct Calculator {
                 sp.dsum = table_h[j.slot].ds;
                 sp.wsum = table_h[j.slot].ws;
                 sp.mult = j.scaling;
+                by_class(sp, j.b, j.a);
                 plan.specs.push_back(sp);
                 pairs += (long long)A.n * B.n;
                 biggest = std::max({biggest, A.n, B.n});
             }
         }
         const size_t table_bytes = align_up(sizeof(CalcSlot) * n_slots, 256);
-        std::vector<PairJob> pj[3];
-        long long tiles[3] = {0, 0, 0};
-        int rows[3] = {1, 1, 1};
-        const int tile = biggest >= 16384 ? 512 : 256;
-        append_pair_jobs(plan, tile, false, pj, tiles, rows);
-        table.ensure(table_bytes + align_up(sizeof(PairJob) * std::max<size_t>(1, pj[0].size()), 256));
-        AUSAXS_CUDA(cudaMemcpyAsync(table.p, table_h.data(), sizeof(CalcSlot) * n_slots, cudaMemcpyHostToDevice, s));
-        PairJob* jobs_dev = reinterpret_cast<PairJob*>(table.as<char>() + table_bytes);
-        if (!pj[0].empty()) {
-            AUSAXS_CUDA(cudaMemcpyAsync(jobs_dev, pj[0].data(), sizeof(PairJob) * pj[0].size(), cudaMemcpyHostToDevice, s));
-            PairLaunch L{};
-            L.jobs = jobs_dev;
-            L.n_jobs = (int)pj[0].size();
-            L.total_tiles = tiles[0];
-            L.smem_rows = 1;
-            L.smem_bins = nb;
-            L.tile_counter = counter;
-            L.overflow = overflow;
-            L.weighted = 1;
-            L.wscale = wscale;
-            L.dreg = 0;
-            L.inv_w = plan.inv_w;
-            pair_sqrt_prepare(plan.inv_w, nb);
-            const size_t smem = pairhist_launch_smem(1, nb, true, tile);
-            const int per_sm = pairhist_ctas_per_sm(smem, tile, false, true);
-            const int grid = (int)std::min<long long>((long long)C.sm_count * per_sm, std::max<long long>(1, tiles[0]));
-            L.chunk = (int)std::max<long long>(1, std::min<long long>(8, tiles[0] / ((long long)grid * 8)));
+        PackLaunch PL{};
+        PackTable PT;
+        int shape = 0, pack_grid = 0;
+        if (K.n && !plan.specs.empty()) {
+            AUSAXS_CUDA(cudaMemcpyAsync(set_jobs.p, sj.data(), sizeof(TypedSetJob) * n_sets, cudaMemcpyHostToDevice, s));
+            typed_sets_launch(set_jobs.as<TypedSetJob>(), n_sets, max_n, map, s);
+            C.check_launch("calculator typed lists");
+            C.launches += 1;  // two kernels
+            if (!choose_pack(plan, C.sm_count, PL, shape, pack_grid, PT, false))
+                throw Error{AUSAXS_ERR_CAPACITY, "too many distance bins for the on-chip histogram"};
+            const size_t jobs_bytes = sizeof(PackJob) * PT.jobs.size(), out_bytes = sizeof(void*) * PT.out.size();
+            std::vector<char> bytes(table_bytes + jobs_bytes + out_bytes);
+            std::memcpy(bytes.data(), table_h.data(), sizeof(CalcSlot) * n_slots);
+            std::memcpy(bytes.data() + table_bytes, PT.jobs.data(), jobs_bytes);
+            std::memcpy(bytes.data() + table_bytes + jobs_bytes, PT.out.data(), out_bytes);
+            table.ensure(bytes.size());
+            AUSAXS_CUDA(cudaMemcpyAsync(table.p, bytes.data(), bytes.size(), cudaMemcpyHostToDevice, s));
+            PL.jobs = reinterpret_cast<const PackJob*>(table.as<char>(table_bytes));
+            PL.out = reinterpret_cast<unsigned long long* const*>(table.as<char>(table_bytes + jobs_bytes));
+            PL.tile_counter = counter;
+            PL.overflow = overflow;
+            PL.covered = covered;
             cudaEvent_t ev;
             C.time_begin(0, &ev);
-            pairhist_launch(L, tile, grid, smem, s);
+            pack_launch(PL, shape, pack_grid, s);
             C.check_launch("calculator pairs");
             C.time_end(0, ev);
+        } else {
+            std::vector<PairJob> pj[3];
+            long long tiles[3] = {0, 0, 0};
+            int rows[3] = {1, 1, 1};
+            const int tile = biggest >= 16384 ? 512 : 256;
+            append_pair_jobs(plan, tile, false, pj, tiles, rows);
+            table.ensure(table_bytes + align_up(sizeof(PairJob) * std::max<size_t>(1, pj[0].size()), 256));
+            AUSAXS_CUDA(cudaMemcpyAsync(table.p, table_h.data(), sizeof(CalcSlot) * n_slots, cudaMemcpyHostToDevice, s));
+            PairJob* jobs_dev = reinterpret_cast<PairJob*>(table.as<char>() + table_bytes);
+            if (!pj[0].empty()) {
+                AUSAXS_CUDA(cudaMemcpyAsync(jobs_dev, pj[0].data(), sizeof(PairJob) * pj[0].size(), cudaMemcpyHostToDevice, s));
+                PairLaunch L{};
+                L.jobs = jobs_dev;
+                L.n_jobs = (int)pj[0].size();
+                L.total_tiles = tiles[0];
+                L.smem_rows = 1;
+                L.smem_bins = nb;
+                L.tile_counter = counter;
+                L.overflow = overflow;
+                L.weighted = 1;
+                L.wscale = wscale;
+                L.dreg = 0;
+                L.inv_w = plan.inv_w;
+                pair_sqrt_prepare(plan.inv_w, nb);
+                const size_t smem = pairhist_launch_smem(1, nb, true, tile);
+                const int per_sm = pairhist_ctas_per_sm(smem, tile, false, true);
+                const int grid = (int)std::min<long long>((long long)C.sm_count * per_sm, std::max<long long>(1, tiles[0]));
+                L.chunk = (int)std::max<long long>(1, std::min<long long>(8, tiles[0] / ((long long)grid * 8)));
+                cudaEvent_t ev;
+                C.time_begin(0, &ev);
+                pairhist_launch(L, tile, grid, smem, s);
+                C.check_launch("calculator pairs");
+                C.time_end(0, ev);
+            }
         }
         const int threads = 256;
         calc_finalize_kernel<<<dim3((unsigned)((nb + threads - 1) / threads), (unsigned)n_slots), threads, 0, s>>>(
-            reinterpret_cast<const CalcSlot*>(table.p), nb, wscale, plan.c, plan.scale);
+            reinterpret_cast<const CalcSlot*>(table.p), nb, wscale, plan.c, plan.scale, K);
         C.check_launch("calculator finalize");
         unsigned long long of = 0;
         AUSAXS_CUDA(cudaMemcpyAsync(&of, overflow, 8, cudaMemcpyDeviceToHost, s));
@@ -304,6 +487,7 @@ struct Calculator {
     }
 
     long long pairs_last = 0;
+    double class_share = 1;
 };
 
 }  // namespace ausaxs_b200

@@ -24,9 +24,14 @@ void DevBuf::ensure(size_t bytes) {
     n = bytes;
 }
 
-DevBuf::~DevBuf() {
+void DevBuf::release() {
     if (p && owned) cudaFree(p);
+    p = nullptr;
+    n = 0;
+    owned = true;
 }
+
+DevBuf::~DevBuf() { release(); }
 
 PrepStats* Ctx::stats_slots(size_t n) {
     if (n > n_stats_many) {
@@ -121,8 +126,8 @@ void Structure::load_begin(const float* atoms, int n_atoms, const float* waters,
 }
 
 // layout of Structure::typed: lists, prefix table, chunk counts, places
-static size_t typed_off_pre(int n) { return align_up((size_t)std::max(1, n) * 16, 256); }
-static size_t typed_off_counts(int n) { return typed_off_pre(n) + align_up((size_t)typed_pre_stride(n) * 4 * kMaxTypes + 4, 256); }
+size_t typed_off_pre(int n) { return align_up((size_t)std::max(1, n) * 16, 256); }
+size_t typed_off_counts(int n) { return typed_off_pre(n) + align_up((size_t)typed_pre_stride(n) * 4 * kMaxTypes + 4, 256); }
 static size_t typed_off_pos(int n) { return typed_off_counts(n) + align_up((size_t)typed_chunks(n) * 16 * 4 + 4, 256); }
 size_t Structure::typed_bytes(int n) { return typed_off_pos(n) + align_up((size_t)std::max(1, n) * 4, 256); }
 int32_t* Structure::typed_pos() const { return typed.as<int32_t>(typed_off_pos(n_a)); }
@@ -347,6 +352,7 @@ void append_pack_jobs(const Plan& P, int outer, bool joint, PackLaunch& L, PackT
             p.tail_from_outer = j.tail_from_outer >= 0 ? j.tail_from_outer : j.self;
             p.seg_pairs = pack_segment_pairs(j.spread_bins > 0 ? std::min(j.spread_bins, P.nb) : P.nb, share);
             p.cnt_row = rows;
+            p.mult = j.mult;
             for (int r = 0; r < p.rows; ++r) T.out.push_back(j.counts + (size_t)(pair_rows ? r * j.typed->types + t : r) * P.nb);
             rows += p.rows;
             if (j.dsum) {

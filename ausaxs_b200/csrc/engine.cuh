@@ -36,6 +36,7 @@ struct DevBuf {
     size_t n = 0;
     bool owned = true;  // false: a view into memory owned elsewhere (never grown or freed here)
     void ensure(size_t bytes);
+    void release();
     void view(void* ptr, size_t bytes) {
         p = ptr;
         n = bytes;
@@ -56,6 +57,9 @@ struct TypedSet {
     int start[16] = {}, count[16] = {};
 };
 
+// byte offsets of the prefix table and the chunk counts in a list's memory (Structure::typed_bytes)
+size_t typed_off_pre(int n);
+size_t typed_off_counts(int n);
 // The lists of `in` (typed_lists_launch) in mem (Structure::typed_bytes(n)); count: points of each type.
 TypedSet typed_lists(const float4* in, float4* dense, int n, const TypeMap& map, int types, const int* count, char* mem,
                      bool want_pos, cudaStream_t s);
@@ -235,6 +239,10 @@ struct Ctx {
     std::shared_ptr<GridExv> grid;  // molecular-grid workspace of one-shot calls (gridexv.cuh)
     std::shared_ptr<Hydrator> hyd;  // hydration workspace (hydrate.cuh)
     DevBuf io;                     // q / I(q) / profiles of one-shot host calls
+    // SimpleCalculator runs (each synchronises before it returns): points and lists, accumulators, outputs,
+    // tables; kept up to kCalcKeep bytes each
+    static constexpr size_t kCalcKeep = 256u << 20;
+    DevBuf calc[4];
     DevBuf tc;                     // tensor-core scratch of one-shot host calls
     XBufs x;                       // exact tensor-core transform of one-shot host calls
     int last_fp64_columns = 0;     // q values the last host transform evaluated in FP64

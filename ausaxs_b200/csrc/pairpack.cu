@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
     __syncthreads();
 
     int cur = -1, cur_group = -1, taken = 0;
-    int grp_out = 0, grp_rows = 0, grp_sums = 0, grp_bins = 0;
+    int grp_out = 0, grp_rows = 0, grp_sums = 0, grp_bins = 0, grp_mult = 1;
     int len = 1;         // quads per group of a segment
     int slow_left = 0;   // segments still to be evaluated with two atomics per pair
     int room = kRoom;    // what the u32 offset sums (in 2^23) and u16 counts (in 128) still hold for certain
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
                 s_sums[(r - grp_rows) * pad + b] = 0;
             }
             if (v) {
-                if (b < grp_bins) atomicAdd(L.out[grp_out + r] + b, static_cast<u64>(v));
+                if (b < grp_bins) atomicAdd(L.out[grp_out + r] + b, static_cast<u64>(v) * grp_mult);
                 else if (r < grp_rows) atomicAdd(L.overflow, static_cast<u64>(v));
             }
         }
@@ -374,6 +374,7 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
                 grp_rows = J.group_rows;
                 grp_sums = J.group_sums;
                 grp_bins = nb;
+                grp_mult = J.mult;
             }
             len = max(1, min(kMaxLen, J.seg_pairs / (NT * R * 4)));
             slow_left = 0;

@@ -27,7 +27,8 @@ struct alignas(16) PackJob {
     // group goes to out[group_out + r], offset sum s to out[group_out + group_rows + s].
     int32_t group, group_out, group_rows, group_sums;
     int32_t cnt_row, sum_slot;
-    int32_t pad[2];
+    int32_t mult;         // multiplicity of every pair (jobs of a group share it)
+    int32_t pad;
 };
 static_assert(sizeof(PackJob) == 128, "copied in 16-byte words");
 

@@ -83,8 +83,7 @@ __global__ void radius_kernel(const float4* a, int na, const float4* w, int nw, 
 
 // Dense copy of the points (w = dense type; type map null: w already is), and the points of each
 // type in every chunk of kTypedChunk points.
-__global__ void __launch_bounds__(kTypedChunk) dense_count_kernel(const float4* in, float4* out, int n, TypeMap map,
-                                                                  int32_t* counts) {
+__device__ void dense_count(const float4* in, float4* out, int n, const TypeMap& map, int32_t* counts) {
     __shared__ int s_count[16];
     if (threadIdx.x < 16) s_count[threadIdx.x] = 0;
     __syncthreads();
@@ -111,7 +110,7 @@ __global__ void __launch_bounds__(kTypedChunk) dense_count_kernel(const float4* 
 
 // The lists of points by type, ascending index (a stable partition): chunk c writes its points after
 // those of the earlier chunks.  w of a listed point is its index.
-__global__ void __launch_bounds__(kTypedChunk) typed_scatter_kernel(const float4* dense, int n, TypedOut o, const int32_t* counts) {
+__device__ void typed_scatter(const float4* dense, int n, const TypedOut& o, const int32_t* counts) {
     constexpr int kW = kTypedChunk / 32;
     __shared__ int s_warp[kW + 1][16];  // points of a type in the warps before
     __shared__ int s_base[16];          // ... in the chunks before
@@ -152,6 +151,23 @@ __global__ void __launch_bounds__(kTypedChunk) typed_scatter_kernel(const float4
     }
 }
 
+__global__ void __launch_bounds__(kTypedChunk) dense_count_kernel(const float4* in, float4* out, int n, TypeMap map,
+                                                                  int32_t* counts) {
+    dense_count(in, out, n, map, counts);
+}
+__global__ void __launch_bounds__(kTypedChunk) typed_scatter_kernel(const float4* dense, int n, TypedOut o, const int32_t* counts) {
+    typed_scatter(dense, n, o, counts);
+}
+// many sets: blockIdx.y selects the set
+__global__ void __launch_bounds__(kTypedChunk) dense_count_sets_kernel(const TypedSetJob* sets, TypeMap map) {
+    const TypedSetJob& S = sets[blockIdx.y];
+    if (static_cast<int>(blockIdx.x) * kTypedChunk < S.n) dense_count(S.in, S.dense, S.n, map, S.counts);
+}
+__global__ void __launch_bounds__(kTypedChunk) typed_scatter_sets_kernel(const TypedSetJob* sets) {
+    const TypedSetJob& S = sets[blockIdx.y];
+    if (static_cast<int>(blockIdx.x) * kTypedChunk < S.n) typed_scatter(S.dense, S.n, S.out, S.counts);
+}
+
 // slot of w in a table of distinct values, inserted where it is new; -1: the table is full
 __device__ int class_slot(unsigned* bits, unsigned w) {
     for (int k = 0; k < kMaxClasses; ++k) {
@@ -163,7 +179,7 @@ __device__ int class_slot(unsigned* bits, unsigned w) {
 }
 
 // every block's distinct weights in shared memory, then into the global table
-__global__ void weight_classes_kernel(const float4* p, int n, WeightClasses* out) {
+__device__ void weight_classes(const float4* p, int n, WeightClasses* out) {
     __shared__ unsigned s_bits[16];
     __shared__ int s_count[16], s_over;
     if (threadIdx.x < 16) {
@@ -189,6 +205,10 @@ __global__ void weight_classes_kernel(const float4* p, int n, WeightClasses* out
         else atomicAdd(&out->count[k], s_count[threadIdx.x]);
     }
     if (threadIdx.x == 0 && s_over) out->over = 1;
+}
+__global__ void weight_classes_kernel(const float4* p, int n, WeightClasses* out) { weight_classes(p, n, out); }
+__global__ void weight_classes_sets_kernel(const TypedSetJob* sets, WeightClasses* out) {
+    weight_classes(sets[blockIdx.y].in, sets[blockIdx.y].n, out + blockIdx.y);
 }
 
 __global__ void set_type_kernel(float4* p, int n, int32_t value) {
@@ -224,6 +244,17 @@ void typed_lists_launch(const float4* in, float4* dense, int n, const TypeMap& m
 void weight_classes_launch(const float4* p, int n, WeightClasses* out, int sm_count, cudaStream_t s) {
     if (n <= 0) return;
     weight_classes_kernel<<<std::min((n + 255) / 256, sm_count * 2), 256, 0, s>>>(p, n, out);
+}
+
+void weight_classes_sets_launch(const TypedSetJob* sets_dev, int sets, int max_n, WeightClasses* out, cudaStream_t s) {
+    if (sets > 0 && max_n > 0) weight_classes_sets_kernel<<<dim3(std::min((max_n + 255) / 256, 32), sets), 256, 0, s>>>(sets_dev, out);
+}
+
+void typed_sets_launch(const TypedSetJob* sets_dev, int sets, int max_n, const TypeMap& map, cudaStream_t s) {
+    if (sets <= 0 || max_n <= 0) return;
+    const dim3 grid(typed_chunks(max_n), sets);
+    dense_count_sets_kernel<<<grid, kTypedChunk, 0, s>>>(sets_dev, map);
+    typed_scatter_sets_kernel<<<grid, kTypedChunk, 0, s>>>(sets_dev);
 }
 
 void set_type_launch(float4* p, int n, int32_t value, int sm_count, cudaStream_t s) {

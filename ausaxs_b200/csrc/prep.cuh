@@ -53,6 +53,16 @@ struct TypeMap {
 };
 void typed_lists_launch(const float4* in, float4* dense, int n, const TypeMap& map, const TypedOut& o, int32_t* counts,
                         cudaStream_t s);
+// the same for many sets, and their classes (device tables; max_n >= every n)
+struct TypedSetJob {
+    const float4* in;
+    float4* dense;
+    int32_t* counts;
+    int32_t n;
+    TypedOut out;
+};
+void weight_classes_sets_launch(const TypedSetJob* sets_dev, int sets, int max_n, WeightClasses* out, cudaStream_t s);
+void typed_sets_launch(const TypedSetJob* sets_dev, int sets, int max_n, const TypeMap& map, cudaStream_t s);
 // the distinct weights of n points, added to *out (slots preset to kNoClass, counts to 0)
 void weight_classes_launch(const float4* p, int n, WeightClasses* out, int sm_count, cudaStream_t s);
 void set_type_launch(float4* p, int n, int32_t value, int sm_count, cudaStream_t s);
