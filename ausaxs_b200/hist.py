@@ -273,14 +273,16 @@ class _Manager:
         a, w, x = self._inputs()
         nb = self.bin_count
         ff = self.manager != _capi.MANAGER_MT
+        # sized for bin_count bins (14 MB at 8,000), of which the call writes the first max_bin of every row,
+        # packed, and the slices below take those: clearing them took 470 of the 820 us of a 2,700-atom call
         bufs = {
-            "aa": np.zeros(NFF * NFF * nb if ff else nb),
-            "aw": np.zeros(NFF * nb if ff else nb),
-            "ww": np.zeros(nb),
-            "tot": np.zeros(nb),
-            "d_axis": np.zeros(nb),
-            "d_axis_ax": np.zeros(nb),
-            "d_axis_xx": np.zeros(nb),
+            "aa": np.empty(NFF * NFF * nb if ff else nb),
+            "aw": np.empty(NFF * nb if ff else nb),
+            "ww": np.empty(nb),
+            "tot": np.empty(nb),
+            "d_axis": np.empty(nb),
+            "d_axis_ax": np.empty(nb),
+            "d_axis_xx": np.empty(nb),
         }
         r = HistResult()
         for k, v in bufs.items():

@@ -35,11 +35,13 @@ sys.path.insert(0, ROOT)
 
 import numpy as np  # noqa: E402
 
-# warp instructions per 32 pair evaluations of the pair kernel at 0.25 A bins (the batch and serving
-# configurations; the bin rounding fused with the power-of-two inverse width), counted by ncu on the
-# batch's pair launches (smsp__inst_executed / (shared atomics / 2),
-# profiles/pairhist_kernel_batch_64_structures.md)
-INSTR_PER_PAIR = 31.1
+# warp instructions per 32 pair evaluations of the one-atomic pair kernel at 0.25 A bins (the bin rounding
+# fused with the power-of-two inverse width), segment drains and checks included, counted by ncu
+# (smsp__inst_executed / pairs, profiles/pack_kernel_50k_atoms.md)
+INSTR_PER_PAIR = 17.2
+# FP32 operations per pair that the reference's rounding order and the fixed-point offset need: 3 sub, 3 mul,
+# 2 add, the root's 4, bin rounding, offset 3, and the root's guard
+FP32_PER_PAIR = 17.0
 # DRAM bytes (read + write) of the pair launches of one step of the 256-structure batch: 16.6 MB per pass
 # measured by ncu on its first 64 structures (0.86M points), scaled by points to the batch's 3.66M
 BATCH_PAIR_TRAFFIC_BYTES = 7.0e7
@@ -286,20 +288,20 @@ def batch_config(wl):
 def pair_roofline(pairs_per_launch: float, kernel_ms: float, sm_mhz: float, sms: int, atomic_rate: float,
                   atomics_per_pair: int, instr_per_pair: float):
     """Roofline of the pair kernel as pair evaluations per second: the lower of the FP32 bound
-    (sms x 128 lanes x f_SM / 9 FP32 operations per pair) and the shared-atomic bound (measured
+    (sms x 128 lanes x f_SM / 17 FP32 operations per pair) and the shared-atomic bound (measured
     conflict-free atomics/s / atomics per pair).  A secondary figure compares against the issue rate
     at the kernel's own instruction count (ncu)."""
     achieved = pairs_per_launch / (kernel_ms / 1e3)
-    fp32 = sms * 128 * sm_mhz * 1e6 / 9.0
+    fp32 = sms * 128 * sm_mhz * 1e6 / FP32_PER_PAIR
     atom = atomic_rate / atomics_per_pair
     peak = min(fp32, atom)
     issue = sms * 4 * sm_mhz * 1e6 * 32 / instr_per_pair
-    return {"bound": "fp32" if fp32 <= atom else "smem_atomic", "kernel": "pairhist_kernel",
+    return {"bound": "fp32" if fp32 <= atom else "smem_atomic", "kernel": "pack_kernel",
             "achieved": achieved / 1e9, "peak": peak / 1e9, "unit": "Gpair/s", "frac": achieved / peak,
             "fp32_bound": fp32 / 1e9, "smem_atomic_bound": atom / 1e9, "smem_atomics_per_s": atomic_rate,
             "atomics_per_pair": atomics_per_pair, "sm_mhz": sm_mhz, "issue_frac": achieved / issue,
             "instr_per_pair": instr_per_pair, "kernel_ms_per_step": kernel_ms,
-            "peak_source": (f"min({sms} SMs x 128 x {sm_mhz:.0f} MHz / 9 FP32 ops per pair, measured conflict-free "
+            "peak_source": (f"min({sms} SMs x 128 x {sm_mhz:.0f} MHz / 17 FP32 ops per pair, measured conflict-free "
                             f"shared atomics / {atomics_per_pair} per pair)")}
 
 
@@ -474,14 +476,14 @@ def run_batch(args, rank, world, local_rank):
     sms = torch.cuda.get_device_properties(local_rank).multi_processor_count
     timed_pairs = [x for x in pair_ms if x is not None]
     kernel_ms = statistics.mean(timed_pairs) if timed_pairs else float(cand_ms[choice])
-    roof = pair_roofline(pairs, kernel_ms, sm_mhz, sms, atomic_rate, 2, INSTR_PER_PAIR)
+    roof = pair_roofline(pairs, kernel_ms, sm_mhz, sms, atomic_rate, 1, INSTR_PER_PAIR)
     if not timed_pairs:
         roof["kernel_ms_source"] = "autotuner's timing of the chosen pair plan (graph events unavailable)"
     roof["traffic"] = BATCH_PAIR_TRAFFIC_BYTES
     roof["smem_atomics_per_s_random_bins"] = atomic_rate_random
     roof["note"] = ("kernel_ms = device time of the pair stage (accumulator clearing + every pair launch of the "
-                    "graph), events inside the graph, mean over the timed steps; FFAvg pairs add two shared "
-                    "atomics (count, distance offset)")
+                    "graph), events inside the graph, mean over the timed steps; a pair is one shared "
+                    "atomic (count and distance offset in one word)")
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": total_ms / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
@@ -672,7 +674,7 @@ def serving_measure(args, rank, world, local_rank, compact=False):
     sms = torch.cuda.get_device_properties(local_rank).multi_processor_count
     atomic_rate, _ = _capi.smem_atomic_rate(local_rank, True)
     # pair evaluations of the saturated run per second of it (every other stage of a request included)
-    line["roofline"] = pair_roofline(pairs_per_move, 1e3 / sat["moves_per_s"], sm_mhz, sms, atomic_rate, 2,
+    line["roofline"] = pair_roofline(pairs_per_move, 1e3 / sat["moves_per_s"], sm_mhz, sms, atomic_rate, 1,
                                      INSTR_PER_PAIR)
     line["roofline"]["traffic"] = None
     line["roofline"]["note"] = "pair evaluations of the saturated serving run (moved body x the rest + its own pairs)"
@@ -812,7 +814,7 @@ def run_ours(args, rank, world, local_rank):
                 "d2h_bytes_per_step": int(nq * 8 + 8), "p50_ms": 1e3 * float(np.percentile(lat, 50)),
                 "p99_ms": 1e3 * float(np.percentile(lat, 99)), "max_rel_diff_vs_resident": e2e_match},
         "gpu_launches": int(launches),
-        "roofline": dict(pair_roofline(pairs - lattice_pairs, kernel_ms, sm_mhz, sms, atomic_rate, 2, INSTR_PER_PAIR),
+        "roofline": dict(pair_roofline(pairs - lattice_pairs, kernel_ms, sm_mhz, sms, atomic_rate, 1, INSTR_PER_PAIR),
                          traffic=None, kernel_launches_per_step=k_n / args.steps,
                          note="pair evaluations of the pair kernel per second of its launches (the grid dummies' "
                               "self pairs, when the lattice kernel takes them, are not counted)"),
@@ -1269,7 +1271,7 @@ def run_fit(args, rank, world, local_rank):
                 "d2h_bytes_per_step": int(8 * (NFF * NFF + NFF + 3) * h.max_bin + 56),
                 "p50_ms": 1e3 * float(np.percentile(lat, 50)), "p99_ms": 1e3 * float(np.percentile(lat, 99))},
         "gpu_launches": int(launches),
-        "roofline": {"bound": "issue", "kernel": "pairhist_kernel", "achieved": pair_rate / 1e9, "peak": issue_peak / 1e9,
+        "roofline": {"bound": "issue", "kernel": "pack_kernel", "achieved": pair_rate / 1e9, "peak": issue_peak / 1e9,
                      "unit": "Gpair/s", "frac": pair_rate / issue_peak, "traffic": None,
                      "note": "a 5k-atom histogram is launch-latency bound; the fit kernel itself is one CTA"},
         "clocks": clocks,
