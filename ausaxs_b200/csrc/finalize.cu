@@ -33,8 +33,8 @@ __device__ __forceinline__ double weighted_bin(double dsum, double count, int b,
 // Post-processing takes one launch: the blocks write the rows of their bins and raise max_bin, and the
 // block that finishes last forms the distance axes, which depend on it (their bin width is
 // (max_bin * width) / max_bin, bins beyond it are zero).  Bound: the latency of one round of loads; a
-// thread per (bin, row slice) has all of its loads in flight at once (two launches with a thread per bin
-// and serial row loads took 7 + 17 us at any size, this one 5).
+// thread per (bin, row slice) has all of its loads in flight at once (cold, 5,000 atoms: two launches with
+// a thread per bin and serial row loads took 7 + 17 us, this one 10).
 constexpr int kFinBins = 32, kFinSlices = 8;
 
 // Whether this block is the last of `blocks` of its structure to get here; what the others wrote is then
