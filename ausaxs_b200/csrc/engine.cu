@@ -633,7 +633,8 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     const float4* W = raw_w.as<float4>();
     const float4* X = raw_x.as<float4>();
     // Weighted points of few classes of weight: the counts by class pair give the weight sums, so the pairs
-    // go through the one-atomic kernel (20,000 atoms of four weights + 4,000 waters: see the finalisation).
+    // go through the one-atomic kernel (20,011 weighted atoms + 4,003 waters, a whole profile: 636 us by the
+    // two-atomic kernel with weight sums, 300 us by class).
     bool by_class = false;
     if (mt && (n_a == 0 || n_cls[0] > 0) && (n_w == 0 || n_cls[1] > 0) && n_a + n_w > 0) {
         pair_sqrt_prepare(P.inv_w, nb);
