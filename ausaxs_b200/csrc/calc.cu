@@ -240,10 +240,9 @@ struct Calculator {
             dmax = std::min(std::sqrt(d2), 2 * std::sqrt(r2)) * (1 + 1e-6) + 1e-3;
         }
         const float inv_w = (float)(1.0 / bin_width);
-        int nb = (int)std::ceil(dmax * inv_w) + 2;
-        nb = std::max(nb, 11);
-        const bool covered = nb <= bin_count;
-        nb = std::min(nb, bin_count);
+        const BinSpan span = bin_span(dmax, inv_w, bin_count);
+        const int nb = span.bins;
+        const bool covered = span.covered;
         // the classes of all sets together (ascending bit patterns): K.n 0 when there are more than kMaxClasses
         CalcClasses K{};
         TypeMap map;

@@ -560,10 +560,9 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
                                             : "the weighted manager needs weighted atoms"};
     const int weighted = cfg.weighted_bins ? 1 : 0;
     const float inv_w = (float)(1.0 / cfg.bin_width);
-    int nb = (int)std::ceil((double)(dmax + dmax_extra) * inv_w) + 2;
-    nb = std::max(nb, 11);
-    const bool covered = nb <= cfg.bin_count;
-    nb = std::min(nb, cfg.bin_count);
+    const BinSpan span = bin_span(dmax + dmax_extra, inv_w, cfg.bin_count);
+    const int nb = span.bins;
+    const bool covered = span.covered;
     if (P.manager == cfg.manager && P.weighted == weighted && P.bin_count == cfg.bin_count &&
         P.bin_width == cfg.bin_width && P.n_a == n_a && P.n_w == n_w && P.n_x == n_x && P.T == T && P.nb >= nb &&
         P.nb <= nb + 64 && (cfg.manager != AUSAXS_MANAGER_FFGRID || n_x < kLatticeMinPoints || lat.tried) &&

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../../include/ausaxs_b200.h"
+#include "bins.cuh"
 #include "debye.cuh"
 #include "finalize.cuh"
 #include "lattice.cuh"
