@@ -418,13 +418,14 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
             break;  // no other copy is in flight: the next tile's is issued below
         }
         // quads in place: {x y z w} x 4 -> {-x}{-y}{-z}{index}, scaled by 2^-23.  Where the order does not
-        // matter (no masked pairs, not the last tile of the list) a quad takes points a quarter of the tile
-        // apart: a segment of quads then spans four stretches of the chain, its distances more bins, and
-        // the fullest word takes longer to fill.
+        // matter (no masked pairs, none of the list's last three points, which may be scalar-tail partners and are
+        // looked for from the tile's end) a quad takes points a quarter of the tile apart: a segment of quads
+        // then spans four stretches of the chain, its distances more bins, and the fullest word takes longer to
+        // fill.
         Quad* const s_q = stage0 + buf * stage_quads;
         {
             const int nq = (t.jn + 3) / 4;
-            const bool spread = !ragged && !crossed && t.j0 + t.jn < J.nb;
+            const bool spread = !ragged && !crossed && t.j0 + t.jn + 3 <= J.nb;
             const int first = spread ? tid : 4 * tid, step = spread ? nq : 1;
             float4 v[4];
             if (tid < nq) {
