@@ -564,8 +564,8 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     const int nb = span.bins;
     const bool covered = span.covered;
     if (P.manager == cfg.manager && P.weighted == weighted && P.bin_count == cfg.bin_count &&
-        P.bin_width == cfg.bin_width && P.n_a == n_a && P.n_w == n_w && P.n_x == n_x && P.T == T && P.nb >= nb &&
-        P.nb <= nb + 64 && (cfg.manager != AUSAXS_MANAGER_FFGRID || n_x < kLatticeMinPoints || lat.tried) &&
+        P.bin_width == cfg.bin_width && P.points == point_buffers() && P.n_a == n_a && P.n_w == n_w && P.n_x == n_x &&
+        P.T == T && P.nb >= nb && P.nb <= nb + 64 && (cfg.manager != AUSAXS_MANAGER_FFGRID || n_x < kLatticeMinPoints || lat.tried) &&
         std::equal(n_cls, n_cls + 2, P.n_cls) && std::memcmp(cls, P.cls, sizeof cls) == 0 &&
         std::memcmp(cls_count, P.cls_count, sizeof cls_count) == 0 && std::equal(type_ff, type_ff + T, P.type_ff)) {
         // one-shot calls of one shape: only the lists by type have other lengths
@@ -581,6 +581,7 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     P.weighted = weighted;
     P.bin_count = cfg.bin_count;
     P.bin_width = cfg.bin_width;
+    P.points = point_buffers();
     P.n_a = n_a;
     P.n_w = n_w;
     P.n_x = n_x;

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <array>
 #include <memory>
 #include <string>
 #include <vector>
@@ -110,6 +111,9 @@ struct Plan {
     int n_cls[2] = {0, 0};      // weighted: the classes of atoms and waters behind the rows (0: by value)
     float cls[2][16] = {};
     int cls_count[2][16] = {};
+    // The point buffers behind the job tables (Structure::point_buffers).  Loads that are not followed by a plan
+    // (grid dummies of another molecule, a rejected one) may have moved them.
+    std::array<const void*, 8> points{};
     // shapes
     int nb = 0, tile = 256;
     struct Group {  // one pair-kernel launch
@@ -198,6 +202,9 @@ struct Structure {
     void load_end(const PrepStats& st);
     int32_t hmeta[2 * kNff] = {};  // host copy of meta (type counts, ff -> dense type)
     const float4* atoms_for_pairs() const { return ff_typed ? dense_a.as<float4>() : raw_a.as<float4>(); }
+    std::array<const void*, 8> point_buffers() const {
+        return {raw_a.p, raw_w.p, raw_x.p, dense_a.p, dense_w.p, typed.p, typed_w.p, meta.p};
+    }
     Plan& plan_for(const ausaxs_hist_config& cfg);
     bool upload_pack(Plan& P);
     void enqueue_histogram(const ausaxs_hist_config& cfg);

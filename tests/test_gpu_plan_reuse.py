@@ -1,0 +1,57 @@
+"""One-shot calls share a context's buffers and keep its last plan: calls in any order give what a context that
+makes only the one call gives."""
+import numpy as np
+import pytest
+
+import ausaxs_b200 as ab
+from ausaxs_b200 import _capi, hist, synth
+
+pytestmark = pytest.mark.gpu
+
+Q = np.linspace(0.01, 0.5, 40)
+MANAGERS = {"ffavg": hist.HistogramManagerMTFFAvg, "ffexplicit": hist.HistogramManagerMTFFExplicit, "mt": hist.HistogramManagerMT}
+
+
+def molecule(seed, n=600, nw=100):
+    xyz, ff = synth.globule(seed, n)
+    rng = np.random.default_rng(seed)
+    ff = np.resize(np.array([3, 7, 11, 3], np.int32), n)  # the same types in every molecule of a size
+    return ab.Molecule(atoms=xyz, ff_types=ff, weights=synth.ff_charge(ff), waters=rng.normal(0, 12, (nw, 3)),
+                       water_weights=np.full(nw, 10.0), volume=18.0 * n)
+
+
+def profile(kind, m, ctx):
+    return ab.profile(MANAGERS[kind](m, True, 0.25, 8000, ctx), Q)
+
+
+def alone(kind, m):
+    ctx = _capi.Context(0)
+    I = profile(kind, m, ctx)
+    ctx.close()
+    return I
+
+
+def load_only(how, m, ctx):
+    """A call that loads the molecule's points and makes no plan."""
+    a, w, _ = m.compact_ff()
+    if how == "grid":
+        assert len(_capi.grid_exv(ctx, a, w)[0]) > 0
+    else:
+        bad = ab.Molecule(atoms=m.atoms, ff_types=np.full(len(m.atoms), 15, np.int32), waters=m.waters, volume=m.volume)
+        with pytest.raises(_capi.AusaxsError) as e:
+            profile("ffavg", bad, ctx)
+        assert e.value.code == _capi.ERR_FORM_FACTOR
+
+
+@pytest.mark.parametrize("how", ["grid", "rejected"])
+@pytest.mark.parametrize("kind", list(MANAGERS))
+def test_larger_load_between(kind, how):
+    """The larger load moves the point buffers that the kept plan's tables point into."""
+    ctx = _capi.Context(0)
+    for n in (5000, 20000):
+        first = molecule(3)
+        np.testing.assert_array_equal(profile(kind, first, ctx), alone(kind, first))
+        load_only(how, molecule(4, n, n // 5), ctx)
+        again = molecule(5)
+        np.testing.assert_array_equal(profile(kind, again, ctx), alone(kind, again))
+    ctx.close()
