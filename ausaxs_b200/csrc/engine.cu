@@ -421,7 +421,7 @@ bool Structure::lattice_ready() {
 
 // The plan's pair passes as launches of the two-atomic kernel (weighted plans, and widths or row counts
 // the one-atomic kernel does not take).
-static void plan_groups(Plan& P, char* base, Ctx& C) {
+static void plan_groups(Plan& P, char* base, Ctx& C, bool w_launch) {
     // Jobs split into launch groups by the rows they keep on chip: one-row jobs (ww, xx, wx and all
     // Simple jobs) run with a small footprint and high occupancy, multi-row jobs (aa, aw, ax) get the
     // shared memory they need.  Large structures: one launch per row class (1, T, T*T rows) so each
@@ -434,8 +434,6 @@ static void plan_groups(Plan& P, char* base, Ctx& C) {
     append_pair_jobs(P, P.tile, split, group_jobs, group_tiles, group_rows, 0, true);
     if (group_jobs[0].size() + group_jobs[1].size() + group_jobs[2].size() > 64)
         throw Error{AUSAXS_ERR_CAPACITY, "too many row groups"};
-    const bool w_launch = P.manager == AUSAXS_MANAGER_MT;  // Simple histograms always carry weight sums (values)
-    P.n_launch = 0;
     size_t job_off = P.off_jobs;
     for (int g = 0; g < 3; ++g) {
         if (group_jobs[g].empty()) continue;
@@ -531,6 +529,8 @@ bool choose_pack(const Plan& P, int sm_count, PackLaunch& L, int& shape, int& gr
 // The plan's launch of the one-atomic-per-pair kernel and its tables; false where it does not apply.
 bool Structure::upload_pack(Plan& P) {
     PackTable table;
+    const int manager = P.manager;
+    P.manager = 0;  // (until the tables are on their way)
     if (!choose_pack(P, ctx->sm_count, P.pack, P.pack_shape, P.pack_grid, table)) return false;
     std::copy(type_count, type_count + T, P.type_count);
     char* base = P.dev.as<char>();
@@ -546,6 +546,7 @@ bool Structure::upload_pack(Plan& P) {
     std::memcpy(bytes.data() + jobs_bytes, table.out.data(), out_bytes);
     // pageable source: staged on return
     AUSAXS_CUDA(cudaMemcpyAsync(base + P.off_jobs, bytes.data(), bytes.size(), cudaMemcpyHostToDevice, ctx->stream));
+    P.manager = manager;
     return true;
 }
 
@@ -563,13 +564,13 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     const BinSpan span = bin_span(dmax + dmax_extra, inv_w, cfg.bin_count);
     const int nb = span.bins;
     const bool covered = span.covered;
-    if (P.manager == cfg.manager && P.weighted == weighted && P.bin_count == cfg.bin_count &&
+    const bool same = P.manager == cfg.manager && P.weighted == weighted && P.bin_count == cfg.bin_count &&
         P.bin_width == cfg.bin_width && P.points == point_buffers() && P.n_a == n_a && P.n_w == n_w && P.n_x == n_x &&
         P.T == T && P.nb >= nb && P.nb <= nb + 64 && (cfg.manager != AUSAXS_MANAGER_FFGRID || n_x < kLatticeMinPoints || lat.tried) &&
         std::equal(n_cls, n_cls + 2, P.n_cls) && std::memcmp(cls, P.cls, sizeof cls) == 0 &&
-        std::memcmp(cls_count, P.cls_count, sizeof cls_count) == 0 && std::equal(type_ff, type_ff + T, P.type_ff)) {
-        // one-shot calls of one shape: only the lists by type have other lengths
-        if (P.packed && !std::equal(type_count, type_count + T, P.type_count)) upload_pack(P);
+        std::memcmp(cls_count, P.cls_count, sizeof cls_count) == 0 && std::equal(type_ff, type_ff + T, P.type_ff);
+    // one-shot calls of one shape: only the lists by type have other lengths
+    if (same && (!P.packed || std::equal(type_count, type_count + T, P.type_count) || upload_pack(P))) {
         P.covered = covered;
         P.pack.covered = covered;
         P.fin_ff.z_exv = cfg.z_exv;  // per call: other molecules of the same shape have other volumes
@@ -577,7 +578,10 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     }
 
     Ctx& C = *ctx;
-    P.manager = cfg.manager;
+    // no call may match the plan until it is complete: what follows can throw
+    P.manager = 0;
+    P.packed = false;
+    P.n_launch = 0;
     P.weighted = weighted;
     P.bin_count = cfg.bin_count;
     P.bin_width = cfg.bin_width;
@@ -782,9 +786,9 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     }
 
     pair_sqrt_prepare(P.inv_w, nb);  // once per width and process: the Newton-Raphson root where it bins exactly
-    P.n_launch = 0;
     P.packed = (!mt || by_class) && upload_pack(P);
-    if (!P.packed) plan_groups(P, base, C);
+    // (Simple histograms always carry weight sums, their values)
+    if (!P.packed) plan_groups(P, base, C, mt);
 
     // finalisation (its counter is cleared with the accumulators, or here where they are not)
     AUSAXS_CUDA(cudaMemsetAsync(base + P.off_maxbin, 0, 256, C.stream));
@@ -891,6 +895,7 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     }
     AUSAXS_CUDA(cudaMemcpyAsync(base + P.off_rows, rd.data(), sizeof(RowDesc) * R, cudaMemcpyHostToDevice, C.stream));
     P.rows_host = rd;
+    P.manager = cfg.manager;
     return P;
 }
 

@@ -55,3 +55,17 @@ def test_larger_load_between(kind, how):
         again = molecule(5)
         np.testing.assert_array_equal(profile(kind, again, ctx), alone(kind, again))
     ctx.close()
+
+
+@pytest.mark.parametrize("kind", list(MANAGERS))
+def test_rejected_call_leaves_no_plan(kind):
+    """A call whose bins do not fit on chip is refused however often it is made, and the calls around it are as ever."""
+    ctx = _capi.Context(0)
+    m = molecule(3)
+    for _ in range(2):
+        for _ in range(2):
+            with pytest.raises(_capi.AusaxsError) as e:
+                ab.profile(MANAGERS[kind](m, True, 5e-4, 400000, ctx), Q)
+            assert e.value.code == _capi.ERR_CAPACITY
+        np.testing.assert_array_equal(profile(kind, m, ctx), alone(kind, m))
+    ctx.close()
