@@ -54,6 +54,13 @@ __device__ bool last_block(unsigned* done, unsigned blocks) {
     return s_last;
 }
 
+// max_bin past the warp's last bin in use (lane l holds bin b of the warp's 32 in order), at least the minimum
+// size (HistogramManagerMT.cpp:48).  All 32 lanes call it: what they did for their bins may have parted them.
+__device__ __forceinline__ void raise_max_bin(int32_t* max_bin, bool in_use, int b) {
+    const unsigned at = __ballot_sync(0xffffffffu, in_use);
+    if ((threadIdx.x & 31) == 0) atomicMax(max_bin, max(10, at ? b + 32 - __clz(at) : 0));
+}
+
 __device__ void ff_finalize_body(const FinalizeFF& F, unsigned blocks) {
     __shared__ unsigned long long s_n[3][kFinSlices][kFinBins];  // aa pairs, aw pairs, ax pairs of the slice's types
     const int T = F.T;
@@ -96,6 +103,7 @@ __device__ void ff_finalize_body(const FinalizeFF& F, unsigned blocks) {
     s_n[1][slice][lane] = n_aw;
     s_n[2][slice][lane] = n_ax;
     __syncthreads();
+    bool in_use = false;
     if (slice == 0 && b < F.nb) {
         for (int k = 1; k < kFinSlices; ++k) {
             n_aa += s_n[0][k][lane];
@@ -129,9 +137,9 @@ __device__ void ff_finalize_body(const FinalizeFF& F, unsigned blocks) {
             F.d_axis_xx[b] = 2.0 * dist_sum(F.ds_xx, n_xx, b, F.c, F.scale);
             used = used || xx != 0 || n_wx != 0;
         }
-        const unsigned at = __ballot_sync(__activemask(), used && b >= 10);
-        if (lane == 0) atomicMax(F.max_bin, max(10, at ? b + 32 - __clz(at) : 0));  // minimum size (HistogramManagerMT.cpp:48)
+        in_use = used && b >= 10;
     }
+    if (slice == 0) raise_max_bin(F.max_bin, in_use, b);
     if (!last_block(F.done, blocks)) return;
     const int mb = __ldcg(F.max_bin);
     const double width = (static_cast<double>(mb) * F.bin_width) / mb;  // Axis(0, mb*width, mb).width()
@@ -255,6 +263,7 @@ __device__ MTSum mt_sum(const unsigned long long* cnt, const long long* w, int r
 __global__ void mt_finalize_kernel(FinalizeMT F) {
     const size_t nb = F.nb;
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    bool in_use = false;
     if (b < F.nb) {
         const float wscale = F.ta ? F.wscale_v : *F.wscale;
         const double inv = 1.0 / static_cast<double>(wscale);
@@ -279,9 +288,9 @@ __global__ void mt_finalize_kernel(FinalizeMT F) {
         F.H[nb + b] = aw;
         F.H[2 * nb + b] = ww;
         F.tot[b] = aa + ww + aw;
-        const unsigned at = __ballot_sync(__activemask(), v != 0 && b >= 10);
-        if ((threadIdx.x & 31) == 0) atomicMax(F.max_bin, max(10, at ? b + 32 - __clz(at) : 0));  // minimum size (HistogramManagerMT.cpp:48)
+        in_use = v != 0 && b >= 10;
     }
+    raise_max_bin(F.max_bin, in_use, b);
     if (!last_block(F.done, gridDim.x)) return;
     const int mb = __ldcg(F.max_bin);
     const double width = (static_cast<double>(mb) * F.bin_width) / mb;
