@@ -153,8 +153,8 @@ struct Calculator {
         results.assign((size_t)n_slots * 3 * bin_count, 0.0);
         result_info = slot_info;
         if (n_slots == 0) return clear();
-        // the points, and every set's distinct weights, counted while the host finds the largest distance
-        // (buffers of the context: a calculator lives for one run, and allocating took longer than the pairs)
+        // the points, and where it can pay every set's distinct weights, counted while the host finds the largest
+        // distance (buffers of the context: a calculator lives for one run, and allocating took longer than the pairs)
         struct Keep {
             Ctx& C;
             ~Keep() {
@@ -163,43 +163,82 @@ struct Calculator {
             }
         } keep{C};
         DevBuf &in = C.calc[0], &acc = C.calc[1], &out = C.calc[2], &table = C.calc[3];
+        const int n_sets = (int)sets.size();
+        long long pairs = 0;
+        for (const Job& j : jobs) {
+            const long long na = sets[j.a].n;
+            pairs += j.b < 0 ? na * (na - 1) / 2 : na * sets[j.b].n;
+        }
+        // Pairs go by class of weight where the rows by class (every result's, cleared and read once) are few against
+        // the pairs, and stay within what the context keeps; by value elsewhere.  Measured (6 sets merged into
+        // 2 results / 21 results, by class and by value): 300 points each, 15 classes 262 and 256 us / 1,045
+        // and 985 us, 8 classes 222 and 256 / 959 and 985; 3,000 points, 15 classes 436 and 431 / 1,347 and 1,357,
+        // 4 classes 365 and 431 / 1,221 and 1,357; 50 points (13,700 pairs), 8 classes 217 and 192.
+        auto rows_pay = [&](long long classes, long long bins) {
+            const long long words = n_slots * classes * classes * bins;
+            return words * 8 <= (long long)Ctx::kCalcKeep && 4 * words <= pairs;
+        };
+        // first by a sample of the points, which costs no launch: its classes and extent are lower bounds
+        bool classify = false;
+        {
+            std::vector<uint32_t> seen;
+            double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+            for (int k = 0; k < n_sets && (int)seen.size() <= kMaxClasses; ++k) {
+                const float4* q = staged.data() + sets[k].off;
+                for (int i = 0; i < sets[k].n && (int)seen.size() <= kMaxClasses; i += 1 + sets[k].n / 64) {
+                    uint32_t w;
+                    std::memcpy(&w, &q[i].w, 4);
+                    if (std::find(seen.begin(), seen.end(), w) == seen.end()) seen.push_back(w);
+                    const double v[3] = {q[i].x, q[i].y, q[i].z};
+                    for (int d = 0; d < 3; ++d) lo[d] = std::min(lo[d], v[d]), hi[d] = std::max(hi[d], v[d]);
+                }
+            }
+            double extent = 0;
+            for (int d = 0; d < 3; ++d) extent = std::max(extent, hi[d] - lo[d]);
+            classify = !seen.empty() && (int)seen.size() <= kMaxClasses &&
+                       rows_pay((long long)seen.size(), bin_span(extent, (float)(1.0 / bin_width), bin_count).bins);
+        }
         const size_t pts_bytes = align_up(std::max<size_t>(1, staged.size()) * 16, 256);
-        size_t list_bytes = 256;
-        for (const Set& q : sets) list_bytes += align_up(Structure::typed_bytes(q.n), 256);
-        const size_t jobs_bytes_in = align_up(sizeof(TypedSetJob) * std::max<size_t>(1, sets.size()), 256);
-        const size_t class_bytes = align_up(sizeof(WeightClasses) * std::max<size_t>(1, sets.size()), 256);
-        in.ensure(2 * pts_bytes + list_bytes + jobs_bytes_in + class_bytes);
+        size_t list_bytes = 256, jobs_bytes_in = 256, class_bytes = 256;
+        if (classify) {
+            for (const Set& q : sets) list_bytes += align_up(Structure::typed_bytes(q.n), 256);
+            jobs_bytes_in = align_up(sizeof(TypedSetJob) * n_sets, 256);
+            class_bytes = align_up(sizeof(WeightClasses) * n_sets, 256);
+        }
+        const size_t dense_bytes = classify ? pts_bytes : 256;
+        in.ensure(pts_bytes + dense_bytes + list_bytes + jobs_bytes_in + class_bytes);
         DevBuf points, dense, lists, set_jobs, classes;
         points.view(in.p, pts_bytes);
-        dense.view(in.as<char>(pts_bytes), pts_bytes);
-        lists.view(in.as<char>(2 * pts_bytes), list_bytes);
-        set_jobs.view(in.as<char>(2 * pts_bytes + list_bytes), jobs_bytes_in);
-        classes.view(in.as<char>(2 * pts_bytes + list_bytes + jobs_bytes_in), class_bytes);
+        dense.view(in.as<char>(pts_bytes), dense_bytes);
+        lists.view(in.as<char>(pts_bytes + dense_bytes), list_bytes);
+        set_jobs.view(in.as<char>(pts_bytes + dense_bytes + list_bytes), jobs_bytes_in);
+        classes.view(in.as<char>(pts_bytes + dense_bytes + list_bytes + jobs_bytes_in), class_bytes);
         AUSAXS_CUDA(cudaMemcpyAsync(points.p, staged.data(), staged.size() * 16, cudaMemcpyHostToDevice, s));
         const float4* P = points.as<float4>();
-        const int n_sets = (int)sets.size();
         int max_n = 0;
-        std::vector<TypedSetJob> sj(n_sets);
-        std::vector<WeightClasses> wc(n_sets);
-        size_t list_at = 0;
-        for (int k = 0; k < n_sets; ++k) {
-            const int n = sets[k].n;
-            char* mem = lists.as<char>(list_at);
-            list_at += align_up(Structure::typed_bytes(n), 256);
-            sj[k] = TypedSetJob{};
-            sj[k].in = P + sets[k].off;
-            sj[k].dense = dense.as<float4>() + sets[k].off;
-            sj[k].counts = reinterpret_cast<int32_t*>(mem + typed_off_counts(n));
-            sj[k].n = n;
-            sj[k].out.pts = reinterpret_cast<float4*>(mem);
-            sj[k].out.pre = reinterpret_cast<int32_t*>(mem + typed_off_pre(n));
-            sj[k].out.pre_stride = typed_pre_stride(n);
-            max_n = std::max(max_n, n);
-            std::fill(wc[k].bits, wc[k].bits + 16, kNoClass);
-            std::fill(wc[k].count, wc[k].count + 16, 0);
-            wc[k].over = 0;
-        }
-        if (max_n > 0) {
+        std::vector<TypedSetJob> sj;
+        std::vector<WeightClasses> wc;
+        if (classify) {
+            sj.resize(n_sets);
+            wc.resize(n_sets);
+            size_t list_at = 0;
+            for (int k = 0; k < n_sets; ++k) {
+                const int n = sets[k].n;
+                char* mem = lists.as<char>(list_at);
+                list_at += align_up(Structure::typed_bytes(n), 256);
+                sj[k] = TypedSetJob{};
+                sj[k].in = P + sets[k].off;
+                sj[k].dense = dense.as<float4>() + sets[k].off;
+                sj[k].counts = reinterpret_cast<int32_t*>(mem + typed_off_counts(n));
+                sj[k].n = n;
+                sj[k].out.pts = reinterpret_cast<float4*>(mem);
+                sj[k].out.pre = reinterpret_cast<int32_t*>(mem + typed_off_pre(n));
+                sj[k].out.pre_stride = typed_pre_stride(n);
+                max_n = std::max(max_n, n);
+                std::fill(wc[k].bits, wc[k].bits + 16, kNoClass);
+                std::fill(wc[k].count, wc[k].count + 16, 0);
+                wc[k].over = 0;
+            }
             // pageable sources: staged on return
             AUSAXS_CUDA(cudaMemcpyAsync(set_jobs.p, sj.data(), sizeof(TypedSetJob) * n_sets, cudaMemcpyHostToDevice, s));
             AUSAXS_CUDA(cudaMemcpyAsync(classes.p, wc.data(), sizeof(WeightClasses) * n_sets, cudaMemcpyHostToDevice, s));
@@ -247,7 +286,7 @@ struct Calculator {
         CalcClasses K{};
         TypeMap map;
         std::vector<TypedSet> typed(n_sets);
-        if (max_n > 0) {
+        if (classify) {
             AUSAXS_CUDA(cudaMemcpyAsync(wc.data(), classes.p, sizeof(WeightClasses) * n_sets, cudaMemcpyDeviceToHost, s));
             AUSAXS_CUDA(cudaStreamSynchronize(s));
             std::map<unsigned, int> found;
@@ -265,7 +304,8 @@ struct Calculator {
             fit.group_sums = fit.offsets = 1;
             fit.bins = nb;
             fit.tile_j = kPackMaxTileJ;
-            if (few && found.size() <= (size_t)kMaxClasses && fit.nr > 0 && pack_shape(fit) >= 0) {
+            if (few && found.size() <= (size_t)kMaxClasses && rows_pay((long long)found.size(), nb) && fit.nr > 0 &&
+                pack_shape(fit) >= 0) {
                 float m = 0;
                 int most = 0;
                 for (auto& f : found) {
@@ -343,7 +383,6 @@ struct Calculator {
             table_h[k].diag_value = table_h[k].diag_count = 0;
             table_h[k].out = out.as<double>() + (size_t)k * 3 * nb;
         }
-        long long pairs = 0;
         int biggest = 0;
         for (const Job& j : jobs) {
             const Set& A = sets[j.a];
@@ -371,7 +410,6 @@ struct Calculator {
                 sp.mult = j.scaling;
                 by_class(sp, j.a, j.a);
                 plan.specs.push_back(sp);
-                pairs += (long long)A.n * (A.n - 1) / 2;
                 biggest = std::max(biggest, A.n);
             } else {
                 // enqueue_calculate_cross(data_1 = a, data_2 = b): b outer, a inner from 0
@@ -391,7 +429,6 @@ struct Calculator {
                 sp.mult = j.scaling;
                 by_class(sp, j.b, j.a);
                 plan.specs.push_back(sp);
-                pairs += (long long)A.n * B.n;
                 biggest = std::max({biggest, A.n, B.n});
             }
         }

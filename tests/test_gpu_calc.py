@@ -121,3 +121,44 @@ def test_calculator_empty_sets_and_repeated_runs(gpu_ctx):
     o = O.calculator([a], [(0, None, 3, 7)], 0.25, 8000)
     check_result(r["self"][7], o[(0, 7)], [a], 0.25, 8000)
     calc.close()
+
+
+def class_sets(classes, sizes, seed=11):
+    """Point sets whose weights are drawn from `classes` values, the first set without the larger half of them."""
+    rng = np.random.default_rng(seed)
+    values = np.concatenate([[-3.5], rng.uniform(0.5, 16, max(0, classes - 1))]).astype(np.float32)[:classes]
+    sets = []
+    for k, n in enumerate(sizes):
+        few = max(1, classes // 2) if k == 0 else classes
+        w = values[rng.integers(0, few, n) ** 2 // max(1, few - 1) if few > 1 else np.zeros(n, int)]  # uneven shares
+        if k and n >= classes:
+            w[:classes] = values
+        sets.append(np.column_stack([rng.normal(0, 4 + k, (n, 3)), w]).astype(np.float32))
+    return sets
+
+
+@pytest.mark.parametrize("classes", [1, 2, 8, 15, 16])
+@pytest.mark.parametrize("sizes", [(40, 60, 0, 50), (700, 1100, 0, 900)])
+def test_weights_by_class(classes, sizes, gpu_ctx):
+    """Few distinct weights go by class of weight where the rows are few against the pairs (the larger sets), by
+    value elsewhere: the same results, with merged ones, scalings, an empty set and a set that lacks classes."""
+    sets = class_sets(classes, sizes)
+    jobs = [(0, None, 3, 0), (1, None, 1, 0), (3, None, 2, 1), (0, 1, 5, 0), (1, 0, 1, 0), (3, 1, 2, 4), (2, 1, 1, 7),
+            (2, None, 1, 9)]
+    out, _ = run_gpu(gpu_ctx, sets, jobs, 0.25)
+    for (cross, mid), ref in O.calculator(sets, jobs, 0.25, 8000).items():
+        check_result(out["cross" if cross else "self"][mid], ref, [s for s in sets if len(s)], 0.25, 8000)
+
+
+def test_many_results_by_class(gpu_ctx):
+    """A result per job: rows by class of all results would take 500 x 225 x bins words, so the run goes by value."""
+    sets = class_sets(15, (60,) * 25)
+    jobs = [(a, b, 1, -1) for a in range(25) for b in range(25) if a != b][:500]
+    before = gpu_ctx.launches
+    out, idx = run_gpu(gpu_ctx, sets, jobs, 0.25)
+    assert gpu_ctx.launches - before == 3  # weight scale, pairs, results: no lists by class
+    assert sorted(out["cross"]) == list(range(500))
+    for k in (0, 77, 499):
+        a, b, _, _ = jobs[k]
+        ref = O.calculator(sets, [(a, b, 1, 0)], 0.25, 8000)[(1, 0)]
+        check_result(out["cross"][idx[k]], ref, sets, 0.25, 8000)
