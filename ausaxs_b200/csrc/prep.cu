@@ -246,15 +246,22 @@ void weight_classes_launch(const float4* p, int n, WeightClasses* out, int sm_co
     weight_classes_kernel<<<std::min((n + 255) / 256, sm_count * 2), 256, 0, s>>>(p, n, out);
 }
 
+constexpr int kMaxSets = 65535;  // gridDim.y of one launch
+
 void weight_classes_sets_launch(const TypedSetJob* sets_dev, int sets, int max_n, WeightClasses* out, cudaStream_t s) {
-    if (sets > 0 && max_n > 0) weight_classes_sets_kernel<<<dim3(std::min((max_n + 255) / 256, 32), sets), 256, 0, s>>>(sets_dev, out);
+    if (max_n <= 0) return;
+    for (int at = 0; at < sets; at += kMaxSets)
+        weight_classes_sets_kernel<<<dim3(std::min((max_n + 255) / 256, 32), std::min(sets - at, kMaxSets)), 256, 0, s>>>(sets_dev + at,
+                                                                                                                   out + at);
 }
 
 void typed_sets_launch(const TypedSetJob* sets_dev, int sets, int max_n, const TypeMap& map, cudaStream_t s) {
-    if (sets <= 0 || max_n <= 0) return;
-    const dim3 grid(typed_chunks(max_n), sets);
-    dense_count_sets_kernel<<<grid, kTypedChunk, 0, s>>>(sets_dev, map);
-    typed_scatter_sets_kernel<<<grid, kTypedChunk, 0, s>>>(sets_dev);
+    if (max_n <= 0) return;
+    for (int at = 0; at < sets; at += kMaxSets) {
+        const dim3 grid(typed_chunks(max_n), std::min(sets - at, kMaxSets));
+        dense_count_sets_kernel<<<grid, kTypedChunk, 0, s>>>(sets_dev + at, map);
+        typed_scatter_sets_kernel<<<grid, kTypedChunk, 0, s>>>(sets_dev + at);
+    }
 }
 
 void set_type_launch(float4* p, int n, int32_t value, int sm_count, cudaStream_t s) {

@@ -162,3 +162,25 @@ def test_many_results_by_class(gpu_ctx):
         a, b, _, _ = jobs[k]
         ref = O.calculator(sets, [(a, b, 1, 0)], 0.25, 8000)[(1, 0)]
         check_result(out["cross"][idx[k]], ref, sets, 0.25, 8000)
+
+
+def test_more_sets_than_a_grid_has_rows(gpu_ctx):
+    rng = np.random.default_rng(8)
+    n, m = 65540, 8
+    pts = np.zeros((n * m, 4), np.float32)
+    pts[:, :3] = rng.normal(0, 1, (n * m, 3))
+    pts[:, 3] = 6.0
+    calc = _capi.Calculator(gpu_ctx, 1.0, 8000)
+    for k in range(n):
+        calc.enqueue_calculate_self(pts[k * m:(k + 1) * m], 1, 0 if k < 65535 else 1)
+    before = gpu_ctx.launches
+    out = calc.run()
+    calc.close()
+    assert gpu_ctx.launches - before == 5  # classes, lists (two kernels), pairs, results: the route by class
+    x = pts[:, :3].reshape(n, m, 3)
+    d = np.sqrt(((x[:, :, None] - x[:, None]) ** 2).sum(-1, dtype=np.float32))[:, *np.triu_indices(m, 1)]
+    for mid, part in ((0, d[:65535]), (1, d[65535:])):
+        count = np.bincount(np.rint(part).astype(int).ravel(), minlength=8000).astype(float) * 2
+        count[0] += np.floor(36.0 * m) * len(part)
+        assert np.abs(out["self"][mid][1] - count).sum() <= 40  # (roundings at bin edges)
+        assert out["self"][mid][1].sum() == count.sum()
