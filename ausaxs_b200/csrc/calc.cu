@@ -174,11 +174,12 @@ struct Calculator {
         // 2 results / 21 results, by class and by value): 300 points each, 15 classes 262 and 256 us / 1,045
         // and 985 us, 8 classes 222 and 256 / 959 and 985; 3,000 points, 15 classes 436 and 431 / 1,347 and 1,357,
         // 4 classes 365 and 431 / 1,221 and 1,357; 50 points (13,700 pairs), 8 classes 217 and 192.
-        auto rows_pay = [&](long long classes, long long bins) {
+        auto rows_pay = [&](long long classes, long long bins, int least) {
             const long long words = n_slots * classes * classes * bins;
-            return words * 8 <= (long long)Ctx::kCalcKeep && 4 * words <= pairs;
+            return words * 8 <= (long long)Ctx::kCalcKeep && least * words <= pairs;
         };
-        // first by a sample of the points, which costs no launch: its classes and extent are lower bounds
+        // by a sample of the points, which costs no launch (its classes and extent are lower bounds); more points
+        // than the sample has seldom change the answer, so the exact numbers only bound it
         bool classify = false;
         {
             std::vector<uint32_t> seen;
@@ -193,10 +194,9 @@ struct Calculator {
                     for (int d = 0; d < 3; ++d) lo[d] = std::min(lo[d], v[d]), hi[d] = std::max(hi[d], v[d]);
                 }
             }
-            double extent = 0;
-            for (int d = 0; d < 3; ++d) extent = std::max(extent, hi[d] - lo[d]);
+            const double extent = std::hypot(hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2]);
             classify = !seen.empty() && (int)seen.size() <= kMaxClasses &&
-                       rows_pay((long long)seen.size(), bin_span(extent, (float)(1.0 / bin_width), bin_count).bins);
+                       rows_pay((long long)seen.size(), bin_span(extent, (float)(1.0 / bin_width), bin_count).bins, 6);
         }
         const size_t pts_bytes = align_up(std::max<size_t>(1, staged.size()) * 16, 256);
         size_t list_bytes = 256, jobs_bytes_in = 256, class_bytes = 256;
@@ -235,9 +235,7 @@ struct Calculator {
                 sj[k].out.pre = reinterpret_cast<int32_t*>(mem + typed_off_pre(n));
                 sj[k].out.pre_stride = typed_pre_stride(n);
                 max_n = std::max(max_n, n);
-                std::fill(wc[k].bits, wc[k].bits + 16, kNoClass);
-                std::fill(wc[k].count, wc[k].count + 16, 0);
-                wc[k].over = 0;
+                wc[k].clear();
             }
             // pageable sources: staged on return
             AUSAXS_CUDA(cudaMemcpyAsync(set_jobs.p, sj.data(), sizeof(TypedSetJob) * n_sets, cudaMemcpyHostToDevice, s));
@@ -290,12 +288,12 @@ struct Calculator {
             AUSAXS_CUDA(cudaMemcpyAsync(wc.data(), classes.p, sizeof(WeightClasses) * n_sets, cudaMemcpyDeviceToHost, s));
             AUSAXS_CUDA(cudaStreamSynchronize(s));
             std::map<unsigned, int> found;
+            std::vector<std::vector<std::pair<unsigned, int>>> of_set(n_sets);
             bool few = true;
             long long total = 0;
-            for (const WeightClasses& w : wc) {
-                few = few && !w.over;
-                for (int i = 0; i < kMaxClasses; ++i)
-                    if (w.bits[i] != kNoClass) found[w.bits[i]] += w.count[i], total += w.count[i];
+            for (int k = 0; k < n_sets; ++k) {
+                few = wc[k].sorted(of_set[k]) && few;
+                for (auto& f : of_set[k]) found[f.first] += f.second, total += f.second;
             }
             pair_sqrt_prepare(inv_w, nb);
             PackLaunch fit{};
@@ -304,7 +302,7 @@ struct Calculator {
             fit.group_sums = fit.offsets = 1;
             fit.bins = nb;
             fit.tile_j = kPackMaxTileJ;
-            if (few && found.size() <= (size_t)kMaxClasses && rows_pay((long long)found.size(), nb) && fit.nr > 0 &&
+            if (few && found.size() <= (size_t)kMaxClasses && rows_pay((long long)found.size(), nb, 3) && fit.nr > 0 &&
                 pack_shape(fit) >= 0) {
                 float m = 0;
                 int most = 0;
@@ -327,8 +325,7 @@ struct Calculator {
                     t.pre = sj[k].out.pre;
                     t.pre_stride = sj[k].out.pre_stride;
                     t.types = sj[k].out.types = K.n;
-                    for (int i = 0; i < kMaxClasses; ++i)
-                        if (wc[k].bits[i] != kNoClass) t.count[std::distance(found.begin(), found.find(wc[k].bits[i]))] = wc[k].count[i];
+                    for (auto& f : of_set[k]) t.count[std::distance(found.begin(), found.find(f.first))] = f.second;
                     for (int i = 0, at = 0; i < K.n; ++i) {
                         t.start[i] = sj[k].out.start[i] = at;
                         at += t.count[i];

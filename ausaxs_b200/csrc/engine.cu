@@ -110,17 +110,13 @@ void Structure::load_begin(const float* atoms, int n_atoms, const float* waters,
 
     PrepStats init{};
     for (int k = 0; k < 3; ++k) init.lo[k] = 0xffffffffu, init.hi[k] = 0;
-    for (auto& w : init.weights) std::fill(w.bits, w.bits + 16, kNoClass);
+    for (auto& w : init.weights) w.clear();
     *h_stats = init;  // pinned: the copy below reads it asynchronously, the census result overwrites it
     AUSAXS_CUDA(cudaMemcpyAsync(d_stats, h_stats, sizeof(PrepStats), cudaMemcpyHostToDevice, s));
-    census_launch(raw_a.as<float4>(), n_a, ff_typed, d_stats, C.sm_count, s);
-    census_launch(raw_w.as<float4>(), n_w, 0, d_stats, C.sm_count, s);
-    census_launch(raw_x.as<float4>(), n_x, 0, d_stats, C.sm_count, s);
+    census_launch(raw_a.as<float4>(), n_a, ff_typed, d_stats, ff_typed ? nullptr : &d_stats->weights[0], C.sm_count, s);
+    census_launch(raw_w.as<float4>(), n_w, 0, d_stats, ff_typed ? nullptr : &d_stats->weights[1], C.sm_count, s);
+    census_launch(raw_x.as<float4>(), n_x, 0, d_stats, nullptr, C.sm_count, s);
     radius_launch(raw_a.as<float4>(), n_a, raw_w.as<float4>(), n_w, raw_x.as<float4>(), n_x, d_stats, C.sm_count, s);
-    if (!ff_typed) {
-        weight_classes_launch(raw_a.as<float4>(), n_a, &d_stats->weights[0], C.sm_count, s);
-        weight_classes_launch(raw_w.as<float4>(), n_w, &d_stats->weights[1], C.sm_count, s);
-    }
     C.check_launch("census");
     AUSAXS_CUDA(cudaMemcpyAsync(h_stats, d_stats, sizeof(PrepStats), cudaMemcpyDeviceToHost, s));
 }
@@ -205,21 +201,19 @@ void Structure::load_end(const PrepStats& st) {
         if (n_a > 0) C.launches += 1;  // two kernels
         return;
     }
-    // weighted: the points by class of weight
+    // weighted: the points by class of weight, where both sets have few of them
     n_cls[0] = n_cls[1] = 0;
+    std::vector<std::pair<unsigned, int>> found[2];
+    if (!st.weights[0].sorted(found[0]) || !st.weights[1].sorted(found[1])) return;
     for (int k = 0; k < 2; ++k) {
         const int n = k ? n_w : n_a;
-        if (st.weights[k].over || n == 0) continue;
-        std::vector<std::pair<unsigned, int>> found;
-        for (int i = 0; i < kMaxClasses; ++i)
-            if (st.weights[k].bits[i] != kNoClass) found.push_back({st.weights[k].bits[i], st.weights[k].count[i]});
-        std::sort(found.begin(), found.end());
+        if (n == 0) continue;
         TypeMap map;
-        map.classes = n_cls[k] = (int)found.size();
-        for (size_t i = 0; i < found.size(); ++i) {
-            map.bits[i] = found[i].first;
-            std::memcpy(&cls[k][i], &found[i].first, 4);
-            cls_count[k][i] = found[i].second;
+        map.classes = n_cls[k] = (int)found[k].size();
+        for (size_t i = 0; i < found[k].size(); ++i) {
+            map.bits[i] = found[k][i].first;
+            std::memcpy(&cls[k][i], &found[k][i].first, 4);
+            cls_count[k][i] = found[k][i].second;
         }
         DevBuf& dense = k ? dense_w : dense_a;
         DevBuf& mem = k ? typed_w : typed;

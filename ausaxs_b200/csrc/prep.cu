@@ -18,7 +18,73 @@ __device__ __forceinline__ unsigned int f2o(float f) {
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-__global__ void census_kernel(const float4* p, int n, int ff_typed, PrepStats* st) {
+// first slot of a weight in a table of classes
+__device__ __forceinline__ unsigned class_hash(unsigned w) { return (w * 2654435761u) >> 27; }
+static_assert(kClassSlots == 32, "one slot per lane, and five hash bits");
+
+// The block's table starts with the weights of its first warp of points, one after the other (lane k keeps slot k):
+// with every thread inserting its own, the first round was a string of compare-and-swaps of many lanes to one
+// word.
+__device__ void class_begin(WeightClasses& t, const float4* p, int n) {  // (a barrier follows)
+    const int lane = threadIdx.x;
+    if (lane >= 32) return;
+    const int i = blockIdx.x * blockDim.x + lane;
+    const unsigned w = i < n ? __float_as_uint(p[i].w) : kNoClass;
+    unsigned left = __ballot_sync(0xffffffffu, i < n);
+    unsigned mine = kNoClass;
+    int found = 0;
+    bool over = false;
+    while (left) {
+        const unsigned x = __shfl_sync(0xffffffffu, w, __ffs(left) - 1);
+        if (x == kNoClass || ++found > kMaxClasses) {
+            over = true;
+            break;
+        }
+        const unsigned h = class_hash(x), empty = __ballot_sync(0xffffffffu, mine == kNoClass);
+        if (lane == static_cast<int>((__ffs(__funnelshift_r(empty, empty, h)) - 1 + h) & 31u)) mine = x;
+        left &= ~__ballot_sync(0xffffffffu, w == x);
+    }
+    t.bits[lane] = mine;
+    t.count[lane] = 0;
+    if (lane == 0) t.over = over;
+}
+
+// Slots are never emptied, so a weight is met before the first empty slot after its own.
+__device__ void class_add(WeightClasses& t, unsigned w) {
+    if (*reinterpret_cast<volatile int*>(&t.over)) return;
+    for (unsigned j = 0, k = class_hash(w); w != kNoClass && j < kClassSlots; ++j, k = (k + 1) & 31u) {
+        unsigned have = *reinterpret_cast<volatile unsigned*>(t.bits + k);
+        if (have == kNoClass) have = atomicCAS(t.bits + k, kNoClass, w);
+        if (have == kNoClass || have == w) {
+            atomicAdd(t.count + k, 1);
+            return;
+        }
+    }
+    t.over = 1;
+}
+
+// The block's table into the device's, a thread per slot (a barrier precedes).
+__device__ void class_merge(const WeightClasses& t, WeightClasses* out) {
+    if (threadIdx.x < kClassSlots && t.bits[threadIdx.x] != kNoClass && !t.over) {
+        const unsigned w = t.bits[threadIdx.x];
+        unsigned j = 0;
+        for (unsigned k = class_hash(w); j < kClassSlots; ++j, k = (k + 1) & 31u) {
+            unsigned have = __ldcg(out->bits + k);
+            if (have == kNoClass) have = atomicCAS(out->bits + k, kNoClass, w);
+            if (have == kNoClass || have == w) {
+                atomicAdd(out->count + k, t.count[threadIdx.x]);
+                break;
+            }
+        }
+        if (j == kClassSlots) out->over = 1;
+    }
+    if (threadIdx.x == 0 && t.over) out->over = 1;
+}
+
+// classes: also the points' distinct weights, or null
+__global__ void census_kernel(const float4* p, int n, int ff_typed, PrepStats* st, WeightClasses* classes) {
+    __shared__ WeightClasses s_class;
+    if (classes) class_begin(s_class, p, n);
     __shared__ unsigned int s_lo[3], s_hi[3], s_mask, s_bad;
     __shared__ int s_count[kNff];
     if (threadIdx.x < 3) {
@@ -45,6 +111,7 @@ __global__ void census_kernel(const float4* p, int n, int ff_typed, PrepStats* s
                 atomicAdd(&s_count[t], 1);
             }
         }
+        if (classes) class_add(s_class, __float_as_uint(v.w));
     }
     for (int k = 0; k < 3; ++k) {
         atomicMin(&s_lo[k], lo[k]);
@@ -60,6 +127,7 @@ __global__ void census_kernel(const float4* p, int n, int ff_typed, PrepStats* s
         atomicOr(&st->mask, s_mask);
         atomicOr(&st->bad, s_bad);
     }
+    if (classes) class_merge(s_class, classes);
 }
 
 __device__ __forceinline__ float o2f(unsigned int o) {
@@ -168,47 +236,15 @@ __global__ void __launch_bounds__(kTypedChunk) typed_scatter_sets_kernel(const T
     if (static_cast<int>(blockIdx.x) * kTypedChunk < S.n) typed_scatter(S.dense, S.n, S.out, S.counts);
 }
 
-// slot of w in a table of distinct values, inserted where it is new; -1: the table is full
-__device__ int class_slot(unsigned* bits, unsigned w) {
-    for (int k = 0; k < kMaxClasses; ++k) {
-        unsigned have = *reinterpret_cast<volatile unsigned*>(bits + k);
-        if (have == kNoClass) have = atomicCAS(bits + k, kNoClass, w);
-        if (have == kNoClass || have == w) return k;
-    }
-    return -1;
-}
-
-// every block's distinct weights in shared memory, then into the global table
-__device__ void weight_classes(const float4* p, int n, WeightClasses* out) {
-    __shared__ unsigned s_bits[16];
-    __shared__ int s_count[16], s_over;
-    if (threadIdx.x < 16) {
-        s_bits[threadIdx.x] = kNoClass;
-        s_count[threadIdx.x] = 0;
-    }
-    if (threadIdx.x == 0) s_over = 0;
-    __syncthreads();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const unsigned w = __float_as_uint(p[i].w);
-        const int k = w == kNoClass ? -1 : class_slot(s_bits, w);
-        if (k < 0) {
-            s_over = 1;
-            continue;
-        }
-        const unsigned same = __match_any_sync(__activemask(), k);
-        if ((threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&s_count[k], __popc(same));
-    }
-    __syncthreads();
-    if (threadIdx.x < kMaxClasses && s_bits[threadIdx.x] != kNoClass) {
-        const int k = class_slot(out->bits, s_bits[threadIdx.x]);
-        if (k < 0) out->over = 1;
-        else atomicAdd(&out->count[k], s_count[threadIdx.x]);
-    }
-    if (threadIdx.x == 0 && s_over) out->over = 1;
-}
-__global__ void weight_classes_kernel(const float4* p, int n, WeightClasses* out) { weight_classes(p, n, out); }
 __global__ void weight_classes_sets_kernel(const TypedSetJob* sets, WeightClasses* out) {
-    weight_classes(sets[blockIdx.y].in, sets[blockIdx.y].n, out + blockIdx.y);
+    __shared__ WeightClasses s_class;
+    const float4* p = sets[blockIdx.y].in;
+    const int n = sets[blockIdx.y].n;
+    class_begin(s_class, p, n);
+    __syncthreads();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) class_add(s_class, __float_as_uint(p[i].w));
+    __syncthreads();
+    class_merge(s_class, out + blockIdx.y);
 }
 
 __global__ void set_type_kernel(float4* p, int n, int32_t value) {
@@ -217,11 +253,25 @@ __global__ void set_type_kernel(float4* p, int n, int32_t value) {
 
 }  // namespace
 
-void census_launch(const float4* p, int n, int ff_typed, PrepStats* st, int sm_count, cudaStream_t s) {
+void WeightClasses::clear() {
+    std::fill(bits, bits + kClassSlots, kNoClass);
+    std::fill(count, count + kClassSlots, 0);
+    over = 0;
+}
+
+bool WeightClasses::sorted(std::vector<std::pair<unsigned, int>>& out) const {
+    out.clear();
+    for (int k = 0; k < kClassSlots; ++k)
+        if (bits[k] != kNoClass) out.push_back({bits[k], count[k]});
+    std::sort(out.begin(), out.end());
+    return !over && out.size() <= static_cast<size_t>(kMaxClasses);
+}
+
+void census_launch(const float4* p, int n, int ff_typed, PrepStats* st, WeightClasses* classes, int sm_count, cudaStream_t s) {
     if (n <= 0) return;
     int blocks = (n + 255) / 256;
     if (blocks > sm_count * 2) blocks = sm_count * 2;
-    census_kernel<<<blocks, 256, 0, s>>>(p, n, ff_typed, st);
+    census_kernel<<<blocks, 256, 0, s>>>(p, n, ff_typed, st, classes);
 }
 
 void radius_launch(const float4* a, int na, const float4* w, int nw, const float4* x, int nx, PrepStats* st,
@@ -239,11 +289,6 @@ void typed_lists_launch(const float4* in, float4* dense, int n, const TypeMap& m
     const int chunks = typed_chunks(n);
     dense_count_kernel<<<chunks, kTypedChunk, 0, s>>>(in, dense, n, map, counts);
     typed_scatter_kernel<<<chunks, kTypedChunk, 0, s>>>(dense ? dense : in, n, o, counts);
-}
-
-void weight_classes_launch(const float4* p, int n, WeightClasses* out, int sm_count, cudaStream_t s) {
-    if (n <= 0) return;
-    weight_classes_kernel<<<std::min((n + 255) / 256, sm_count * 2), 256, 0, s>>>(p, n, out);
 }
 
 constexpr int kMaxSets = 65535;  // gridDim.y of one launch

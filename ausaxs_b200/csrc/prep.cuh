@@ -1,17 +1,25 @@
 // Point-set preparation kernels (see prep.cu).
 #pragma once
+#include <utility>
+#include <vector>
+
 #include <string.h>
 #include "common.cuh"
 
 namespace ausaxs_b200 {
 
-// The distinct weights of a point set (bit patterns, in the order they were met) and their points.
+// The distinct weights of a point set and their points, by bit pattern: a hashed table with open addressing, so
+// that blocks meet in few of its slots.  Up to kMaxClasses of them are used; a table of more is of no use.
 constexpr int kMaxClasses = 15;
+constexpr int kClassSlots = 32;
 constexpr unsigned kNoClass = 0xffffffffu;  // an empty slot (a NaN pattern)
 struct WeightClasses {
-    unsigned bits[16];
-    int count[16];
-    int over;  // more than kMaxClasses of them (or kNoClass itself)
+    unsigned bits[kClassSlots];
+    int count[kClassSlots];
+    int over;  // some block met more than kMaxClasses (or kNoClass itself)
+    void clear();
+    // the weights in ascending order of their bit patterns, and their points; false: more than kMaxClasses
+    bool sorted(std::vector<std::pair<unsigned, int>>& out) const;
 };
 
 struct PrepStats {
@@ -24,7 +32,8 @@ struct PrepStats {
     WeightClasses weights[2];  // weighted structures: atoms, waters
 };
 
-void census_launch(const float4* p, int n, int ff_typed, PrepStats* st, int sm_count, cudaStream_t s);
+// classes: the points' distinct weights are added to it (cleared before); may be null
+void census_launch(const float4* p, int n, int ff_typed, PrepStats* st, WeightClasses* classes, int sm_count, cudaStream_t s);
 // After the census launches on the same stream: the radius of the points about the box centre
 // (every pair distance is at most twice it).
 void radius_launch(const float4* a, int na, const float4* w, int nw, const float4* x, int nx, PrepStats* st,
@@ -63,8 +72,6 @@ struct TypedSetJob {
 };
 void weight_classes_sets_launch(const TypedSetJob* sets_dev, int sets, int max_n, WeightClasses* out, cudaStream_t s);
 void typed_sets_launch(const TypedSetJob* sets_dev, int sets, int max_n, const TypeMap& map, cudaStream_t s);
-// the distinct weights of n points, added to *out (slots preset to kNoClass, counts to 0)
-void weight_classes_launch(const float4* p, int n, WeightClasses* out, int sm_count, cudaStream_t s);
 void set_type_launch(float4* p, int n, int32_t value, int sm_count, cudaStream_t s);
 float ordered_to_float(unsigned int o);
 
