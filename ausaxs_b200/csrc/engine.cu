@@ -810,10 +810,11 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
         F.max_bin = reinterpret_cast<int32_t*>(base + P.off_maxbin);
         F.done = reinterpret_cast<unsigned*>(base + P.off_maxbin) + 16;
         F.n32 = reinterpret_cast<unsigned long long*>(base + slot_ws[2]);
+        F.by_class = by_class;
         F.ta = F.tw = 0;
         if (by_class) {
-            F.ta = std::max(1, n_cls[0]);  // (no atoms: their empty row)
-            F.tw = std::max(1, n_cls[1]);
+            F.ta = n_cls[0];
+            F.tw = n_cls[1];
             std::copy(cls[0], cls[0] + 16, F.class_a);
             std::copy(cls[1], cls[1] + 16, F.class_w);
             // 2^k with max|w_i w_j| * 2^k <= 2^30, and the diagonal sums of float(w * w)
@@ -900,7 +901,7 @@ void Structure::enqueue_histogram(const ausaxs_hist_config& cfg) {
     char* base = P.dev.as<char>();
     AUSAXS_CUDA(cudaMemsetAsync(base + P.off_acc, 0, P.acc_bytes, s));
     const bool mt = cfg.manager == AUSAXS_MANAGER_MT;
-    if (mt && P.fin_mt.ta == 0) {
+    if (mt && !P.fin_mt.by_class) {
         weight_scale_launch(raw_a.as<float4>(), n_a, raw_w.as<float4>(), n_w, reinterpret_cast<float*>(base + P.off_wscale), s);
         weight_square_sum_launch(raw_a.as<float4>(), n_a, reinterpret_cast<double*>(base + P.off_self), s);
         weight_square_sum_launch(raw_w.as<float4>(), n_w, reinterpret_cast<double*>(base + P.off_self) + 1, s);

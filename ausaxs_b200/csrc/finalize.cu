@@ -237,7 +237,8 @@ __global__ void weight_scale_kernel(const float4* a, int na, const float4* b, in
 }
 
 // Pairs and fixed-point weight sum of one job in bin b.  The two-atomic kernel adds rint(w_i w_j * wscale) +
-// 2^30 per pair (unsigned, wrapping) and the bias of n pairs is removed; rows by class give the same sum.
+// 2^30 per pair (unsigned, wrapping) and the bias of n pairs is removed; rows by class give the same sum.  rows 0:
+// not by class, or no such pairs (one row of zeros).
 struct MTSum {
     unsigned long long n;
     long long w;
@@ -265,11 +266,11 @@ __global__ void mt_finalize_kernel(FinalizeMT F) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     bool in_use = false;
     if (b < F.nb) {
-        const float wscale = F.ta ? F.wscale_v : *F.wscale;
+        const float wscale = F.by_class ? F.wscale_v : *F.wscale;
         const double inv = 1.0 / static_cast<double>(wscale);
         const MTSum s_aa = mt_sum(F.c_aa, F.w_aa, F.ta, F.ta, F.class_a, F.class_a, wscale, nb, b);
         const MTSum s_aw = mt_sum(F.c_aw, F.w_aw, F.ta ? F.tw : 0, F.ta, F.class_w, F.class_a, wscale, nb, b);
-        const MTSum s_ww = mt_sum(F.c_ww, F.w_ww, F.ta ? F.tw : 0, F.tw, F.class_w, F.class_w, wscale, nb, b);
+        const MTSum s_ww = mt_sum(F.c_ww, F.w_ww, F.tw, F.tw, F.class_w, F.class_w, wscale, nb, b);
         double aa = 2.0 * (static_cast<double>(s_aa.w) * inv);
         double aw = 2.0 * (static_cast<double>(s_aw.w) * inv);
         double ww = 2.0 * (static_cast<double>(s_ww.w) * inv);
@@ -279,7 +280,7 @@ __global__ void mt_finalize_kernel(FinalizeMT F) {
                           2.0 * dist_sum(F.ds_aw, s_aw.n, b, F.c, F.scale);
         double v = aa + ww + aw;  // (the order in which bins count as used)
         if (b == 0) {
-            const double d_aa = F.ta ? F.self_v[0] : *F.self_aa, d_ww = F.ta ? F.self_v[1] : *F.self_ww;
+            const double d_aa = F.by_class ? F.self_v[0] : *F.self_aa, d_ww = F.by_class ? F.self_v[1] : *F.self_ww;
             aa += d_aa;
             ww += d_ww;
             v += d_aa + d_ww;

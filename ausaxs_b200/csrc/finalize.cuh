@@ -53,9 +53,10 @@ struct FinalizeMT {
     const unsigned long long *c_aa, *c_aw, *c_ww;
     const unsigned long long *ds_aa, *ds_aw, *ds_ww;
     const long long *w_aa, *w_aw, *w_ww;
-    // Weights of few distinct values (ta > 0): the counts are rows by the two points' classes, [ta][ta], [tw][ta]
-    // and [tw][tw], and the weight sums follow from them; scale and diagonal sums are given by value.
-    int32_t ta, tw;
+    // Weights of few distinct values (by_class): the counts are rows by the two points' classes, [ta][ta], [tw][ta]
+    // and [tw][tw], and the weight sums follow from them; scale and diagonal sums are given by value.  ta or tw 0:
+    // no such points, and none of their rows.
+    int32_t by_class, ta, tw;
     float class_a[16], class_w[16];
     float wscale_v;
     double self_v[2];

@@ -5,6 +5,7 @@ import pytest
 
 import ausaxs_b200 as ab
 from ausaxs_b200 import _capi, hist, synth
+from oracle import py as O
 
 pytestmark = pytest.mark.gpu
 
@@ -68,4 +69,27 @@ def test_rejected_call_leaves_no_plan(kind):
                 ab.profile(MANAGERS[kind](m, True, 5e-4, 400000, ctx), Q)
             assert e.value.code == _capi.ERR_CAPACITY
         np.testing.assert_array_equal(profile(kind, m, ctx), alone(kind, m))
+    ctx.close()
+
+
+@pytest.mark.parametrize("classes", [1, 5, 8, 15])
+@pytest.mark.parametrize("n", [60, 301, 900])
+def test_weighted_points_of_one_kind(classes, n):
+    """Only atoms, or only waters, after a molecule of both: no rows of the missing kind are read.  The weights are
+    whole numbers, so the sums are exact; a bin's mean is within the quantisation of its offsets."""
+    ctx = _capi.Context(0)
+    rng = np.random.default_rng(n + classes)
+    w = (1.0 + np.arange(n) % classes)[rng.permutation(n)]
+    xyz, none = synth.globule(n, n)[0], np.zeros((0, 3))
+    both = ab.Molecule(atoms=xyz, weights=w, waters=xyz[::2] + 7.3, water_weights=w[::2])
+    for atoms, waters in ((True, True), (True, False), (False, True)):
+        m = ab.Molecule(atoms=both.atoms if atoms else none, weights=w if atoms else w[:0],
+                        waters=both.waters if waters else none, water_weights=w[::2] if waters else w[:0])
+        h = hist.HistogramManagerMT(m, True, 0.25, 8000, ctx).calculate_all()
+        o = O.hist_simple(*m.compact_w(), 0.25, 8000)
+        assert h.max_bin == len(o.tot)
+        for got, want in ((h.get_aa_counts(), o.aa), (h.get_aw_counts(), o.aw), (h.get_ww_counts(), o.ww),
+                          (h.get_counts(), o.tot)):
+            np.testing.assert_array_equal(got, want)
+        np.testing.assert_allclose(h.get_d_axis(), o.d_axis, rtol=0, atol=0.25 * 2.0 ** -15)
     ctx.close()
