@@ -203,6 +203,7 @@ void Structure::load_end(const PrepStats& st) {
     }
     // weighted: the points by class of weight, where both sets have few of them
     n_cls[0] = n_cls[1] = 0;
+    std::memset(cls_count, 0, sizeof cls_count);
     std::vector<std::pair<unsigned, int>> found[2];
     if (!st.weights[0].sorted(found[0]) || !st.weights[1].sorted(found[1])) return;
     for (int k = 0; k < 2; ++k) {
@@ -527,6 +528,7 @@ bool Structure::upload_pack(Plan& P) {
     P.manager = 0;  // (until the tables are on their way)
     if (!choose_pack(P, ctx->sm_count, P.pack, P.pack_shape, P.pack_grid, table)) return false;
     std::copy(type_count, type_count + T, P.type_count);
+    std::memcpy(P.cls_count, cls_count, sizeof cls_count);
     char* base = P.dev.as<char>();
     const size_t jobs_bytes = sizeof(PackJob) * table.jobs.size(), out_bytes = sizeof(void*) * table.out.size();
     if (jobs_bytes + out_bytes > P.off_acc - P.off_jobs) throw Error{AUSAXS_ERR_CAPACITY, "too many pair jobs"};
@@ -542,6 +544,27 @@ bool Structure::upload_pack(Plan& P) {
     AUSAXS_CUDA(cudaMemcpyAsync(base + P.off_jobs, bytes.data(), bytes.size(), cudaMemcpyHostToDevice, ctx->stream));
     P.manager = manager;
     return true;
+}
+
+// The classes' weights of the loaded points, with the scale 2^k of their products (max|w_i w_j| * 2^k <= 2^30) and the
+// diagonal sums of float(w * w).
+void Structure::set_classes(FinalizeMT& F) const {
+    F.ta = n_cls[0];
+    F.tw = n_cls[1];
+    std::copy(cls[0], cls[0] + 16, F.class_a);
+    std::copy(cls[1], cls[1] + 16, F.class_w);
+    float m = 0;
+    for (int k = 0; k < 2; ++k) {
+        F.self_v[k] = 0;
+        for (int i = 0; i < n_cls[k]; ++i) {
+            m = std::max(m, std::fabs(cls[k][i]));
+            F.self_v[k] += (double)cls_count[k][i] * (double)(cls[k][i] * cls[k][i]);
+        }
+    }
+    const double p = (double)m * m;
+    int e = 0;
+    if (p > 0) std::frexp(p, &e);
+    F.wscale_v = std::ldexp(1.0f, std::min(60, 30 - e));
 }
 
 Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
@@ -561,10 +584,11 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     const bool same = P.manager == cfg.manager && P.weighted == weighted && P.bin_count == cfg.bin_count &&
         P.bin_width == cfg.bin_width && P.points == point_buffers() && P.n_a == n_a && P.n_w == n_w && P.n_x == n_x &&
         P.T == T && P.nb >= nb && P.nb <= nb + 64 && (cfg.manager != AUSAXS_MANAGER_FFGRID || n_x < kLatticeMinPoints || lat.tried) &&
-        std::equal(n_cls, n_cls + 2, P.n_cls) && std::memcmp(cls, P.cls, sizeof cls) == 0 &&
-        std::memcmp(cls_count, P.cls_count, sizeof cls_count) == 0 && std::equal(type_ff, type_ff + T, P.type_ff);
-    // one-shot calls of one shape: only the lists by type have other lengths
-    if (same && (!P.packed || std::equal(type_count, type_count + T, P.type_count) || upload_pack(P))) {
+        std::equal(n_cls, n_cls + 2, P.n_cls) && std::equal(type_ff, type_ff + T, P.type_ff);
+    // one-shot calls of one shape: only the lists by type or class have other lengths, and the classes other weights
+    const bool same_lists = std::equal(type_count, type_count + T, P.type_count) && std::memcmp(cls_count, P.cls_count, sizeof cls_count) == 0;
+    if (same && (!P.packed || same_lists || upload_pack(P))) {
+        if (cfg.manager == AUSAXS_MANAGER_MT && P.fin_mt.by_class) set_classes(P.fin_mt);
         P.covered = covered;
         P.pack.covered = covered;
         P.fin_ff.z_exv = cfg.z_exv;  // per call: other molecules of the same shape have other volumes
@@ -587,7 +611,6 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     std::copy(type_ff, type_ff + T, P.type_ff);
     std::copy(type_count, type_count + T, P.type_count);
     std::copy(n_cls, n_cls + 2, P.n_cls);
-    std::memcpy(P.cls, cls, sizeof cls);
     std::memcpy(P.cls_count, cls_count, sizeof cls_count);
     P.covered = covered;
     P.row_share = 1.0;
@@ -812,25 +835,7 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
         F.n32 = reinterpret_cast<unsigned long long*>(base + slot_ws[2]);
         F.by_class = by_class;
         F.ta = F.tw = 0;
-        if (by_class) {
-            F.ta = n_cls[0];
-            F.tw = n_cls[1];
-            std::copy(cls[0], cls[0] + 16, F.class_a);
-            std::copy(cls[1], cls[1] + 16, F.class_w);
-            // 2^k with max|w_i w_j| * 2^k <= 2^30, and the diagonal sums of float(w * w)
-            float m = 0;
-            for (int k = 0; k < 2; ++k) {
-                F.self_v[k] = 0;
-                for (int i = 0; i < n_cls[k]; ++i) {
-                    m = std::max(m, std::fabs(cls[k][i]));
-                    F.self_v[k] += (double)cls_count[k][i] * (double)(cls[k][i] * cls[k][i]);
-                }
-            }
-            const double p = (double)m * m;
-            int e = 0;
-            if (p > 0) std::frexp(p, &e);
-            F.wscale_v = std::ldexp(1.0f, std::min(60, 30 - e));
-        }
+        if (by_class) set_classes(F);
         F.H = reinterpret_cast<double*>(base + P.off_H);
         F.tot = reinterpret_cast<double*>(base + P.off_tot);
         F.d_axis = reinterpret_cast<double*>(base + P.off_d);

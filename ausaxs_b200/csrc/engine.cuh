@@ -109,7 +109,6 @@ struct Plan {
     int type_ff[kNff] = {};     // the form-factor types behind the rows
     int type_count[kNff] = {};  // and the sizes of the typed lists
     int n_cls[2] = {0, 0};      // weighted: the classes of atoms and waters behind the rows (0: by value)
-    float cls[2][16] = {};
     int cls_count[2][16] = {};
     // The point buffers behind the job tables (Structure::point_buffers).  Loads that are not followed by a plan
     // (grid dummies of another molecule, a rejected one) may have moved them.
@@ -207,6 +206,7 @@ struct Structure {
     }
     Plan& plan_for(const ausaxs_hist_config& cfg);
     bool upload_pack(Plan& P);
+    void set_classes(FinalizeMT& F) const;
     void enqueue_histogram(const ausaxs_hist_config& cfg);
     void enqueue_debye(const ausaxs_hist_config& cfg, const double* q_dev, int nq, const ausaxs_debye_params& p,
                        double* Iq_dev, double* prof_dev);

@@ -93,3 +93,24 @@ def test_weighted_points_of_one_kind(classes, n):
             np.testing.assert_array_equal(got, want)
         np.testing.assert_allclose(h.get_d_axis(), o.d_axis, rtol=0, atol=0.25 * 2.0 ** -15)
     ctx.close()
+
+
+@pytest.mark.parametrize("classes", [(4, 4), (4, 9), (15, 15), (6, 40)])
+def test_weights_change_between_calls(classes):
+    """Molecules of one shape and other weights: the same number of classes with other values and shares, another
+    number, and more than the route by class takes."""
+    ctx = _capi.Context(0)
+    n = 700
+    xyz = synth.globule(2, n)[0]
+    for k in range(4):
+        c = classes[k % 2]
+        rng = np.random.default_rng(10 * k + c)
+        values = rng.permutation(60)[:c] - 9.0
+        m = ab.Molecule(atoms=xyz + 0.01 * k, weights=values[np.concatenate([np.arange(c), rng.integers(0, 1 + c // 2, n - c)])],
+                        waters=xyz[::5] + 6.1, water_weights=np.full(len(xyz[::5]), 10.0 + k))
+        h = hist.HistogramManagerMT(m, True, 0.25, 8000, ctx).calculate_all()
+        o = O.hist_simple(*m.compact_w(), 0.25, 8000)
+        assert h.max_bin == len(o.tot)
+        for got, want in ((h.get_aa_counts(), o.aa), (h.get_aw_counts(), o.aw), (h.get_ww_counts(), o.ww)):
+            np.testing.assert_array_equal(got, want)
+    ctx.close()
