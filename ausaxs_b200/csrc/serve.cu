@@ -311,9 +311,9 @@ struct Assembly {
         std::vector<PairJob> all_jobs;
         std::vector<ZeroRange> all_zero;
         work.resize(B + 1);
-        int max_rows = 1;
-        for (int k = 0; k <= B; ++k) {  // k == B: every partial
-            Plan tmp;  // job-building view of the plan
+        std::vector<Plan> views(B + 1);  // job-building views of the plan
+        for (int k = 0; k <= B; ++k) {   // k == B: every partial
+            Plan& tmp = views[k];
             tmp.T = T;
             tmp.nb = nb;
             tmp.inv_w = P.inv_w;
@@ -335,51 +335,57 @@ struct Assembly {
                 zr.push_back({part.as<unsigned long long>(pt.off), (long long)((pt.rows + 1) * (size_t)nb)});
             }
             zr.push_back({part.as<unsigned long long>(counter_off), 1});
-            std::vector<PairJob> js[3];
-            long long tiles[3] = {0, 0, 0};
-            int rows[3] = {1, 1, 1};
-            append_pair_jobs(tmp, tile, false, js, tiles, rows);
             Work& Wk = work[k];
             Wk.zero_off = all_zero.size();
             Wk.n_zero = (int)zr.size();
             all_zero.insert(all_zero.end(), zr.begin(), zr.end());
-            Wk.L.n_jobs = (int)js[0].size();
-            Wk.L.total_tiles = tiles[0];
-            Wk.L.smem_rows = rows[0];
-            Wk.L.smem_bins = nb;
-            Wk.L.tile_counter = part.as<unsigned long long>(counter_off);
-            Wk.L.overflow = P.dev.as<unsigned long long>(P.off_overflow);
-            Wk.L.weighted = 0;
-            Wk.L.wscale = nullptr;
-            Wk.L.inv_w = P.inv_w;
-            Wk.L.jobs = reinterpret_cast<const PairJob*>(all_jobs.size());  // index, rebased below
-            all_jobs.insert(all_jobs.end(), js[0].begin(), js[0].end());
-            max_rows = std::max(max_rows, rows[0]);
-            if (packed) {
-                // Short-lived CTAs of one tile each, so that the block scheduler mixes moves (measured: two moves
-                // of a 10,000-atom body of 70,000 2.21 ms against 2.23 with two tiles per CTA and 2.73 with the
-                // two-atomic kernel).
-                PackTable T1;
-                int persistent = 0;
-                packed = choose_pack(tmp, sms, Wk.K, Wk.shape, persistent, T1, false) || tmp.specs.empty();
-                Wk.K.jobs = reinterpret_cast<const PackJob*>(pack_tables.jobs.size());  // indices, rebased below
-                Wk.K.out = reinterpret_cast<unsigned long long* const*>(pack_tables.out.size());
-                pack_tables.jobs.insert(pack_tables.jobs.end(), T1.jobs.begin(), T1.jobs.end());
-                pack_tables.out.insert(pack_tables.out.end(), T1.out.begin(), T1.out.end());
-                Wk.K.tile_counter = Wk.L.tile_counter;
-                Wk.K.overflow = Wk.L.overflow;
-                Wk.K.max_tiles = 1;
+            if (!packed) continue;
+            // Short-lived CTAs of one tile each, so that the block scheduler mixes moves (measured: two moves
+            // of a 10,000-atom body of 70,000 2.21 ms against 2.23 with two tiles per CTA and 2.73 with the
+            // two-atomic kernel).
+            PackTable T1;
+            int persistent = 0;
+            packed = choose_pack(tmp, sms, Wk.K, Wk.shape, persistent, T1, false) || tmp.specs.empty();
+            Wk.K.jobs = reinterpret_cast<const PackJob*>(pack_tables.jobs.size());  // indices, rebased below
+            Wk.K.out = reinterpret_cast<unsigned long long* const*>(pack_tables.out.size());
+            pack_tables.jobs.insert(pack_tables.jobs.end(), T1.jobs.begin(), T1.jobs.end());
+            pack_tables.out.insert(pack_tables.out.end(), T1.out.begin(), T1.out.end());
+            Wk.K.tile_counter = part.as<unsigned long long>(counter_off);
+            Wk.K.overflow = P.dev.as<unsigned long long>(P.off_overflow);
+            Wk.K.max_tiles = 1;
+        }
+        if (!packed) {
+            pack_tables = PackTable{};
+            int max_rows = 1;
+            for (int k = 0; k <= B; ++k) {
+                work[k].K = PackLaunch{};
+                std::vector<PairJob> js[3];
+                long long tiles[3] = {0, 0, 0};
+                int rows[3] = {1, 1, 1};
+                append_pair_jobs(views[k], tile, false, js, tiles, rows);
+                PairLaunch& L = work[k].L;
+                L.n_jobs = (int)js[0].size();
+                L.total_tiles = tiles[0];
+                L.smem_rows = rows[0];
+                L.smem_bins = nb;
+                L.tile_counter = part.as<unsigned long long>(counter_off);
+                L.overflow = P.dev.as<unsigned long long>(P.off_overflow);
+                L.weighted = 0;
+                L.wscale = nullptr;
+                L.inv_w = P.inv_w;
+                L.jobs = reinterpret_cast<const PairJob*>(all_jobs.size());  // index, rebased below
+                all_jobs.insert(all_jobs.end(), js[0].begin(), js[0].end());
+                max_rows = std::max(max_rows, rows[0]);
+            }
+            smem = pairhist_launch_smem(max_rows, nb, false, tile);
+            // two thread groups per CTA (pairhist_groups): a tile of a move's short-lived CTAs takes half
+            // the time, which shortens the last wave of a move (measured: the largest body's lone move
+            // 1.43 -> 1.38 ms p50, 2.54 -> 2.21 ms max; saturated moves/s +3 %)
+            for (Work& Wk : work) {
+                Wk.L.dreg = pairhist_dreg(max_rows, nb, false, tile) ? 1 : 0;
+                Wk.L.groups = Wk.L.dreg ? 1 : 2;
             }
         }
-        smem = pairhist_launch_smem(max_rows, nb, false, tile);
-        // two thread groups per CTA (pairhist_groups): a tile of a move's short-lived CTAs takes half
-        // the time, which shortens the last wave of a move (measured: the largest body's lone move
-        // 1.43 -> 1.38 ms p50, 2.54 -> 2.21 ms max; saturated moves/s +3 %)
-        for (Work& Wk : work) {
-            Wk.L.dreg = pairhist_dreg(max_rows, nb, false, tile) ? 1 : 0;
-            Wk.L.groups = Wk.L.dreg ? 1 : 2;
-        }
-        const int per_sm = pairhist_ctas_per_sm(smem, tile, pairhist_dreg(max_rows, nb, false, tile), false);
         // device tables: jobs, zero ranges, partial pointers of the master sum
         std::vector<const unsigned long long*> ptrs[3];
         for (const Part& pt : parts) ptrs[pt.kind].push_back(part.as<unsigned long long>(pt.off));
@@ -398,26 +404,27 @@ struct Assembly {
                                    cudaMemcpyHostToDevice));
             AUSAXS_CUDA(cudaMemcpy(tables.as<char>(pack_out_off), pack_tables.out.data(), sizeof(void*) * pack_tables.out.size(),
                                    cudaMemcpyHostToDevice));
+        } else {
+            AUSAXS_CUDA(cudaMemcpy(tables.p, all_jobs.data(), sizeof(PairJob) * all_jobs.size(), cudaMemcpyHostToDevice));
         }
-        AUSAXS_CUDA(cudaMemcpy(tables.p, all_jobs.data(), sizeof(PairJob) * all_jobs.size(), cudaMemcpyHostToDevice));
         AUSAXS_CUDA(cudaMemcpy(tables.as<char>(jobs_bytes), all_zero.data(), sizeof(ZeroRange) * all_zero.size(),
                                cudaMemcpyHostToDevice));
         for (int s = 0; s < 3; ++s)
             AUSAXS_CUDA(cudaMemcpy(tables.as<char>(ptr_off[s]), ptrs[s].data(), sizeof(void*) * ptrs[s].size(),
                                    cudaMemcpyHostToDevice));
         for (Work& Wk : work) {
-            Wk.L.jobs = tables.as<PairJob>() + reinterpret_cast<size_t>(Wk.L.jobs);
             Wk.zero_off = jobs_bytes + Wk.zero_off * sizeof(ZeroRange);
-            // short-lived CTAs of kServeTilesPerCta tiles each (one tile per grab), at least one wave
-            Wk.L.chunk = 1;
-            Wk.L.max_grabs = kServeTilesPerCta;
-            const long long need = (Wk.L.total_tiles + kServeTilesPerCta - 1) / kServeTilesPerCta;
-            Wk.grid = (int)std::max<long long>(1, std::min<long long>(need, (long long)INT32_MAX));
-            (void)per_sm;
             if (packed) {
                 Wk.K.jobs = tables.as<PackJob>(pack_jobs_off) + reinterpret_cast<size_t>(Wk.K.jobs);
                 Wk.K.out = tables.as<unsigned long long*>(pack_out_off) + reinterpret_cast<size_t>(Wk.K.out);
                 Wk.grid = (int)std::max<long long>(1, std::min<long long>(Wk.K.total_tiles, (long long)INT32_MAX));
+            } else {
+                Wk.L.jobs = tables.as<PairJob>() + reinterpret_cast<size_t>(Wk.L.jobs);
+                // short-lived CTAs of kServeTilesPerCta tiles each (one tile per grab), at least one wave
+                Wk.L.chunk = 1;
+                Wk.L.max_grabs = kServeTilesPerCta;
+                const long long need = (Wk.L.total_tiles + kServeTilesPerCta - 1) / kServeTilesPerCta;
+                Wk.grid = (int)std::max<long long>(1, std::min<long long>(need, (long long)INT32_MAX));
             }
         }
         // pair evaluations of a move of each body (the body against the rest, and its own pairs)
@@ -499,7 +506,7 @@ struct Assembly {
     void enqueue_pairs(const Work& Wk) {
         zero_ranges_launch(tables.as<ZeroRange>(Wk.zero_off), Wk.n_zero, C.stream);
         C.check_launch("zero");
-        if (packed && Wk.K.n_jobs > 0) {
+        if (Wk.K.n_jobs > 0) {
             pack_launch(Wk.K, Wk.shape, Wk.grid, C.stream);
             C.check_launch("pairpack");
         } else if (Wk.L.n_jobs > 0) {
