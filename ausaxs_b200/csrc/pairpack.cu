@@ -672,7 +672,9 @@ int pack_segment_pairs(int bins, double largest_row_share) {
 void pack_launch(const PackLaunch& L, int shape, int grid, cudaStream_t s) {
     const size_t smem = pack_smem_bytes(L);
     Kernel k = L.covered ? pick_shape<false>(shape, L.nr, L.offsets != 0) : pick_shape<true>(shape, L.nr, L.offsets != 0);
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    // the most any launch takes, not this one's: the limit belongs to the process, and another thread's launch may
+    // come between the two calls
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kPairSmemCap));
     k<<<grid, kPackShapes[shape].threads, smem, s>>>(L);
 }
 
