@@ -525,7 +525,7 @@ struct Batch {
         ctx->check_launch("qfactors");
         int max_R = 1;
         for (auto& S : items) max_R = std::max(max_R, S->plan.R);
-        debye_fp64_batch_launch(args.as<DebyeArgs>(), (int)items.size(), nq, max_R, s);
+        debye_fp64_batch_launch(args.as<DebyeArgs>(), (int)items.size(), nq, max_R, max_nb, s);
         ctx->check_launch("debye");
     }
 

@@ -165,15 +165,29 @@ __global__ void debye_qfactors_kernel(DebyeArgs A, double* out) {
 }
 
 // q values per CTA by the transform's q count: few enough that small transforms reach most SMs (200 q: 100
-// CTAs), more for larger ones, whose CTAs then share every row they read.  The decomposition depends on
-// nq alone, so a structure's I(q) has the same bits alone or in a batch.
+// CTAs), more for larger ones, whose CTAs then share every row they read.  The sums are cut where chunks of bins
+// end and are the same for any q count otherwise.
 constexpr int debye_qt(int nq) { return nq <= 296 ? 2 : (nq <= 592 ? 4 : (nq <= 2368 ? 8 : 16)); }
+
+constexpr int debye_chunk(int qt) { return 4096 / qt; }  // bins per chunk: 32 KB of sinc values
+
+// Batches that fill the GPU many times over (more than 8 CTAs of 256 threads per SM) take more q values per CTA, a
+// CTA of a few rows and bins being mostly its start: 300 structures of 300 atoms, 200 q, a whole profile 1,066
+// us with two q values per CTA, 535 with up to 16; 32 of 500 atoms 220 and 169; with limits of 2,368 and 4,736
+// CTAs 185 and 220.  Only where every structure's bins are one chunk either way, so that I(q) has the same bits
+// alone or in a batch.
+constexpr int kBatchCtas = 1184;
+constexpr int debye_batch_qt(int nq, int n, int max_nb) {
+    int qt = debye_qt(nq);
+    while (qt < 16 && max_nb <= debye_chunk(2 * qt) && static_cast<long long>((nq + qt - 1) / qt) * n > kBatchCtas) qt *= 2;
+    return qt;
+}
 
 // Shared memory of a CTA of QT q values: per-q factors, the chunk's sinc values [kCB][QT], the row sums
 // [QT][R] and the rows' distance-axis groups.
 template <int QT>
 struct QTile {
-    static constexpr int kCB = 4096 / QT;  // bins per chunk: 32 KB of sinc values
+    static constexpr int kCB = debye_chunk(QT);
     static constexpr size_t kOffS = ((sizeof(QFactors) * QT + 15) / 16) * 16;
     static constexpr size_t kOffAcc = kOffS + sizeof(double) * kCB * QT;
     static constexpr size_t smem(int R) { return kOffAcc + sizeof(double) * QT * R + sizeof(int) * R; }
@@ -450,9 +464,9 @@ void debye_fp64_launch(const DebyeArgs& A, cudaStream_t s) {
         default: debye_kernel<16><<<(A.nq + 15) / 16, kThreads, QTile<16>::smem(A.R), s>>>(A); break;
     }
 }
-void debye_fp64_batch_launch(const DebyeArgs* As_dev, int n, int nq, int max_R, cudaStream_t s) {
+void debye_fp64_batch_launch(const DebyeArgs* As_dev, int n, int nq, int max_R, int max_nb, cudaStream_t s) {
     debye_configure();
-    switch (debye_qt(nq)) {
+    switch (debye_batch_qt(nq, n, max_nb)) {
         case 2: debye_batch_kernel<2><<<dim3((nq + 1) / 2, n), kThreads, QTile<2>::smem(max_R), s>>>(As_dev); break;
         case 4: debye_batch_kernel<4><<<dim3((nq + 3) / 4, n), kThreads, QTile<4>::smem(max_R), s>>>(As_dev); break;
         case 8: debye_batch_kernel<8><<<dim3((nq + 7) / 8, n), kThreads, QTile<8>::smem(max_R), s>>>(As_dev); break;

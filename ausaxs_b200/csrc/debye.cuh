@@ -77,8 +77,8 @@ void debye_fp64_launch(const DebyeArgs& A, cudaStream_t s);
 // parameters into out [debye_qfactors_doubles(nq)]
 size_t debye_qfactors_doubles(int nq);
 void debye_qfactors_launch(const DebyeArgs& A, double* out, cudaStream_t s);
-// n transforms at once (device array of arguments; max_nq >= every nq, max_R >= every R)
-void debye_fp64_batch_launch(const DebyeArgs* As_dev, int n, int max_nq, int max_R, cudaStream_t s);
+// n transforms of nq q values each at once (device array of arguments; max_R >= every R, max_nb >= every nb)
+void debye_fp64_batch_launch(const DebyeArgs* As_dev, int n, int nq, int max_R, int max_nb, cudaStream_t s);
 
 // Split-BF16 tensor-core contraction sinqd[r][q] = sum_b H[r][b] sinc(q d_{g(r)}[b]) for all rows,
 // with the bound sum_b |H||sinc| per element (debye_tc.cu).  Returns false when the launch could not

@@ -25,3 +25,19 @@ def test_q_counts(nq, histogram):
     q = np.linspace(0.004, 0.9, nq)
     I = h.debye_transform(q)[1]
     np.testing.assert_allclose(I, O.debye_ff(0, o, q)[0], rtol=1e-6)  # (the mean distances are quantised)
+
+
+@pytest.mark.parametrize("spread", [1.0, 5.0, 9.0])
+@pytest.mark.parametrize("k,nq", [(3, 200), (40, 100), (40, 200), (40, 600), (200, 30), (200, 300)])
+def test_batches_equal_single_calls(spread, k, nq, gpu_ctx):
+    """Batches choose their q values per CTA by all of their structures: the same bits as each alone."""
+    molecules = []
+    for i in range(k):
+        xyz, ff = synth.globule(i, 40 + 7 * (i % 9))
+        molecules.append(hist.Molecule(atoms=xyz * spread, ff_types=ff, waters=xyz[::8] * spread + 3.1, volume=18.0 * len(xyz)))
+    q = np.linspace(0.005, 0.7, nq)
+    b = hist.BatchedProfiles(molecules, ctx=gpu_ctx)
+    I = b.debye_transform(q)
+    b.close()
+    for i in range(0, k, max(1, k // 9)):
+        np.testing.assert_array_equal(I[i], hist.profile(hist.HistogramManagerMTFFAvg(molecules[i], True, 0.25, 8000, gpu_ctx), q))
