@@ -182,11 +182,12 @@ struct Calculator {
         // than the sample has seldom change the answer, so the exact numbers only bound it
         bool classify = false;
         {
+            const int per_set = std::max(8, 256 / std::max(1, n_sets));  // (a cache miss each)
             std::vector<uint32_t> seen;
             double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
             for (int k = 0; k < n_sets && (int)seen.size() <= kMaxClasses; ++k) {
                 const float4* q = staged.data() + sets[k].off;
-                for (int i = 0; i < sets[k].n && (int)seen.size() <= kMaxClasses; i += 1 + sets[k].n / 64) {
+                for (int i = 0; i < sets[k].n && (int)seen.size() <= kMaxClasses; i += 1 + sets[k].n / per_set) {
                     uint32_t w;
                     std::memcpy(&w, &q[i].w, 4);
                     if (std::find(seen.begin(), seen.end(), w) == seen.end()) seen.push_back(w);
