@@ -21,8 +21,14 @@
 //     words that wrapped, the fields add up to N + C - 512 W; a segment has N < 65,536 pairs, hence C <
 //     2^16 N / 2^23 < 512, so the sum is N only if C = W = 0.  A segment that fails is taken back (its
 //     additions repeated, the same words subtracted) and evaluated again at half the length, or, at the
-//     smallest one, with two atomics per pair (count, offset).  The length follows the fullest word (110
-//     to 170 pairs: 1 to 3 % of the segments fail; 90 or 190 as the upper bound measured slower);
+//     smallest one, with two atomics per pair (count, offset).  The length follows the fullest word, scaled to
+//     a full segment (140 to 200 pairs; 110 to 170 measured up to 2 % slower), and a tile is cut into segments of
+//     about equal length (a short last one costs a whole drain: 12,000 atoms of one type, 0.25 A, 148 -> 131 us);
+//   * with few bins a word is full after few pairs.  Jobs then keep several copies of their words, the lanes of
+//     a warp in turn, until a segment lasts 24,576 pairs (pack_copies; 8,192 and 16,384 measured up to 12 %
+//     slower at 0.5 A bins, 32,768 up to 2 % at 0.25 A).  Whole calls without and with copies: 12,000 atoms of
+//     one type at 1 A 193 -> 146 us, at 2 A 344 -> 182; 25,000 atoms of four types at 1 A 564 -> 511, at 4 A
+//     1,573 -> 661; of 13 types at 2 A, whose water pairs have a word per bin, 4,162 -> 629;
 //   * rows are the outer point's type only: the inner points of a job share one type, so a CTA keeps T
 //     rows instead of T * T and no pair adds a row offset.
 // All accumulations are integer, so results do not depend on scheduling; counts and offsets are those of
@@ -33,6 +39,7 @@
 // warp instructions per 32 pairs, FMA pipe 64 %, shared-memory wavefronts 74 % of peak) against 1,040, of
 // a 264,000-point shell at 3,092 bins 1,240 against 990.  Per-segment drains and checks take about 15 %.
 #include <algorithm>
+#include <type_traits>
 
 #include "pairhist.cuh"
 #include "pairpack.cuh"
@@ -228,9 +235,9 @@ __device__ __forceinline__ void slow_pairs(const Quad* s_q, int k0, int k1, cons
     }
 }
 
-constexpr int kRoom = 512;  // 512 x 2^23 = 2^32 and 511 x 128 < 2^16
+constexpr int kRoom = 511;  // 511 x 2^23 < 2^32 and 511 x 128 < 2^16
 
-// Shared memory of a CTA: packed words [rows][pad], u32 offset sums [group_sums][pad], u16 counts
+// Shared memory of a CTA: packed words [copies][rows][pad], u32 offset sums [group_sums][pad], u16 counts
 // [group_rows][pad], two buffers of tile_j inner points; pad = bins + 1 (the overflow column) rounded up to
 // whole quads of bins.  Counts and offset sums go to the global accumulators when the CTA moves to another
 // group or when they could wrap (kRoom); 16-bit counts keep two CTAs on an SM at the 3,100 bins of a 300 A
@@ -404,7 +411,7 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
             ox[k] = pack2(a.x * S, a.x * S);
             oy[k] = pack2(a.y * S, a.y * S);
             oz[k] = pack2(a.z * S, a.z * S);
-            const int row = rows > 1 ? __float_as_int(a.w) : 0;
+            const int row = (rows > 1 ? __float_as_int(a.w) : 0) + (lane & (J.copies - 1)) * rows;
             caddr[k] = smem_addr(s_pk) + 4u * static_cast<uint32_t>(row * pad) - 4u * static_cast<uint32_t>(kMagicBits);
             gi[k] = J.a_base + i;
             p[k] = on ? 0 : 0x7fffffff;
@@ -477,9 +484,10 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
         auto slow = [&](int k0, int k1, int tail_end) {
             uint32_t row0[R];
             int ts[R];
+            const uint32_t copy = static_cast<uint32_t>((lane & (J.copies - 1)) * rows * pad);
 #pragma unroll
             for (int k = 0; k < R; ++k) {
-                row0[k] = (caddr[k] + 4u * static_cast<uint32_t>(kMagicBits) - smem_addr(s_pk)) / 4u;
+                row0[k] = (caddr[k] + 4u * static_cast<uint32_t>(kMagicBits) - smem_addr(s_pk)) / 4u - copy;
                 const int row_begin = J.tail_from_outer ? gi[k] + 1 : 0;
                 ts[k] = tail_end == 0x7fffffff ? tail_end : tail_end - ((tail_end - row_begin) & 3);
             }
@@ -488,7 +496,12 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
         };
         bool fetched = false, undo = false;
         for (int s0 = 0; s0 < kq || !fetched;) {
-            const int qa = min(kq, s0 + group * len), qb = min(kq, qa + len);
+            // what is left of the tile (quads per group) in segments of about equal length, at most len; quotients of
+            // numbers below 256 half a unit off the whole ones, so that an approximate division is exact
+            const int left = (kq - s0 + G - 1) / G;
+            const int parts = max(1, __float2int_rd(__fdividef(left + len - 0.5f, len)));
+            const int seg = __float2int_rd(__fdividef(left + parts - 0.5f, parts));
+            const int qa = min(kq, s0 + group * seg), qb = min(kq, qa + seg);
             int n = 0;
             if (s0 < kq && slow_left == 0) {
                 Consts K;
@@ -524,49 +537,62 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
                 // words -> counts and offset sums (undo: the same words again, taken back)
                 // a word holds less than 2^23 of offsets and 512 counts; what a segment adds stays on chip
                 // until its check, so that it can be taken back
-                const int use = max(rows, 4);
-                if (!undo && room < 2 * use) flush();
-                room -= use;
+                const int pk_rows = rows * J.copies, most = J.copies * max(rows, 4);
+                if (!undo && room < most) flush();
                 int sum = -n;
                 uint32_t fill = 0;
-                // few quads of bins: several threads share a quad's rows
+                // few quads of bins: several threads share a quad's rows (and, with several copies, a quad of counts)
                 const int quads = nb / 4 + 1;
-                const int split = quads * 2 <= NT ? min(rows, NT / quads) : 1;
-                const int first = split > 1 ? tid / quads : 0;
-                for (int b = (tid - first * quads) * 4; b <= nb && first < split; b += NT * 4) {
-                    uint4 off = make_uint4(0, 0, 0, 0);
-                    for (int r = first; r < rows; r += split) {
-                        uint4* const pw = reinterpret_cast<uint4*>(s_pk + r * pad + b);
-                        uint2* const pc = reinterpret_cast<uint2*>(s_cnt + r * pad + b);
-                        const uint4 w = *pw;
-                        uint2 c = *pc;
-                        *pw = make_uint4(0, 0, 0, 0);
-                        const uint32_t n0 = w.x >> kPackCountShift, n1 = w.y >> kPackCountShift, n2 = w.z >> kPackCountShift,
-                                       n3 = w.w >> kPackCountShift;
-                        const uint32_t c0 = n0 | n1 << 16, c1 = n2 | n3 << 16;
-                        c = undo ? make_uint2(c.x - c0, c.y - c1) : make_uint2(c.x + c0, c.y + c1);
-                        off = make_uint4(off.x + (w.x & kOffsetMask), off.y + (w.y & kOffsetMask), off.z + (w.z & kOffsetMask),
-                                         off.w + (w.w & kOffsetMask));
-                        *pc = c;
-                        sum += static_cast<int>(n0 + n1) + static_cast<int>(n2 + n3);
-                        fill = max(max(fill, w.x), w.y);
-                        fill = max(max(fill, w.z), w.w);
-                    }
-                    if (DSUM) {
-                        if (undo) off = make_uint4(0u - off.x, 0u - off.y, 0u - off.z, 0u - off.w);
-                        if (split > 1) {
-                            const uint32_t a = smem_addr(s_dacc + b);
-                            if (off.x) shared_red_add(a, off.x);
-                            if (off.y) shared_red_add(a + 4, off.y);
-                            if (off.z) shared_red_add(a + 8, off.z);
-                            if (off.w) shared_red_add(a + 12, off.w);
-                        } else {
-                            uint4* const pd = reinterpret_cast<uint4*>(s_dacc + b);
-                            const uint4 d = *pd;
-                            *pd = make_uint4(d.x + off.x, d.y + off.y, d.z + off.z, d.w + off.w);
+                auto drain = [&](auto several) {
+                    constexpr bool MANY = decltype(several)::value;
+                    const int split = quads * 2 <= NT ? min(pk_rows, NT / quads) : 1;
+                    const int first = split > 1 ? tid / quads : 0;
+                    for (int b = (tid - first * quads) * 4; b <= nb && first < split; b += NT * 4) {
+                        uint4 off = make_uint4(0, 0, 0, 0);
+                        int row = first;  // of the counts
+                        for (int r = first; r < pk_rows; r += split) {
+                            if (MANY)
+                                while (row >= rows) row -= rows;
+                            uint4* const pw = reinterpret_cast<uint4*>(s_pk + r * pad + b);
+                            uint2* const pc = reinterpret_cast<uint2*>(s_cnt + (MANY ? row : r) * pad + b);
+                            const uint4 w = *pw;
+                            uint2 c = MANY ? make_uint2(0, 0) : *pc;
+                            *pw = make_uint4(0, 0, 0, 0);
+                            const uint32_t n0 = w.x >> kPackCountShift, n1 = w.y >> kPackCountShift, n2 = w.z >> kPackCountShift,
+                                           n3 = w.w >> kPackCountShift;
+                            const uint32_t c0 = n0 | n1 << 16, c1 = n2 | n3 << 16;
+                            c = undo ? make_uint2(c.x - c0, c.y - c1) : make_uint2(c.x + c0, c.y + c1);
+                            off = make_uint4(off.x + (w.x & kOffsetMask), off.y + (w.y & kOffsetMask), off.z + (w.z & kOffsetMask),
+                                             off.w + (w.w & kOffsetMask));
+                            if (MANY) {
+                                if (c.x) shared_red_add(smem_addr(pc), c.x);
+                                if (c.y) shared_red_add(smem_addr(pc) + 4, c.y);
+                                row += split;
+                            } else {
+                                *pc = c;
+                            }
+                            sum += static_cast<int>(n0 + n1) + static_cast<int>(n2 + n3);
+                            fill = max(max(fill, w.x), w.y);
+                            fill = max(max(fill, w.z), w.w);
+                        }
+                        if (DSUM) {
+                            if (undo) off = make_uint4(0u - off.x, 0u - off.y, 0u - off.z, 0u - off.w);
+                            if (split > 1) {
+                                const uint32_t a = smem_addr(s_dacc + b);
+                                if (off.x) shared_red_add(a, off.x);
+                                if (off.y) shared_red_add(a + 4, off.y);
+                                if (off.z) shared_red_add(a + 8, off.z);
+                                if (off.w) shared_red_add(a + 12, off.w);
+                            } else {
+                                uint4* const pd = reinterpret_cast<uint4*>(s_dacc + b);
+                                const uint4 d = *pd;
+                                *pd = make_uint4(d.x + off.x, d.y + off.y, d.z + off.z, d.w + off.w);
+                            }
                         }
                     }
-                }
+                };
+                if (J.copies > 1) drain(std::true_type{});
+                else drain(std::false_type{});
                 sum = __reduce_add_sync(0xffffffffu, sum);
                 fill = __reduce_max_sync(0xffffffffu, fill);
                 if (lane == 0) {
@@ -586,24 +612,28 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
                         undo = true;
                         continue;
                     }
-                    s0 += G * len;
+                    // (a count has taken at most the fullest word's of every copy, the offset sums 2^23 of every word)
+                    room -= min(most, max(J.copies * static_cast<int>((full >> 7) + 1), pk_rows));
+                    s0 += G * seg;
                     // the fullest word's count decides the next segments' length
-                    if (full > 170) len = max(1, len - (len + 3) / 4);
-                    else if (full < 110) len = min(kMaxLen, len + (len + 7) / 8);
+                    if (full * len > 200 * seg) len = max(1, len - (len + 3) / 4);
+                    else if (full * len < 140 * seg) len = min(kMaxLen, len + (len + 7) / 8);
                     continue;
                 }
                 undo = false;
-                if (len > 1) {
-                    len = max(1, len / 2);
+                if (seg > 1) {
+                    len = seg / 2;
                     continue;
                 }
+                len = 1;
                 slow_left = 64;
             }
             // two atomics per pair: the segments after one whose words could not hold it at the smallest length
-            flush();
+            constexpr int kUse = NT * R * 4 / 128;  // one quad per thread and outer point
+            if (room < kUse) flush();
+            room -= kUse;
             slow(4 * qa, min(kt, 4 * qb), 0x7fffffff);
-            flush();
-            s0 += G * len;
+            s0 += G * seg;
             --slow_left;
         }
         if (kt < t.jn) {
@@ -664,9 +694,20 @@ int pack_shape(const PackLaunch& L) {
     return pack_ctas_per_sm(3, L) > 0 ? 3 : -1;
 }
 
+constexpr int kLongSegment = 24576;  // pairs of a segment that is long enough
+constexpr int kCopyWords = 4096;     // words that copies may take: a quarter of a resident CTA's shared memory
+
 int pack_segment_pairs(int bins, double largest_row_share) {
-    const double n = 52.0 * bins / std::max(0.05, largest_row_share);
+    const double n = 52.0 * bins / std::max(0.01, largest_row_share);
     return static_cast<int>(std::min<double>(n, kPackMaxPairs));
+}
+
+int pack_copies(int rows, int bins, int spread, double largest_row_share) {
+    int n = 1;
+    while (n < 16 && 2 * n * rows * pack_pad(bins) <= kCopyWords &&
+           pack_segment_pairs(spread, largest_row_share / n) < kLongSegment)
+        n *= 2;
+    return n;
 }
 
 void pack_launch(const PackLaunch& L, int shape, int grid, cudaStream_t s) {

@@ -28,7 +28,7 @@ struct alignas(16) PackJob {
     int32_t group, group_out, group_rows, group_sums;
     int32_t cnt_row, sum_slot;
     int32_t mult;         // multiplicity of every pair (jobs of a group share it)
-    int32_t pad;
+    int32_t copies;       // packed words of every row: a power of two, lanes take turns (pack_copies)
 };
 static_assert(sizeof(PackJob) == 128, "copied in 16-byte words");
 
@@ -37,7 +37,7 @@ struct PackLaunch {
     unsigned long long* const* out;  // u64 accumulators [nbins] of every group's rows and offset sums
     int32_t n_jobs;
     int64_t total_tiles;
-    int32_t rows;         // most rows of a job
+    int32_t rows;         // most packed rows (rows x copies) of a job
     int32_t group_rows, group_sums;  // most rows and offset sums of a group
     int32_t bins;         // most bins of a job
     int32_t tile_j;       // inner points per tile (a multiple of 4, at most kPackMaxTileJ)
@@ -70,6 +70,8 @@ int pack_shape(const PackLaunch& L);
 // pairs of a job's first segments: the most frequent cell of a protein-like distance distribution
 // then holds about 100 pairs
 int pack_segment_pairs(int bins, double largest_row_share);
+// copies of the packed words of a job of `rows` rows whose distances spread over `spread` of its bins
+int pack_copies(int rows, int bins, int spread, double largest_row_share);
 void pack_launch(const PackLaunch& L, int shape, int grid, cudaStream_t s);
 
 }  // namespace ausaxs_b200
