@@ -174,9 +174,18 @@ struct Calculator {
         // 2 results / 21 results, by class and by value): 300 points each, 15 classes 262 and 256 us / 1,045
         // and 985 us, 8 classes 222 and 256 / 959 and 985; 3,000 points, 15 classes 436 and 431 / 1,347 and 1,357,
         // 4 classes 365 and 431 / 1,221 and 1,357; 50 points (13,700 pairs), 8 classes 217 and 192.
+        // A class also costs a pass of its own per job, and what a class saves is a part of the pairs' time: the price
+        // of such a pass, in pairs, is from the second list on (40 sets, all pairs of sets: 100 points, 5 and 15 classes
+        // 713 and 4,430 us against 260 by value; 300 points, 2 and 5 classes 576 and 931 / 522; 1,000 points, 5
+        // classes 1,769 / 1,893; 12 sets of 1,000, 5 and 15 classes 331 and 554 / 345).  Jobs of at least 256 x 256
+        // points gain something whatever their number, since they are cut into more tiles (6 sets of 300, 8 classes
+        // 172 / 186; 2 of 1,000, 5 classes 166 / 219).
+        const long long n_jobs = (long long)jobs.size();
         auto rows_pay = [&](long long classes, long long bins, int least) {
             const long long words = n_slots * classes * classes * bins;
-            return words * 8 <= (long long)Ctx::kCalcKeep && least * words <= pairs;
+            const long long price = n_jobs * (classes - 1) * (150000 + 15000 * classes);
+            return words * 8 <= (long long)Ctx::kCalcKeep && least * words <= pairs &&
+                   price <= pairs + (pairs >= 65536 * n_jobs ? 72000000 : 0);
         };
         // by a sample of the points, which costs no launch (its classes and extent are lower bounds); more points
         // than the sample has seldom change the answer, so the exact numbers only bound it

@@ -184,3 +184,17 @@ def test_more_sets_than_a_grid_has_rows(gpu_ctx):
         count[0] += np.floor(36.0 * m) * len(part)
         assert np.abs(out["self"][mid][1] - count).sum() <= 40  # (roundings at bin edges)
         assert out["self"][mid][1].sum() == count.sum()
+
+
+@pytest.mark.parametrize("classes,sizes,launches", [(5, (60,) * 20, 3), (15, (300,) * 20, 3), (1, (60,) * 20, 5), (5, (900,) * 3, 5)])
+def test_many_jobs_by_class(classes, sizes, launches, gpu_ctx):
+    """A pass per class and job: many small jobs of several classes go by value (weight scale, pairs, results), others by
+    class (classes, lists of two kernels, pairs, results)."""
+    sets = class_sets(classes, sizes)
+    jobs = [(a, None, 1, 0) for a in range(len(sets))]
+    jobs += [(a, b, 2, 1) for a in range(len(sets)) for b in range(a + 1, len(sets))]
+    before = gpu_ctx.launches
+    out, _ = run_gpu(gpu_ctx, sets, jobs, 0.25)
+    assert gpu_ctx.launches - before == launches
+    for (cross, mid), ref in O.calculator(sets, jobs, 0.25, 8000).items():
+        check_result(out["cross" if cross else "self"][mid], ref, sets, 0.25, 8000)
