@@ -20,6 +20,7 @@ Structure& scratch(Ctx& C) {
     if (!C.scratch) {
         C.scratch = std::make_unique<Structure>();
         C.scratch->ctx = &C;
+        C.scratch->one_shot = true;
     }
     return *C.scratch;
 }

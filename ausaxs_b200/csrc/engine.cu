@@ -85,6 +85,27 @@ void Ctx::time_collect() {
     }
 }
 
+// Distinct weights among a sample of host points (at most kMaxClasses + 1 are counted).
+static int sampled_weights(const float* pts, int n) {
+    unsigned seen[kMaxClasses + 1];
+    int found = 0;
+    for (int i = 0; i < n && found <= kMaxClasses; i += 1 + n / 128) {
+        unsigned w;
+        std::memcpy(&w, pts + 4 * (size_t)i + 3, 4);
+        if (std::find(seen, seen + found, w) == seen + found) seen[found++] = w;
+    }
+    return found;
+}
+
+// Whether points of so many distinct weights go by class: at most kMaxClasses per set, and where the count rows, which
+// are cleared and read, are few against the points.  One-shot calls also make the lists for the one profile.
+// 15 classes, whole one-shot calls by class and by value: 200 points + 40 waters 182 and 169 us, 500 + 100 187
+// and 199; a kept structure's profile: 60 + 12 67 and 51 us, 200 + 40 74 and 90, 500 + 100 78 and 118.
+bool Structure::weights_pay(int atoms, int waters) const {
+    if (atoms > kMaxClasses || waters > kMaxClasses) return false;
+    return (long long)atoms * atoms + atoms * waters + waters * waters <= (one_shot ? 1LL : 2LL) * ((long long)n_a + n_w);
+}
+
 void Structure::load_begin(const float* atoms, int n_atoms, const float* waters, int n_waters, const float* exv,
                            int n_exv, int ff_typed_, bool host, PrepStats* h_stats, PrepStats* d_stats, int exv_host) {
     if (n_atoms < 0 || n_waters < 0 || n_exv < 0) throw Error{AUSAXS_ERR_ARGUMENT, "negative point count"};
@@ -111,10 +132,14 @@ void Structure::load_begin(const float* atoms, int n_atoms, const float* waters,
     PrepStats init{};
     for (int k = 0; k < 3; ++k) init.lo[k] = 0xffffffffu, init.hi[k] = 0;
     for (auto& w : init.weights) w.clear();
+    // weights are classified by the census unless a sample already has too many (two censuses with and without
+    // classes of 500 points of 300 weights: 6 us)
+    const bool classes = !ff_typed && (!host || weights_pay(sampled_weights(atoms, n_a), sampled_weights(waters, n_w)));
+    if (!classes) init.weights[0].over = init.weights[1].over = 1;
     *h_stats = init;  // pinned: the copy below reads it asynchronously, the census result overwrites it
     AUSAXS_CUDA(cudaMemcpyAsync(d_stats, h_stats, sizeof(PrepStats), cudaMemcpyHostToDevice, s));
-    census_launch(raw_a.as<float4>(), n_a, ff_typed, d_stats, ff_typed ? nullptr : &d_stats->weights[0], C.sm_count, s);
-    census_launch(raw_w.as<float4>(), n_w, 0, d_stats, ff_typed ? nullptr : &d_stats->weights[1], C.sm_count, s);
+    census_launch(raw_a.as<float4>(), n_a, ff_typed, d_stats, classes ? &d_stats->weights[0] : nullptr, C.sm_count, s);
+    census_launch(raw_w.as<float4>(), n_w, 0, d_stats, classes ? &d_stats->weights[1] : nullptr, C.sm_count, s);
     census_launch(raw_x.as<float4>(), n_x, 0, d_stats, nullptr, C.sm_count, s);
     radius_launch(raw_a.as<float4>(), n_a, raw_w.as<float4>(), n_w, raw_x.as<float4>(), n_x, d_stats, C.sm_count, s);
     C.check_launch("census");
@@ -205,7 +230,9 @@ void Structure::load_end(const PrepStats& st) {
     n_cls[0] = n_cls[1] = 0;
     std::memset(cls_count, 0, sizeof cls_count);
     std::vector<std::pair<unsigned, int>> found[2];
-    if (!st.weights[0].sorted(found[0]) || !st.weights[1].sorted(found[1])) return;
+    if (!st.weights[0].sorted(found[0]) || !st.weights[1].sorted(found[1]) ||
+        !weights_pay((int)found[0].size(), (int)found[1].size()))
+        return;
     for (int k = 0; k < 2; ++k) {
         const int n = k ? n_w : n_a;
         if (n == 0) continue;
@@ -657,7 +684,8 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     const float4* X = raw_x.as<float4>();
     // Weighted points of few classes of weight: the counts by class pair give the weight sums, so the pairs
     // go through the one-atomic kernel (20,011 weighted atoms + 4,003 waters, a whole profile: 636 us by the
-    // two-atomic kernel with weight sums, 300 us by class).
+    // two-atomic kernel with weight sums, 300 us by class; of 8 and 15 classes 305 and 357; 5,000 + 1,000 of 4 and 15
+    // classes 64 and 97 us, by value 135).
     bool by_class = false;
     if (mt && (n_a == 0 || n_cls[0] > 0) && (n_w == 0 || n_cls[1] > 0) && n_a + n_w > 0) {
         pair_sqrt_prepare(P.inv_w, nb);

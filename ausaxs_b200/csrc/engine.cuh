@@ -167,6 +167,7 @@ struct Structure {
     DevBuf raw_a, raw_w, raw_x, dense_a, meta;
     DevBuf typed;           // the atoms' lists by type (typed_bytes)
     TypedSet lists;
+    bool one_shot = false;  // the context's, loaded anew by every one-shot call
     bool want_pos = false;  // also every atom's place in them (typed_pos)
     // Weighted structures whose atoms and waters have at most kMaxClasses distinct weights each: the classes
     // (ascending bit patterns), the points with their class as type, and their lists.  n_cls 0: more.
@@ -207,6 +208,7 @@ struct Structure {
     Plan& plan_for(const ausaxs_hist_config& cfg);
     bool upload_pack(Plan& P);
     void set_classes(FinalizeMT& F) const;
+    bool weights_pay(int atoms, int waters) const;
     void enqueue_histogram(const ausaxs_hist_config& cfg);
     void enqueue_debye(const ausaxs_hist_config& cfg, const double* q_dev, int nq, const ausaxs_debye_params& p,
                        double* Iq_dev, double* prof_dev);

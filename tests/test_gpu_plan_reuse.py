@@ -114,3 +114,25 @@ def test_weights_change_between_calls(classes):
         for got, want in ((h.get_aa_counts(), o.aa), (h.get_aw_counts(), o.aw), (h.get_ww_counts(), o.ww)):
             np.testing.assert_array_equal(got, want)
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [30, 119, 120, 121, 239, 240, 241, 700])
+def test_weights_by_class_or_value(n):
+    """15 classes (225 count rows): few points go by value, sooner in a one-shot call than in a kept structure.  The
+    weights are whole numbers, so every route gives the oracle's sums."""
+    rng = np.random.default_rng(n)
+    xyz = synth.globule(5, n)[0]
+    w = (1.0 + np.arange(n) % 15)[rng.permutation(n)]
+    m = ab.Molecule(atoms=xyz, weights=w)
+    ctx = _capi.Context(0)
+    manager = hist.HistogramManagerMT(m, True, 0.25, 8000, ctx)
+    h = manager.calculate_all()
+    a, waters = m.compact_w()
+    kept = _capi.Structure(ctx, a, waters, ff_typed=False)
+    r, bufs = kept.histogram(manager.config(), 8000)
+    o = O.hist_simple(a, waters, 0.25, 8000)
+    assert h.max_bin == r.max_bin == len(o.tot)
+    np.testing.assert_array_equal(h.get_aa_counts(), o.aa)
+    np.testing.assert_array_equal(bufs["aa"][:r.max_bin], o.aa)
+    kept.close()
+    ctx.close()
