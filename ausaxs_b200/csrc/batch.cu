@@ -254,7 +254,7 @@ struct Batch {
     bool build_packed(const Candidate& c) {
         for (auto& S : items)
             if (!S->plan.packed && S->plan.pairs > 0) return false;
-        const int nr = pair_sqrt_mode(items[order[0]]->plan.inv_w, max_nb);
+        const int nr = pack_sqrt_mode(items[order[0]]->plan.inv_w, max_nb);
         if (!nr) return false;
         const bool grid = cfg.manager == AUSAXS_MANAGER_FFGRID;
         std::vector<Launch> found;

@@ -307,7 +307,7 @@ struct Calculator {
             }
             pair_sqrt_prepare(inv_w, nb);
             PackLaunch fit{};
-            fit.nr = pair_sqrt_mode(inv_w, nb);
+            fit.nr = pack_sqrt_mode(inv_w, nb);
             fit.rows = fit.group_rows = (int)found.size();
             fit.group_sums = fit.offsets = 1;
             fit.bins = nb;

@@ -506,7 +506,7 @@ static double pack_tiles(const std::vector<JobSpec>& specs, int outer, int tile_
 
 bool choose_pack(const Plan& P, int sm_count, PackLaunch& L, int& shape, int& grid, PackTable& T, bool may_join) {
     L = PackLaunch{};
-    L.nr = pair_sqrt_mode(P.inv_w, P.nb);
+    L.nr = pack_sqrt_mode(P.inv_w, P.nb);
     L.offsets = P.weighted;
     if (!L.nr || P.specs.empty()) return false;
     auto table = [&](int s, int tile_j, bool joint) {
@@ -690,7 +690,7 @@ Plan& Structure::plan_for(const ausaxs_hist_config& cfg) {
     if (mt && (n_a == 0 || n_cls[0] > 0) && (n_w == 0 || n_cls[1] > 0) && n_a + n_w > 0) {
         pair_sqrt_prepare(P.inv_w, nb);
         PackLaunch K{};
-        K.nr = pair_sqrt_mode(P.inv_w, nb);
+        K.nr = pack_sqrt_mode(P.inv_w, nb);
         K.rows = K.group_rows = std::max(1, std::max(n_cls[0], n_cls[1]));
         K.group_sums = 1;
         K.bins = nb;

@@ -28,8 +28,10 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 
 #include "pairhist.cuh"
+#include "pairpack.cuh"
 
 namespace ausaxs_b200 {
 
@@ -605,8 +607,14 @@ struct SqrtVerified {
     std::mutex m;
     std::map<uint32_t, int> bins;    // inverse bin width (bits) -> bins verified
     std::map<uint32_t, int> failed;  // -> bins at which the check failed (never tried again from there on)
+    std::set<uint32_t> scalar_only;  // verified, but the packed evaluation of pairpack.cu differs
 };
 SqrtVerified g_sqrt;
+
+bool power_of_two(float inv_w) {
+    int e = 0;
+    return std::frexp(inv_w, &e) == 0.5f;
+}
 
 }  // namespace
 
@@ -641,12 +649,13 @@ bool pair_sqrt_prepare(float inv_w, int bins) {
     uint32_t hi;
     std::memcpy(&hi, &s_max, 4);
     unsigned long long* d = nullptr;
-    unsigned long long h = 1;
+    unsigned long long h[2] = {1, 1};  // mismatches of the root, and of the packed evaluation
     bool ok = false;
-    if (hi < 0x7f800000u && cudaMalloc(&d, sizeof(unsigned long long)) == cudaSuccess) {
-        if (cudaMemset(d, 0, sizeof(unsigned long long)) == cudaSuccess) {
+    if (hi < 0x7f800000u && cudaMalloc(&d, sizeof h) == cudaSuccess) {
+        if (cudaMemset(d, 0, sizeof h) == cudaSuccess) {
             sqrt_check_kernel<<<148 * 8, 256>>>(hi + 1, inv_w, d);
-            ok = cudaMemcpy(&h, d, sizeof(unsigned long long), cudaMemcpyDeviceToHost) == cudaSuccess && h == 0;
+            pack_check_launch(inv_w, want, power_of_two(inv_w), d + 1, nullptr);
+            ok = cudaMemcpy(h, d, sizeof h, cudaMemcpyDeviceToHost) == cudaSuccess && h[0] == 0;
         }
         cudaFree(d);
     }
@@ -654,6 +663,7 @@ bool pair_sqrt_prepare(float inv_w, int bins) {
     std::lock_guard<std::mutex> lk(g_sqrt.m);
     if (ok) g_sqrt.bins[key] = std::max(g_sqrt.bins[key], want);
     else g_sqrt.failed[key] = want;
+    if (ok && h[1]) g_sqrt.scalar_only.insert(key);
     return ok;
 }
 
@@ -665,8 +675,17 @@ int pair_sqrt_mode(float inv_w, int bins) {
     if (!(inv_w > 0) || it == g_sqrt.bins.end() || it->second < bins) return 0;
     // a power-of-two inverse width (0.25 A bins): the product d inv_w is exact, so the rounding to a
     // bin fuses with it (one FMA per pair instead of a product and a sum)
-    int e = 0;
-    return std::frexp(inv_w, &e) == 0.5f ? 2 : 1;
+    return power_of_two(inv_w) ? 2 : 1;
+}
+
+int pack_sqrt_mode(float inv_w, int bins) {
+    {
+        std::lock_guard<std::mutex> lk(g_sqrt.m);
+        uint32_t key;
+        std::memcpy(&key, &inv_w, 4);
+        if (g_sqrt.scalar_only.count(key)) return 0;
+    }
+    return pair_sqrt_mode(inv_w, bins);
 }
 
 void pairhist_launch(const PairLaunch& L0, int tile, int grid, size_t smem, cudaStream_t s) {

@@ -151,5 +151,7 @@ bool pair_sqrt_prepare(float inv_w, int bins);
 // The root launches over at most `bins` bins of this width may take: 0 the correctly rounded one, 1 the
 // Newton-Raphson root (verified), 2 that with a power-of-two inv_w.
 int pair_sqrt_mode(float inv_w, int bins);
+// The same for the packed evaluation of pairpack.cu: 0 also where that was found to differ from the scalar one.
+int pack_sqrt_mode(float inv_w, int bins);
 
 }  // namespace ausaxs_b200

@@ -78,7 +78,8 @@ __device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
 
 // A rounded product that a following sum must not absorb: the assembler contracts mul.rn.f32x2 with
 // add.rn.f32x2 into one fma (seen on squared distances one ulp off), but not an fma with a zero
-// addend, which is the same value for products that are not negative.
+// addend, which is the same value for products that are not negative.  pack_check_kernel makes sure of it: with
+// an assembler that folds these too the two-atomic kernel takes over.
 __device__ __forceinline__ u64 product2(u64 a, u64 b) { return fma2(a, b, 0ull); }
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -133,6 +134,59 @@ struct Consts {
     float dmax;  // scaled distance of the overflow column
 };
 
+__device__ __forceinline__ Consts constants(float inv_w, float c, float scale, int nb) {
+    constexpr float S = 1.0f / 8388608.0f;
+    const float iw = inv_w * 8388608.0f, nc = -c * S, sc = scale * 0x1p-126f;
+    const float off = __uint_as_float((1u << kPackCountShift) + static_cast<uint32_t>(kResBias));
+    Consts K;
+    K.iw = pack2(iw, iw);
+    K.mg = pack2(kMagic, kMagic);
+    K.nmg = pack2(-kMagic, -kMagic);
+    K.nc = pack2(nc, nc);
+    K.sc = pack2(sc, sc);
+    K.off = pack2(off, off);
+    K.dmax = static_cast<float>(nb) * c * S;
+    return K;
+}
+
+// Two inner points (negated) against an outer point (held twice): the bins' magic numbers and the values that
+// are added.
+template <int NR, bool DSUM, bool CLAMP>
+__device__ __forceinline__ void pair_values(u64 ox, u64 oy, u64 oz, u64 bx, u64 by, u64 bz, const Consts& K, float& x0, float& x1,
+                                            uint32_t& v0, uint32_t& v1) {
+    const u64 dx = add2(ox, bx), dy = add2(oy, by), dz = add2(oz, bz);
+    const u64 s = add2(add2(product2(dx, dx), product2(dy, dy)), product2(dz, dz));
+    // d = sqrt(s) as pair_sqrt_scaled
+    float s0, s1, y0, y1;
+    unpack2(s, s0, s1);
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(fmaxf(s0, 1e-36f)));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(fmaxf(s1, 1e-36f)));
+    const u64 d0 = mul2(s, pack2(y0, y1));
+    const u64 h = pack2(__int_as_float(__float_as_int(y0) - 0x00800000), __int_as_float(__float_as_int(y1) - 0x00800000));
+    float d00, d01;
+    unpack2(d0, d00, d01);
+    u64 d = fma2(pack2(__fmaf_rn(-d00, d00, s0), __fmaf_rn(-d01, d01, s1)), h, d0);
+    // distances past the last bin (also NaN and inf) become that of the overflow column's centre,
+    // so that every added value is 2^23 + an offset below 2^16.  Launches whose bins cover every
+    // distance (PackLaunch::covered) leave that out: one instruction of 17 per pair.
+    if (CLAMP) {
+        float d1v, d0v;
+        unpack2(d, d0v, d1v);
+        d = pack2(fminf(d0v, K.dmax), fminf(d1v, K.dmax));
+    }
+    // bin by the magic number; a power-of-two width (NR == 2) fuses the product
+    const u64 xm = NR == 2 ? fma2(d, K.iw, K.mg) : add2(product2(d, K.iw), K.mg);
+    unpack2(xm, x0, x1);
+    v0 = v1 = 1u << kPackCountShift;
+    if (DSUM) {
+        const u64 r = fma2(add2(xm, K.nmg), K.nc, d);
+        float t0, t1;
+        unpack2(fma2(r, K.sc, K.off), t0, t1);
+        v0 = __float_as_uint(t0);
+        v1 = __float_as_uint(t1);
+    }
+}
+
 // Four inner points (one quad) against the thread's R outer points.  MASK: only inner positions in
 // [p[k], kt) of outer point k are valid; n counts the valid pairs.
 template <bool MASK, int R, int NR, bool DSUM, bool CLAMP>
@@ -145,38 +199,9 @@ __device__ __forceinline__ void quad_pairs(const Quad* __restrict__ q, int k0, c
         const u64 bx = u ? X.y : X.x, by = u ? Y.y : Y.x, bz = u ? Z.y : Z.x;
 #pragma unroll
         for (int k = 0; k < R; ++k) {
-            const u64 dx = add2(ox[k], bx), dy = add2(oy[k], by), dz = add2(oz[k], bz);
-            const u64 s = add2(add2(product2(dx, dx), product2(dy, dy)), product2(dz, dz));
-            // d = sqrt(s) as pair_sqrt_scaled
-            float s0, s1, y0, y1;
-            unpack2(s, s0, s1);
-            asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(fmaxf(s0, 1e-36f)));
-            asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(fmaxf(s1, 1e-36f)));
-            const u64 d0 = mul2(s, pack2(y0, y1));
-            const u64 h = pack2(__int_as_float(__float_as_int(y0) - 0x00800000), __int_as_float(__float_as_int(y1) - 0x00800000));
-            float d00, d01;
-            unpack2(d0, d00, d01);
-            u64 d = fma2(pack2(__fmaf_rn(-d00, d00, s0), __fmaf_rn(-d01, d01, s1)), h, d0);
-            // distances past the last bin (also NaN and inf) become that of the overflow column's centre,
-            // so that every added value is 2^23 + an offset below 2^16.  Launches whose bins cover every
-            // distance (PackLaunch::covered) leave that out: one instruction of 17 per pair.
-            if (CLAMP) {
-                float d1v, d0v;
-                unpack2(d, d0v, d1v);
-                d = pack2(fminf(d0v, K.dmax), fminf(d1v, K.dmax));
-            }
-            // bin by the magic number; a power-of-two width (NR == 2) fuses the product
-            const u64 xm = NR == 2 ? fma2(d, K.iw, K.mg) : add2(product2(d, K.iw), K.mg);
             float x0, x1;
-            unpack2(xm, x0, x1);
-            uint32_t v0 = 1u << kPackCountShift, v1 = 1u << kPackCountShift;
-            if (DSUM) {
-                const u64 r = fma2(add2(xm, K.nmg), K.nc, d);
-                float t0, t1;
-                unpack2(fma2(r, K.sc, K.off), t0, t1);
-                v0 = __float_as_uint(t0);
-                v1 = __float_as_uint(t1);
-            }
+            uint32_t v0, v1;
+            pair_values<NR, DSUM, CLAMP>(ox[k], oy[k], oz[k], bx, by, bz, K, x0, x1, v0, v1);
             const uint32_t a0 = caddr[k] + (__float_as_uint(x0) << 2), a1 = caddr[k] + (__float_as_uint(x1) << 2);
             if (MASK) {
                 const int j = k0 + 2 * u;
@@ -504,19 +529,7 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
             const int qa = min(kq, s0 + group * seg), qb = min(kq, qa + seg);
             int n = 0;
             if (s0 < kq && slow_left == 0) {
-                Consts K;
-                {
-                    constexpr float S = 1.0f / 8388608.0f;
-                    const float iw = J.inv_w * 8388608.0f, nc = -J.c * S, sc = J.scale * 0x1p-126f;
-                    const float off = __uint_as_float((1u << kPackCountShift) + static_cast<uint32_t>(kResBias));
-                    K.iw = pack2(iw, iw);
-                    K.mg = pack2(kMagic, kMagic);
-                    K.nmg = pack2(-kMagic, -kMagic);
-                    K.nc = pack2(nc, nc);
-                    K.sc = pack2(sc, sc);
-                    K.off = pack2(off, off);
-                    K.dmax = static_cast<float>(nb) * J.c * S;
-                }
+                const Consts K = constants(J.inv_w, J.c, J.scale, nb);
                 const int m0 = min(qb, max(qa, mq0)), m1 = max(m0, min(qb, mq1));
                 for (int q = max(qa, q_warp); q < m0; ++q)
                     quad_pairs<true, R, NR, DSUM, CLAMP>(s_q + q, 4 * q, ox, oy, oz, caddr, p, kt, K, n);
@@ -654,6 +667,42 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
     }
 }
 
+// The packed evaluation against the scalar one, on points of boxes up to the reach of nb bins: pairs whose bin or
+// offset differs.
+template <int NR>
+__global__ void pack_check_kernel(float inv_w, float c, float scale, int nb, u64* mismatches) {
+    uint32_t state = (blockIdx.x * blockDim.x + threadIdx.x) * 2654435761u + 12345u;
+    const Consts K = constants(inv_w, c, scale, nb);
+    constexpr float S = 1.0f / 8388608.0f;
+    int bad = 0;
+    for (int it = 0; it < 32; ++it) {
+        const float box = 0.5f * static_cast<float>(nb) * c / static_cast<float>(1 << (it & 7));
+        float v[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            state = state * 1664525u + 1013904223u;
+            v[k] = static_cast<float>(state >> 8) * 0x1p-24f * box;
+        }
+        const u64 ox = pack2(v[0] * S, v[0] * S), oy = pack2(v[1] * S, v[1] * S), oz = pack2(v[2] * S, v[2] * S);
+        const u64 bx = pack2(-v[3] * S, -v[6] * S), by = pack2(-v[4] * S, -v[7] * S), bz = pack2(-v[5] * S, -v[8] * S);
+        float x[4];
+        uint32_t add[4];
+        pair_values<NR, true, true>(ox, oy, oz, bx, by, bz, K, x[0], x[1], add[0], add[1]);
+        pair_values<NR, true, false>(ox, oy, oz, bx, by, bz, K, x[2], x[3], add[2], add[3]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float* b = v + 3 + 3 * (k & 1);
+            const float dx = __fsub_rn(v[0], b[0]), dy = __fsub_rn(v[1], b[1]), dz = __fsub_rn(v[2], b[2]);
+            const float d = pair_sqrt_nr(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
+            const float xm = __fadd_rn(__fmul_rn(d, inv_w), kMagic);
+            const float t = __fmaf_rn(__fmaf_rn(-__fsub_rn(xm, kMagic), c, d), scale, kMagic);
+            const uint32_t want = (1u << kPackCountShift) + static_cast<uint32_t>(__float_as_int(t) - kMagicBits + kResBias);
+            if (x[k] != xm || add[k] != want) ++bad;
+        }
+    }
+    if (bad) atomicAdd(mismatches, static_cast<u64>(bad));
+}
+
 using Kernel = void (*)(const PackLaunch);
 
 template <int NT, int G, bool CLAMP>
@@ -708,6 +757,13 @@ int pack_copies(int rows, int bins, int spread, double largest_row_share) {
            pack_segment_pairs(spread, largest_row_share / n) < kLongSegment)
         n *= 2;
     return n;
+}
+
+void pack_check_launch(float inv_w, int bins, bool power_of_two, unsigned long long* mismatches, cudaStream_t s) {
+    const float c = static_cast<float>(1.0 / static_cast<double>(inv_w));
+    const float scale = static_cast<float>(32768.0 / static_cast<double>(c) * (1.0 - 1.0 / 256));
+    if (power_of_two) pack_check_kernel<2><<<148, 256, 0, s>>>(inv_w, c, scale, bins, mismatches);
+    else pack_check_kernel<1><<<148, 256, 0, s>>>(inv_w, c, scale, bins, mismatches);
 }
 
 void pack_launch(const PackLaunch& L, int shape, int grid, cudaStream_t s) {

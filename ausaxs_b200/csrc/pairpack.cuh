@@ -72,6 +72,8 @@ int pack_shape(const PackLaunch& L);
 int pack_segment_pairs(int bins, double largest_row_share);
 // copies of the packed words of a job of `rows` rows whose distances spread over `spread` of its bins
 int pack_copies(int rows, int bins, int spread, double largest_row_share);
+// Adds the pairs of a sample whose packed evaluation differs from the scalar one to *mismatches.
+void pack_check_launch(float inv_w, int bins, bool power_of_two, unsigned long long* mismatches, cudaStream_t s);
 void pack_launch(const PackLaunch& L, int shape, int grid, cudaStream_t s);
 
 }  // namespace ausaxs_b200
