@@ -250,8 +250,9 @@ struct Ctx {
     std::shared_ptr<Hydrator> hyd;  // hydration workspace (hydrate.cuh)
     DevBuf io;                     // q / I(q) / profiles of one-shot host calls
     // SimpleCalculator runs (each synchronises before it returns): points and lists, accumulators, outputs,
-    // tables; kept up to kCalcKeep bytes each
-    static constexpr size_t kCalcKeep = 256u << 20;
+    // tables; a run gives back what is larger than kCalcKeep bytes (as much takes a run so long that allocating
+    // it anew does not show: 600,000 points, or 400 results of 3,000 bins)
+    static constexpr size_t kCalcKeep = 32u << 20;
     DevBuf calc[4];
     DevBuf tc;                     // tensor-core scratch of one-shot host calls
     XBufs x;                       // exact tensor-core transform of one-shot host calls

@@ -198,3 +198,17 @@ def test_many_jobs_by_class(classes, sizes, launches, gpu_ctx):
     assert gpu_ctx.launches - before == launches
     for (cross, mid), ref in O.calculator(sets, jobs, 0.25, 8000).items():
         check_result(out["cross" if cross else "self"][mid], ref, sets, 0.25, 8000)
+
+
+def test_large_buffers_are_given_back(gpu_ctx):
+    """A run keeps small buffers for the next one and gives the large ones back (500 results of 7,600 bins: 90 MB of
+    accumulators and as much of outputs)."""
+    import torch
+
+    pts = [np.array([[0, 0, 0, 1.0], [1900, 0, 0, 2.0 + k]], np.float32) for k in range(500)]
+    run_gpu(gpu_ctx, pts[:2], [(0, None, 1, -1), (1, None, 1, -1)], 0.25)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    out, _ = run_gpu(gpu_ctx, pts, [(k, None, 1, -1) for k in range(500)], 0.25)
+    assert torch.cuda.mem_get_info()[0] >= before - (40 << 20)
+    assert out["self"][499][0][7600] == 2 * (2.0 + 499)
