@@ -509,16 +509,16 @@ bool choose_pack(const Plan& P, int sm_count, PackLaunch& L, int& shape, int& gr
     L.nr = pack_sqrt_mode(P.inv_w, P.nb);
     L.offsets = P.weighted;
     if (!L.nr || P.specs.empty()) return false;
-    auto table = [&](int s, int tile_j, bool joint) {
+    auto table = [&](int s, int tile_j, bool joint, PackTable& to) {
         PackLaunch K{};
         K.nr = L.nr;
         K.offsets = L.offsets;
         K.tile_j = tile_j;
-        T = PackTable{};
-        append_pack_jobs(P, kPackShapes[s].outer(), joint, K, T, true);
+        append_pack_jobs(P, kPackShapes[s].outer(), joint, K, to, true);
         return K;
     };
-    L = table(0, kPackMaxTileJ, false);
+    T = PackTable{};
+    L = table(0, kPackMaxTileJ, false, T);
     const int s0 = pack_shape(L);
     if (s0 < 0) return false;
     // The longest inner tiles that still give every resident CTA two tiles (a tile costs about 3 us beyond
@@ -538,13 +538,25 @@ bool choose_pack(const Plan& P, int sm_count, PackLaunch& L, int& shape, int& gr
         return false;
     };
     if (!pick(s0, 256) && s0 == 0) pick(2, 64);
+    // the tables for other tiles: the same jobs, other tile numbers
+    L.tile_j = tile_j;
+    L.total_tiles = 0;
+    const int outer = kPackShapes[shape].outer();
+    for (PackJob& p : T.jobs) {
+        p.tiles_i = (p.na + outer - 1) / outer;
+        p.tiles_j = (p.nb + tile_j - 1) / tile_j;
+        p.tile_begin = L.total_tiles;
+        L.total_tiles += (long long)p.tiles_i * p.tiles_j;
+    }
     // one group where its rows cost no CTA per SM: a CTA then flushes once, not at every change of job
-    L = table(shape, tile_j, false);
     const int per_sm = pack_ctas_per_sm(shape, L);
     if (may_join) {
-        const PackLaunch joint = table(shape, tile_j, true);
-        if (pack_ctas_per_sm(shape, joint) >= per_sm) L = joint;
-        else L = table(shape, tile_j, false);
+        PackTable together;
+        const PackLaunch joint = table(shape, tile_j, true, together);
+        if (pack_ctas_per_sm(shape, joint) >= per_sm) {
+            L = joint;
+            T = std::move(together);
+        }
     }
     grid = (int)std::min<long long>((long long)sm_count * per_sm, std::max<long long>(1, L.total_tiles));
     return true;

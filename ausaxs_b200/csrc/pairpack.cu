@@ -569,7 +569,8 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
                             uint4* const pw = reinterpret_cast<uint4*>(s_pk + r * pad + b);
                             uint2* const pc = reinterpret_cast<uint2*>(s_cnt + (MANY ? row : r) * pad + b);
                             const uint4 w = *pw;
-                            uint2 c = MANY ? make_uint2(0, 0) : *pc;
+                            const bool shared = MANY && split > 1;
+                            uint2 c = shared ? make_uint2(0, 0) : *pc;
                             *pw = make_uint4(0, 0, 0, 0);
                             const uint32_t n0 = w.x >> kPackCountShift, n1 = w.y >> kPackCountShift, n2 = w.z >> kPackCountShift,
                                            n3 = w.w >> kPackCountShift;
@@ -577,13 +578,13 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
                             c = undo ? make_uint2(c.x - c0, c.y - c1) : make_uint2(c.x + c0, c.y + c1);
                             off = make_uint4(off.x + (w.x & kOffsetMask), off.y + (w.y & kOffsetMask), off.z + (w.z & kOffsetMask),
                                              off.w + (w.w & kOffsetMask));
-                            if (MANY) {
+                            if (shared) {
                                 if (c.x) shared_red_add(smem_addr(pc), c.x);
                                 if (c.y) shared_red_add(smem_addr(pc) + 4, c.y);
-                                row += split;
                             } else {
                                 *pc = c;
                             }
+                            row += split;
                             sum += static_cast<int>(n0 + n1) + static_cast<int>(n2 + n3);
                             fill = max(max(fill, w.x), w.y);
                             fill = max(max(fill, w.z), w.w);

@@ -475,7 +475,7 @@ struct Assembly {
         enqueue_pairs(work[B]);
         AUSAXS_CUDA(cudaStreamSynchronize(C.stream));
         footprint = S.raw_a.n + S.raw_w.n + S.raw_x.n + S.dense_a.n + S.meta.n + P.dev.n + orig.n + part.n + tables.n +
-                    io.n + C.stats.n + S.typed.n + lists.n + lists_orig.n;
+                    io.n + C.stats.n + S.typed.n + lists.n;
     }
 
     // every body's atom lists by type (of the loaded, dense coordinates) and their original coordinates
@@ -485,8 +485,9 @@ struct Assembly {
             list_off.push_back(at);
             at += align_up(Structure::typed_bytes(a_off[k + 1] - a_off[k]), 256);
         }
-        lists.ensure(std::max<size_t>(at, 256));
-        lists_orig.ensure(std::max<size_t>(at, 256));
+        at = std::max<size_t>(at, 256);
+        lists.ensure(2 * at);  // one allocation: they cost more than the lists
+        lists_orig.view(lists.as<char>(at), at);
         body_lists.resize(B);
         for (int k = 0; k < B; ++k) {
             const int n = a_off[k + 1] - a_off[k];
