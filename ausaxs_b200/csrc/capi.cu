@@ -557,7 +557,7 @@ int ausaxs_gpu_grid_exv(ausaxs_gpu_ctx* ctx, const float* atoms, int32_t n_atoms
         *n_exv = 0;
         if (volume) *volume = 0;
         Structure& S = scratch(C);  // census and validation of the points (form-factor types, finite coordinates)
-        S.load(atoms, n_atoms, waters, n_waters, nullptr, 0, 1, host);
+        S.load(atoms, n_atoms, waters, n_waters, nullptr, 0, 1, host, -1, true);
         GridExv& g = grid_workspace(C);
         // device output: the dummies go straight to exv_out; a short buffer fails once the count is known
         float4* direct = (!host && capacity > 0) ? reinterpret_cast<float4*>(exv_out) : nullptr;

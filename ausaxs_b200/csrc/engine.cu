@@ -175,7 +175,7 @@ TypedSet typed_lists(const float4* in, float4* dense, int n, const TypeMap& map,
     return set;
 }
 
-void Structure::load_end(const PrepStats& st) {
+void Structure::load_end(const PrepStats& st, bool census_only) {
     Ctx& C = *ctx;
     cudaStream_t s = C.stream;
     if (st.bad & 1u)
@@ -212,6 +212,7 @@ void Structure::load_end(const PrepStats& st) {
             }
     }
     T = T_new;
+    if (census_only) return;
     meta.ensure(256);
     for (int k = 0; k < kNff; ++k) hmeta[k] = k < T ? type_count[k] : 0, hmeta[kNff + k] = ff_to_type[k];
     // pageable source: the call returns once the bytes are staged, so hmeta may change afterwards
@@ -255,12 +256,12 @@ void Structure::load_end(const PrepStats& st) {
 }
 
 void Structure::load(const float* atoms, int n_atoms, const float* waters, int n_waters, const float* exv, int n_exv,
-                     int ff_typed_, bool host, int exv_host) {
+                     int ff_typed_, bool host, int exv_host, bool census_only) {
     Ctx& C = *ctx;
     C.stats.ensure(sizeof(PrepStats));
     load_begin(atoms, n_atoms, waters, n_waters, exv, n_exv, ff_typed_, host, C.h_stats, C.stats.as<PrepStats>(), exv_host);
     AUSAXS_CUDA(cudaStreamSynchronize(C.stream));
-    load_end(*C.h_stats);
+    load_end(*C.h_stats, census_only);
 }
 
 static long long tri(long long t) { return t * (t + 1) / 2; }
