@@ -34,10 +34,10 @@
 // All accumulations are integer, so results do not depend on scheduling; counts and offsets are those of
 // pairhist.cu bit for bit (the same roundings up to the power-of-two scale).
 //
-// Measured on the B200: the inner loop alone (405 bins) 1,702 Gpair/s against 1,171 for the scalar
-// two-atomic loop of pairhist.cu; launches of 50,000 atoms + 10,000 waters at 0.25 A bins 1,345 Gpair/s (17.2
-// warp instructions per 32 pairs, FMA pipe 64 %, shared-memory wavefronts 74 % of peak) against 1,040, of
-// a 264,000-point shell at 3,092 bins 1,240 against 990.  Per-segment drains and checks take about 15 %.
+// Measured on the B200: the inner loop alone (405 bins) 1,702 Gpair/s with the clamp and 1,815 without against
+// 1,171 for the scalar two-atomic loop of pairhist.cu; launches of 50,000 atoms + 10,000 waters at 0.25 A bins 1,406
+// Gpair/s (16.9 warp instructions per 32 pairs, FMA pipe 67 %, shared-memory wavefronts 76 % of peak) against 1,040,
+// of a 264,000-point shell at 3,092 bins 1,286 against 943.  Per-segment drains and checks take about 15 %.
 #include <algorithm>
 #include <type_traits>
 

@@ -37,14 +37,16 @@ import numpy as np  # noqa: E402
 
 # warp instructions per 32 pair evaluations of the one-atomic pair kernel at 0.25 A bins (the bin rounding
 # fused with the power-of-two inverse width), segment drains and checks included, counted by ncu
-# (smsp__inst_executed / pairs, profiles/pack_kernel_50k_atoms.md)
-INSTR_PER_PAIR = 17.2
+# (smsp__inst_executed / pairs, profiles/pack_kernel_50k_atoms.md; batches and moves add the overflow clamp, about one)
+INSTR_PER_PAIR = 16.9
 # FP32 operations per pair that the reference's rounding order and the fixed-point offset need: 3 sub, 3 mul,
 # 2 add, the root's 4, bin rounding, offset 3, and the root's guard
 FP32_PER_PAIR = 17.0
-# DRAM bytes (read + write) of the pair launches of one step of the 256-structure batch: 16.6 MB per pass
+# DRAM bytes (read + write) of the pair launches of one step of the 256-structure batch: 30.9 MB per pass
 # measured by ncu on its first 64 structures (0.86M points), scaled by points to the batch's 3.66M
-BATCH_PAIR_TRAFFIC_BYTES = 7.0e7
+BATCH_PAIR_TRAFFIC_BYTES = 1.3e8
+# what the pair stage launches: the one-atomic kernel, unless a plan's width or layout does not take it
+PAIR_KERNEL = "pack_kernel (pairhist_kernel where a plan does not take it)"
 METRIC = "I(q) profiles/s & p99 latency vs plain GPU path at ≤1e-4 rel. I(q) error"
 UNIT = "profiles/s"
 
@@ -296,7 +298,7 @@ def pair_roofline(pairs_per_launch: float, kernel_ms: float, sm_mhz: float, sms:
     atom = atomic_rate / atomics_per_pair
     peak = min(fp32, atom)
     issue = sms * 4 * sm_mhz * 1e6 * 32 / instr_per_pair
-    return {"bound": "fp32" if fp32 <= atom else "smem_atomic", "kernel": "pack_kernel",
+    return {"bound": "fp32" if fp32 <= atom else "smem_atomic", "kernel": PAIR_KERNEL,
             "achieved": achieved / 1e9, "peak": peak / 1e9, "unit": "Gpair/s", "frac": achieved / peak,
             "fp32_bound": fp32 / 1e9, "smem_atomic_bound": atom / 1e9, "smem_atomics_per_s": atomic_rate,
             "atomics_per_pair": atomics_per_pair, "sm_mhz": sm_mhz, "issue_frac": achieved / issue,
@@ -1271,7 +1273,7 @@ def run_fit(args, rank, world, local_rank):
                 "d2h_bytes_per_step": int(8 * (NFF * NFF + NFF + 3) * h.max_bin + 56),
                 "p50_ms": 1e3 * float(np.percentile(lat, 50)), "p99_ms": 1e3 * float(np.percentile(lat, 99))},
         "gpu_launches": int(launches),
-        "roofline": {"bound": "issue", "kernel": "pack_kernel", "achieved": pair_rate / 1e9, "peak": issue_peak / 1e9,
+        "roofline": {"bound": "issue", "kernel": PAIR_KERNEL, "achieved": pair_rate / 1e9, "peak": issue_peak / 1e9,
                      "unit": "Gpair/s", "frac": pair_rate / issue_peak, "traffic": None,
                      "note": "a 5k-atom histogram is launch-latency bound; the fit kernel itself is one CTA"},
         "clocks": clocks,
