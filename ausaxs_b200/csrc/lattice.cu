@@ -26,6 +26,7 @@
 #include <cmath>
 
 #include "lattice.cuh"
+#include "pairhist.cuh"
 
 namespace ausaxs_b200 {
 
@@ -359,7 +360,8 @@ __global__ void lattice_tail_kernel(LatticeLaunch L) {
 
 template <int W>
 void launch_w(const LatticeLaunch& L, int grid, size_t smem, cudaStream_t s) {
-    cudaFuncSetAttribute(lattice_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the most any launch takes (pack_launch)
+    cudaFuncSetAttribute(lattice_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemCap);
     lattice_kernel<W><<<grid, lattice_threads<W>(), smem, s>>>(L);
 }
 

@@ -527,7 +527,8 @@ __global__ void __launch_bounds__(NT, DREG ? 1 : (WEIGHTED ? (512 / NT > 1 ? 512
 
 template <int NT, int R, bool WEIGHTED, bool DREG, int NR, int G>
 void launch_one(const PairLaunch& L, int grid, size_t smem, cudaStream_t s) {
-    cudaFuncSetAttribute(pairhist_kernel<NT, R, WEIGHTED, DREG, NR, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the most any launch takes (pack_launch)
+    cudaFuncSetAttribute(pairhist_kernel<NT, R, WEIGHTED, DREG, NR, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemCap);
     pairhist_kernel<NT, R, WEIGHTED, DREG, NR, G><<<grid, NT, smem, s>>>(L);
 }
 
@@ -556,7 +557,7 @@ template <int NT, int R, bool WEIGHTED, bool DREG, int G = 1>
 int occupancy_one(size_t smem) {
     // the root variants share the launch shape; the fewest resident CTAs of them bounds the launch
     auto k = pairhist_kernel<NT, R, WEIGHTED, DREG, 0, G>;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemCap) != cudaSuccess) {
         cudaGetLastError();
         return 1;
     }
@@ -567,7 +568,7 @@ int occupancy_one(size_t smem) {
     }
     for (auto k2 : {pairhist_kernel<NT, R, WEIGHTED, DREG, 1, G>, pairhist_kernel<NT, R, WEIGHTED, DREG, 2, G>}) {
         int n2 = 0;
-        if (cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+        if (cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemCap) == cudaSuccess &&
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n2, k2, NT, smem) == cudaSuccess && n2 < n)
             n = n2;
     }

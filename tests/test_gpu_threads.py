@@ -41,3 +41,36 @@ def test_contexts_of_several_threads():
     for t in threads:
         t.join()
     assert not failed, failed
+
+
+def test_weighted_contexts_of_several_threads():
+    """The same through the kernel that weighted points of many weights take."""
+    molecules = []
+    for k, spread in enumerate((1.0, 3.0, 9.0, 20.0)):
+        xyz, _ = synth.globule(k + 1, 500)
+        molecules.append(ab.Molecule(atoms=xyz * spread, weights=1.0 + np.arange(500) % 40))
+    want, failed = [], []
+
+    def counts(m, ctx):
+        return hist.HistogramManagerMT(m, True, 0.25, 8000, ctx).calculate_all().get_aa_counts()
+
+    for m in molecules:
+        ctx = _capi.Context(0)
+        want.append(counts(m, ctx))
+        ctx.close()
+
+    def work(k):
+        try:
+            ctx = _capi.Context(0)
+            for _ in range(100):
+                np.testing.assert_array_equal(counts(molecules[k], ctx), want[k])
+            ctx.close()
+        except BaseException as e:
+            failed.append((k, e))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
