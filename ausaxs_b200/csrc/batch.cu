@@ -268,10 +268,17 @@ struct Batch {
                     K.offsets = cfg.weighted_bins ? 1 : 0;
                     K.tile_j = b ? c.tile_large : c.tile_small;
                     T = PackTable{};
-                    for (int i : order) {
+                    auto here = [&](int i) {
                         const Structure& S = *items[i];
                         const int biggest = std::max({S.n_a, S.n_w, grid ? S.n_x : 0});
-                        if ((c.tile_small != c.tile_large && biggest >= c.threshold ? 1 : 0) != b) continue;
+                        return (c.tile_small != c.tile_large && biggest >= c.threshold ? 1 : 0) == b;
+                    };
+                    // (known before the first job: copies of packed words are sized for the launch's bins)
+                    for (int i : order)
+                        if (here(i)) K.bins = std::max(K.bins, items[i]->plan.nb);
+                    for (int i : order) {
+                        const Structure& S = *items[i];
+                        if (!here(i)) continue;
                         append_pack_jobs(S.plan, kPackShapes[shape].outer(), joint, K, T, false, c.by_class ? cls : -1);
                     }
                     return K;

@@ -374,7 +374,7 @@ void append_pack_jobs(const Plan& P, int outer, bool joint, PackLaunch& L, PackT
             p.tail_end = j.tail_end >= 0 ? j.tail_end : j.nbp;
             p.tail_from_outer = j.tail_from_outer >= 0 ? j.tail_from_outer : j.self;
             const int spread = j.spread_bins > 0 ? std::min(j.spread_bins, P.nb) : P.nb;
-            p.copies = pack_copies(rows_out, P.nb, spread, share);
+            p.copies = pack_copies(rows_out, std::max(L.bins, P.nb), spread, share);
             p.seg_pairs = pack_segment_pairs(spread, share / p.copies);
             p.cnt_row = rows;
             p.mult = j.mult;
@@ -386,8 +386,8 @@ void append_pack_jobs(const Plan& P, int outer, bool joint, PackLaunch& L, PackT
                 if (it == sums.end()) sums.push_back(j.dsum);
             }
             T.jobs.push_back(p);
-            L.rows = std::max(L.rows, (int)(p.rows * p.copies));
             L.bins = std::max(L.bins, P.nb);
+            L.rows = std::max(L.rows, (int)(p.rows * p.copies));
             L.total_tiles += (long long)p.tiles_i * p.tiles_j;
             if (!joint) close(T.jobs.size() - 1);
         }

@@ -27,8 +27,8 @@
 //   * with few bins a word is full after few pairs.  Jobs then keep several copies of their words, the lanes of
 //     a warp in turn, until a segment lasts 24,576 pairs (pack_copies; 8,192 and 16,384 measured up to 12 %
 //     slower at 0.5 A bins, 32,768 up to 2 % at 0.25 A).  Whole calls without and with copies: 12,000 atoms of
-//     one type at 1 A 193 -> 146 us, at 2 A 344 -> 182; 25,000 atoms of four types at 1 A 564 -> 511, at 4 A
-//     1,573 -> 661; of 13 types at 2 A, whose water pairs have a word per bin, 4,162 -> 629;
+//     one type at 1 A 193 -> 143 us, at 2 A 344 -> 154; 25,000 atoms of four types at 1 A 564 -> 463, at 4 A
+//     1,573 -> 548; of 13 types at 2 A, whose water pairs have a word per bin, 4,162 -> 537;
 //   * rows are the outer point's type only: the inner points of a job share one type, so a CTA keeps T
 //     rows instead of T * T and no pair adds a row offset.
 // All accumulations are integer, so results do not depend on scheduling; counts and offsets are those of
@@ -262,12 +262,14 @@ __device__ __forceinline__ void slow_pairs(const Quad* s_q, int k0, int k1, cons
 
 constexpr int kRoom = 511;  // 511 x 2^23 < 2^32 and 511 x 128 < 2^16
 
-// Shared memory of a CTA: packed words [copies][rows][pad], u32 offset sums [group_sums][pad], u16 counts
+// Shared memory of a CTA: packed words [rows][copies][pad], u32 offset sums [group_sums][pad], u16 counts
 // [group_rows][pad], two buffers of tile_j inner points; pad = bins + 1 (the overflow column) rounded up to
-// whole quads of bins.  Counts and offset sums go to the global accumulators when the CTA moves to another
+// whole quads of bins, an odd number of them: where copies lie a multiple of 32 words apart the lanes of a
+// warp, each on its copy, meet in the bank of their bin (50,000 atoms of one type at 4 A, 28 bins: 3,031 us with 32
+// words, 1,549 with 36).  Counts and offset sums go to the global accumulators when the CTA moves to another
 // group or when they could wrap (kRoom); 16-bit counts keep two CTAs on an SM at the 3,100 bins of a 300 A
 // shell.
-__host__ __device__ inline int pack_pad(int bins) { return (bins + 4) & ~3; }
+__host__ __device__ inline int pack_pad(int bins) { return ((bins + 4) & ~3) | 4; }
 
 // Resident CTAs: 16 to 20 warps per SM already reach the pipes' rates (the inner loop alone: 1,688 Gpair/s
 // at 16 warps, 1,702 at 32), so up to 102 registers per thread buy a loop without spills.
@@ -436,7 +438,7 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
             ox[k] = pack2(a.x * S, a.x * S);
             oy[k] = pack2(a.y * S, a.y * S);
             oz[k] = pack2(a.z * S, a.z * S);
-            const int row = (rows > 1 ? __float_as_int(a.w) : 0) + (lane & (J.copies - 1)) * rows;
+            const int row = (rows > 1 ? __float_as_int(a.w) : 0) * J.copies + (lane & (J.copies - 1));
             caddr[k] = smem_addr(s_pk) + 4u * static_cast<uint32_t>(row * pad) - 4u * static_cast<uint32_t>(kMagicBits);
             gi[k] = J.a_base + i;
             p[k] = on ? 0 : 0x7fffffff;
@@ -509,10 +511,9 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
         auto slow = [&](int k0, int k1, int tail_end) {
             uint32_t row0[R];
             int ts[R];
-            const uint32_t copy = static_cast<uint32_t>((lane & (J.copies - 1)) * rows * pad);
 #pragma unroll
             for (int k = 0; k < R; ++k) {
-                row0[k] = (caddr[k] + 4u * static_cast<uint32_t>(kMagicBits) - smem_addr(s_pk)) / 4u - copy;
+                row0[k] = (caddr[k] + 4u * static_cast<uint32_t>(kMagicBits) - smem_addr(s_pk)) / (4u * pad) / J.copies * pad;
                 const int row_begin = J.tail_from_outer ? gi[k] + 1 : 0;
                 ts[k] = tail_end == 0x7fffffff ? tail_end : tail_end - ((tail_end - row_begin) & 3);
             }
@@ -558,16 +559,14 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
                 const int quads = nb / 4 + 1;
                 auto drain = [&](auto several) {
                     constexpr bool MANY = decltype(several)::value;
+                    const int copy_bits = __ffs(J.copies) - 1;
                     const int split = quads * 2 <= NT ? min(pk_rows, NT / quads) : 1;
                     const int first = split > 1 ? tid / quads : 0;
                     for (int b = (tid - first * quads) * 4; b <= nb && first < split; b += NT * 4) {
                         uint4 off = make_uint4(0, 0, 0, 0);
-                        int row = first;  // of the counts
                         for (int r = first; r < pk_rows; r += split) {
-                            if (MANY)
-                                while (row >= rows) row -= rows;
                             uint4* const pw = reinterpret_cast<uint4*>(s_pk + r * pad + b);
-                            uint2* const pc = reinterpret_cast<uint2*>(s_cnt + (MANY ? row : r) * pad + b);
+                            uint2* const pc = reinterpret_cast<uint2*>(s_cnt + (MANY ? r >> copy_bits : r) * pad + b);
                             const uint4 w = *pw;
                             const bool shared = MANY && split > 1;
                             uint2 c = shared ? make_uint2(0, 0) : *pc;
@@ -584,7 +583,6 @@ __global__ void __launch_bounds__(NT, pack_min_blocks(NT)) pack_kernel(const Pac
                             } else {
                                 *pc = c;
                             }
-                            row += split;
                             sum += static_cast<int>(n0 + n1) + static_cast<int>(n2 + n3);
                             fill = max(max(fill, w.x), w.y);
                             fill = max(max(fill, w.z), w.w);

@@ -70,7 +70,7 @@ int pack_shape(const PackLaunch& L);
 // pairs of a job's first segments: the most frequent cell of a protein-like distance distribution
 // then holds about 100 pairs
 int pack_segment_pairs(int bins, double largest_row_share);
-// copies of the packed words of a job of `rows` rows whose distances spread over `spread` of its bins
+// copies of the packed words of a job of `rows` rows whose distances spread over `spread` of the launch's bins
 int pack_copies(int rows, int bins, int spread, double largest_row_share);
 // Adds the pairs of a sample whose packed evaluation differs from the scalar one to *mismatches.
 void pack_check_launch(float inv_w, int bins, bool power_of_two, unsigned long long* mismatches, cudaStream_t s);
