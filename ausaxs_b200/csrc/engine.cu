@@ -388,6 +388,7 @@ void append_pack_jobs(const Plan& P, int outer, bool joint, PackLaunch& L, PackT
             T.jobs.push_back(p);
             L.bins = std::max(L.bins, P.nb);
             L.rows = std::max(L.rows, (int)(p.rows * p.copies));
+            if (p.copies > 1) L.many = 1;
             L.total_tiles += (long long)p.tiles_i * p.tiles_j;
             if (!joint) close(T.jobs.size() - 1);
         }

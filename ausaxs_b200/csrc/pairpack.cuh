@@ -45,6 +45,7 @@ struct PackLaunch {
     unsigned long long* overflow;
     int32_t nr;           // 1: every job's width is verified for the Newton-Raphson root; 2: and is a power of two
     int32_t offsets;      // 0: no job has offset sums (counts only)
+    int32_t many;         // 1: some job keeps several copies of its words
     int32_t covered;      // 1: no pair's distance lies beyond its job's bins
     int32_t max_tiles;    // > 0: a CTA exits after this many tiles (grid * max_tiles >= total_tiles)
 };
